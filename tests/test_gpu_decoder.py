@@ -40,6 +40,36 @@ def test_stepwise_decode_matches_prefill(wf):
     wf.device_status()
 
 
+@pytest.mark.parametrize("B", [1, 5, 20])
+def test_graphed_step_reads_what_its_predecessor_wrote(wf, B):
+    """In a replayed graph every launch starts while its predecessor still runs.  At widths whose projections read int8
+    copies, made by kernels of their own, each step must use this step's activations and not the previous replay's: the
+    graphed steps equal the same steps launched one by one, with other tokens in every step."""
+    from wrinklefree_monorepo_b200.decoder import DecoderConfig, TernaryDecoder
+
+    cfg = DecoderConfig(layers=2, hidden=4096, n_q=32, n_kv=8, head_dim=128, intermediate=14336, vocab=1000)
+    dev = torch.device("cuda", 0)
+    ids = torch.randint(0, cfg.vocab, (B, 12), generator=torch.Generator().manual_seed(6)).to(dev)
+    m = TernaryDecoder(cfg, B, 16, dev, seed=2)
+    m.capture()
+    assert m.qnorm and m.qact
+
+    def steps(one):
+        m.prefill(ids[:, :6])
+        out = []
+        for t in range(6, 12):
+            m.tok.copy_(ids[:, t])
+            one()
+            torch.cuda.synchronize()
+            out.append(m.logits.clone())
+        return torch.stack(out)
+
+    graphed = steps(lambda: m.graph.replay())
+    plain = steps(lambda: m._decode_step())
+    assert torch.equal(graphed, plain)
+    wf.device_status()
+
+
 def test_fused_elementwise_kernels(wf):
     from wrinklefree_monorepo_b200 import ops
 

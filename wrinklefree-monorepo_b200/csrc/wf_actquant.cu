@@ -35,7 +35,7 @@ __device__ __forceinline__ int block_sum_int(int v, int* sh) {
 // One block per token.  K % 8 == 0.
 template <int DT>
 __global__ void __launch_bounds__(AQ_THREADS)
-    act_quant_token_kernel(const void* __restrict__ x, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q,
+    act_quant_token_kernel(const void* x, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q,
                            float* __restrict__ scale, int32_t* __restrict__ rowsum, int x_ready) {
     __shared__ float shf[AQ_THREADS / 32];
     __shared__ int shi[AQ_THREADS / 32];
@@ -133,7 +133,7 @@ static int act_quant_impl(const void* x, int x_dtype, int64_t M, int64_t K, int6
 // of a thread's loads are in flight together.
 template <int DT, int CHUNKS>
 __global__ void __launch_bounds__(AQ_THREADS)
-    act_quant_token_reg_kernel(const void* __restrict__ x, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q,
+    act_quant_token_reg_kernel(const void* x, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q,
                                float* __restrict__ scale, int32_t* __restrict__ rowsum, int x_ready) {
     __shared__ float shf[AQ_THREADS / 32];
     __shared__ int shi[AQ_THREADS / 32];

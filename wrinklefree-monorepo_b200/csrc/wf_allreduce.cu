@@ -75,7 +75,7 @@ __device__ __forceinline__ void accumulate8(const uint4& u, float (&acc)[8]) {
 // n16: 16-byte chunks of the tensor; CTA c handles the chunks c, c + grid, ...
 template <int DT>
 __global__ void __launch_bounds__(AR_THREADS) allreduce_kernel(ArPeers peers, int world, int rank, size_t slot_bytes,
-                                                               const uint4* __restrict__ in, uint4* __restrict__ out, int64_t n16) {
+                                                               const uint4* in, uint4* __restrict__ out, int64_t n16) {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     uint8_t* mine = peers.base[rank];
     unsigned* step_word = reinterpret_cast<unsigned*>(mine + 2048);
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(AR_THREADS) allreduce_kernel(ArPeers peers, in
     // 1. publish the partial tensor
     uint4* my_slot = reinterpret_cast<uint4*>(mine + slot);
     for (int64_t i = cta * static_cast<int64_t>(AR_THREADS) + tid; i < n16; i += static_cast<int64_t>(gridDim.x) * AR_THREADS)
-        my_slot[i] = in[i];
+        my_slot[i] = ld16_chained(in + i);
     __threadfence_system();
     __syncthreads();
     // 2. tell every peer (and this rank itself)

@@ -92,17 +92,26 @@ struct Elem<WF_BF16> {
     static constexpr int VEC = 8;
 };
 
+// 16 bytes that an earlier kernel of the stream may have written.  Not __ldg, and no `const __restrict__` pointer: both give
+// the non-coherent load, which the compiler may move above griddepcontrol.wait, and a launch that starts while its
+// predecessor still runs then reads what the buffer held before.  The asm keeps its place behind that wait.
+__device__ __forceinline__ uint4 ld16_chained(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 // Loads 8 consecutive elements starting at p (16-byte aligned for 2-byte types,
 // 32-byte aligned pairs of loads for fp32) into f[8].
 template <int DT>
 __device__ __forceinline__ void load8(const void* base, int64_t elem_off, float (&f)[8]) {
     if constexpr (DT == WF_F32) {
-        const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(base) + elem_off);
-        float4 a = __ldg(p), b = __ldg(p + 1);
-        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
-        f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+        const float* p = static_cast<const float*>(base) + elem_off;
+        const uint4 a = ld16_chained(p), b = ld16_chained(p + 4);
+        f[0] = __uint_as_float(a.x); f[1] = __uint_as_float(a.y); f[2] = __uint_as_float(a.z); f[3] = __uint_as_float(a.w);
+        f[4] = __uint_as_float(b.x); f[5] = __uint_as_float(b.y); f[6] = __uint_as_float(b.z); f[7] = __uint_as_float(b.w);
     } else if constexpr (DT == WF_BF16) {
-        uint4 u = __ldg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(base) + elem_off));
+        uint4 u = ld16_chained(static_cast<const __nv_bfloat16*>(base) + elem_off);
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -110,7 +119,7 @@ __device__ __forceinline__ void load8(const void* base, int64_t elem_off, float 
             f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
         }
     } else {
-        uint4 u = __ldg(reinterpret_cast<const uint4*>(static_cast<const __half*>(base) + elem_off));
+        uint4 u = ld16_chained(static_cast<const __half*>(base) + elem_off);
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {

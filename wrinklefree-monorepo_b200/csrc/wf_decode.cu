@@ -129,11 +129,11 @@ struct XCache {
 template <int XDT>
 __device__ __forceinline__ void load8_raw(const void* base, int64_t elem_off, uint4 (&r)[XCache<XDT>::V]) {
     if constexpr (XDT == WF_F32) {
-        const uint4* q = reinterpret_cast<const uint4*>(static_cast<const float*>(base) + elem_off);
-        r[0] = __ldg(q);
-        r[1] = __ldg(q + 1);
+        const float* q = static_cast<const float*>(base) + elem_off;
+        r[0] = ld16_chained(q);
+        r[1] = ld16_chained(q + 4);
     } else {
-        r[0] = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(base) + elem_off));
+        r[0] = ld16_chained(static_cast<const uint16_t*>(base) + elem_off);
     }
 }
 template <int XDT>
@@ -241,7 +241,7 @@ __device__ __forceinline__ void quantize_phase(const wf_problem& p, const void* 
                     const int8_t* row = static_cast<const int8_t*>(x) + static_cast<int64_t>(m0 + tok) * p.ldx;
                     for (int k = lane_in * 16; k < Kp; k += tpt * 16) {
                         uint4 v = make_uint4(0, 0, 0, 0);
-                        if (k < K) v = __ldg(reinterpret_cast<const uint4*>(row + k));
+                        if (k < K) v = ld16_chained(row + k);
                         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {

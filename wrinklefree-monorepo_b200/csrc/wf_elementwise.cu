@@ -29,7 +29,7 @@ constexpr int NORM_CHUNKS = 4;  // 8-element chunks per thread held in registers
 // quantization kernel on the bf16 values (absmax, multiplier 127 / max rounded like torch's, round half to even): the
 // projections that follow read q and q_scale and no kernel stands between the norm and them; y may then be null.
 template <bool VEC>
-__global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(__nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ delta,
+__global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(__nv_bfloat16* __restrict__ h, const __nv_bfloat16* delta,
                                                                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                                                                    int K, float eps, int8_t* __restrict__ q, float* __restrict__ q_scale,
                                                                    float q_eps) {
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(__nv_bfloat16
             const int i = tid + c * NORM_THREADS;
             if (i < chunks) {
                 hv[c] = hrow[i];
-                if (delta) dv[c] = __ldg(reinterpret_cast<const uint4*>(delta + m * K) + i);
+                if (delta) dv[c] = ld16_chained(delta + m * K + 8 * static_cast<int64_t>(i));
             }
         }
 #pragma unroll
@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(__nv_bfloat16
 // rotated in place; key heads are rotated and written to kcache[b, head, slot, :], and the same block copies the
 // value head to vcache[b, head, slot, :].  cos/sin [T, D/2] fp32; the position *pos is read on the device
 // (the caller keeps it below T; it is reduced modulo T only so that a stray value stays inside the tables).
-__global__ void rope_kv_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
-                               const float* __restrict__ cosv, const float* __restrict__ sinv, const int64_t* __restrict__ pos,
+__global__ void rope_kv_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* k, const __nv_bfloat16* v,
+                               const float* __restrict__ cosv, const float* __restrict__ sinv, const int64_t* pos,
                                __nv_bfloat16* __restrict__ kcache, __nv_bfloat16* __restrict__ vcache, int nq, int nkv, int D, int T) {
     pdl_trigger();
     const int heads = nq + nkv, half = D / 2;
@@ -176,7 +176,7 @@ __device__ __forceinline__ float act_one(float a, int mode) {
     }
     return round_bf(t);
 }
-__global__ void __launch_bounds__(256) act_mul_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ u,
+__global__ void __launch_bounds__(256) act_mul_kernel(const __nv_bfloat16* g, const __nv_bfloat16* u,
                                                       __nv_bfloat16* __restrict__ out, int64_t n, int mode) {
     pdl_trigger();
     pdl_wait();
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(256) act_mul_kernel(const __nv_bfloat16* __res
     const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t n8 = n >> 3;
     for (int64_t i = tid; i < n8; i += stride) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(g) + i), b = __ldg(reinterpret_cast<const uint4*>(u) + i);
+        const uint4 a = ld16_chained(g + 8 * i), b = ld16_chained(u + 8 * i);
         const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
         uint32_t o[4];
 #pragma unroll
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(256) act_mul_kernel(const __nv_bfloat16* __res
 // the activation in front of down_proj together with the quantization that projection would otherwise run itself.
 constexpr int AMQ_THREADS = 512;
 constexpr int AMQ_CHUNKS = 4;  // rows up to 16384 elements
-__global__ void __launch_bounds__(AMQ_THREADS) act_mul_quant_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ u,
+__global__ void __launch_bounds__(AMQ_THREADS) act_mul_quant_kernel(const __nv_bfloat16* g, const __nv_bfloat16* u,
                                                                     __nv_bfloat16* __restrict__ out, int8_t* __restrict__ q,
                                                                     float* __restrict__ q_scale, int I, int mode, float q_eps) {
     __shared__ float sh[AMQ_THREADS / 32];
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(AMQ_THREADS) act_mul_quant_kernel(const __nv_b
     for (int c = 0; c < AMQ_CHUNKS; ++c) {
         const int i = tid + c * AMQ_THREADS;
         if (i < chunks) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(g + m * I) + i), b = __ldg(reinterpret_cast<const uint4*>(u + m * I) + i);
+            const uint4 a = ld16_chained(g + m * I + 8 * i), b = ld16_chained(u + m * I + 8 * i);
             const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {

@@ -164,6 +164,30 @@ def test_act_quant_many_tokens(wf, k, dt):
 
 
 # ---------------------------------------------------------------- contraction
+@pytest.mark.parametrize("m,k", [(1, 8), (288, 8), (287, 768), (300, 776), (1153, 1536), (3201, 2560), (9, 2568), (5, 8200), (3, 14336), (2, 14344)])
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+def test_act_quant_every_split_of_a_row(wf, m, k, dt):
+    """A warp per token, a block with the row in 2, 4 or 7 chunks per thread, a row read twice; among the tokens rows of
+    zeros, of values so small that the f16 multiplier overflows, on rounding boundaries, with an infinity and with a NaN.
+    Codes, multipliers and row sums are exact: no tolerance."""
+    rng = np.random.default_rng(m * 131 + k)
+    x = rng.standard_normal((m, k)).astype(np.float32) * (10.0 ** rng.uniform(-4, 3, (m, 1))).astype(np.float32)
+    x[m // 2] = rng.integers(-254, 255, k) / 2.0
+    if m > 4:
+        x[0], x[1], x[2, k // 2], x[3, -1] = 0.0, x[1] * 1e-6, np.inf, np.nan
+    xd = torch.from_numpy(x).to(TDT[dt])
+    q, s, r = wf.act_quant_i8(xd.to(DEV), want_rowsum=True)
+    good = [i for i in range(m) if np.isfinite(xd[i].float().numpy()).all()]
+    with np.errstate(all="ignore"):
+        qo, so = O.act_quant_per_token(xd.float().numpy()[good], dt)
+    finite = np.isfinite(so.reshape(-1))  # an infinite multiplier: 0 * inf is no number, which counts as 0
+    rows = np.asarray(good)[finite]
+    assert np.array_equal(q.cpu().numpy()[rows], qo[finite]) and np.array_equal(s.cpu().numpy()[good], so.reshape(-1))
+    v = xd.to(DEV) * s.to(TDT[dt]).unsqueeze(1)  # the formula itself, for every row
+    want = torch.nan_to_num(v.float(), nan=0.0).round().clamp(-128, 127).to(torch.int8)
+    assert torch.equal(q, want) and torch.equal(r, want.sum(-1, dtype=torch.int32))
+
+
 @pytest.mark.parametrize("name", list(gi.CASES))
 @pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
 def test_decode_against_golden(wf, name, dt):

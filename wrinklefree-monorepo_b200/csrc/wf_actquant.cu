@@ -32,20 +32,10 @@ __device__ __forceinline__ int block_sum_int(int v, int* sh) {
     return t;
 }
 
-// One block per token.  K % 8 == 0.
+// One token quantized by one block; x is read twice.  K % 8 == 0.
 template <int DT>
-__global__ void __launch_bounds__(AQ_THREADS)
-    act_quant_token_kernel(const void* x, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q,
-                           float* __restrict__ scale, int32_t* __restrict__ rowsum, int x_ready) {
-    __shared__ float shf[AQ_THREADS / 32];
-    __shared__ int shi[AQ_THREADS / 32];
-    // chained with a programmatic dependency: the next kernel may start (the contraction fetches its first weights
-    // meanwhile); x may come from the previous kernel and q may still be read by it, so everything else waits for it
-    // -- unless the caller states that neither is the case (x_ready): then only the end of the grid waits, so that
-    // whoever waits for this grid may still rely on everything ahead of it in the stream
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    if (!x_ready) asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    const int64_t m = blockIdx.x;
+__device__ __forceinline__ void quant_token(const void* x, int64_t m, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q,
+                                            float* __restrict__ scale, int32_t* __restrict__ rowsum, float* shf, int* shi) {
     float mx = 0.f;
     for (int64_t k = threadIdx.x * 8; k < K; k += AQ_THREADS * 8) {
         float f[8];
@@ -69,11 +59,26 @@ __global__ void __launch_bounds__(AQ_THREADS)
         }
         *reinterpret_cast<uint2*>(q + m * K + k) = make_uint2(w0, w1);
     }
-    sum = block_sum_int(sum, shi);
+    if (rowsum) sum = block_sum_int(sum, shi);
     if (threadIdx.x == 0) {
         scale[m] = s;
         if (rowsum) rowsum[m] = sum;
     }
+}
+
+template <int DT>
+__global__ void __launch_bounds__(AQ_THREADS)
+    act_quant_token_kernel(const void* x, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q,
+                           float* __restrict__ scale, int32_t* __restrict__ rowsum, int x_ready) {
+    __shared__ float shf[AQ_THREADS / 32];
+    __shared__ int shi[AQ_THREADS / 32];
+    // chained with a programmatic dependency: the next kernel may start (the contraction fetches its first weights
+    // meanwhile); x may come from the previous kernel and q may still be read by it, so everything else waits for it
+    // -- unless the caller states that neither is the case (x_ready): then only the end of the grid waits, so that
+    // whoever waits for this grid may still rely on everything ahead of it in the stream
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    if (!x_ready) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    quant_token<DT>(x, blockIdx.x, K, ldx, eps, q, scale, rowsum, shf, shi);
     // one block stays until the predecessor has completed, so that this grid does not end before it; the others leave
     if (x_ready && blockIdx.x == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
@@ -129,8 +134,179 @@ using namespace wf;
 static int act_quant_impl(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, int mode, float eps, int8_t* q, float* scale,
                           int32_t* rowsum, int x_ready, void* stream);
 
-// The same with the row held in registers between the two passes (K <= 8 * AQ_THREADS * CHUNKS): x is read once, and all
-// of a thread's loads are in flight together.
+// 8 consecutive elements as they lie in memory (zeros when !ok), and their values
+template <int DT>
+struct Raw8 {
+    static constexpr int V = DT == WF_F32 ? 2 : 1;
+    uint4 v[V];
+};
+template <int DT>
+__device__ __forceinline__ void load_raw8(const void* base, int64_t elem_off, bool ok, Raw8<DT>& r) {
+    const char* p = static_cast<const char*>(base) + elem_off * (DT == WF_F32 ? 4 : 2);
+#pragma unroll
+    for (int j = 0; j < Raw8<DT>::V; ++j)  // predicated and not branched around: a thread's loads go out back to back
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.b32 p, %5, 0;\n mov.u32 %0, 0;\n mov.u32 %1, 0;\n mov.u32 %2, 0;\n mov.u32 %3, 0;\n"
+            " @p ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n}\n"
+            : "=&r"(r.v[j].x), "=&r"(r.v[j].y), "=&r"(r.v[j].z), "=&r"(r.v[j].w)
+            : "l"(p + 16 * j), "r"(static_cast<int>(ok))
+            : "memory");
+}
+template <int DT>
+__device__ __forceinline__ void values8(const Raw8<DT>& r, float (&f)[8]) {
+    if constexpr (DT == WF_F32) {
+        f[0] = __uint_as_float(r.v[0].x); f[1] = __uint_as_float(r.v[0].y); f[2] = __uint_as_float(r.v[0].z); f[3] = __uint_as_float(r.v[0].w);
+        f[4] = __uint_as_float(r.v[1].x); f[5] = __uint_as_float(r.v[1].y); f[6] = __uint_as_float(r.v[1].z); f[7] = __uint_as_float(r.v[1].w);
+    } else {
+        const uint32_t w[4] = {r.v[0].x, r.v[0].y, r.v[0].z, r.v[0].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if constexpr (DT == WF_BF16) {
+                f[2 * i] = __uint_as_float(w[i] << 16);
+                f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+            } else {
+                const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                f[2 * i] = v.x;
+                f[2 * i + 1] = v.y;
+            }
+        }
+    }
+}
+
+// ---- the quantization of a row that is held as Raw8, at about four instructions per element (it was fourteen, one of them
+// the quarter-rate conversion to int, and bound the kernel at 58 % of the copy bandwidth):
+//   * the absolute maximum over bit patterns (non-negative values order like theirs), two 16-bit elements at a time;
+//   * the product with the multiplier as one packed multiplication, which rounds once like the fp32 product of two 16-bit
+//     values (exact) rounded to the type;
+//   * the rounding to an integer as an addition of 1.5 * 2^23 (half to even), whose lowest byte is the int8.  |x * s| stays
+//     below 128.5 (three roundings of at most 2^-9 on top of 127), so only the upper bound of the clamp is needed.
+// A row with an infinity or a NaN, and a multiplier that is not finite, take quantize_one instead.
+template <int DT>
+__device__ __forceinline__ uint32_t max_bits8(const Raw8<DT>& r, uint32_t mx) {
+#pragma unroll
+    for (int j = 0; j < Raw8<DT>::V; ++j) {
+        const uint32_t w[4] = {r.v[j].x, r.v[j].y, r.v[j].z, r.v[j].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mx = DT == WF_F32 ? max(mx, w[i] & 0x7fffffffu) : __vmaxu2(mx, w[i] & 0x7fff7fffu);
+    }
+    return mx;
+}
+// over the warp, as one bit pattern of the type
+template <int DT>
+__device__ __forceinline__ uint32_t warp_max_bits(uint32_t mx) {
+    if constexpr (DT != WF_F32) mx = max(mx & 0xffffu, mx >> 16);
+    return __reduce_max_sync(0xffffffffu, mx);
+}
+template <int DT>
+__device__ __forceinline__ bool finite_bits(uint32_t bits) {
+    return bits < (DT == WF_F32 ? 0x7f800000u : (DT == WF_BF16 ? 0x7f80u : 0x7c00u));
+}
+template <int DT>
+__device__ __forceinline__ float bits_value(uint32_t bits) {
+    if constexpr (DT == WF_F32) return __uint_as_float(bits);
+    if constexpr (DT == WF_BF16) return __uint_as_float(bits << 16);
+    return __half2float(__ushort_as_half(static_cast<unsigned short>(bits)));
+}
+constexpr float RINT_MAGIC = 12582912.0f;  // 1.5 * 2^23
+// two values (already rounded products, at most 127) to two bytes in the low half
+__device__ __forceinline__ uint32_t two_bytes(float a, float b) {
+    return __byte_perm(__float_as_uint(__fadd_rn(a, RINT_MAGIC)), __float_as_uint(__fadd_rn(b, RINT_MAGIC)), 0x0040);
+}
+template <int DT>
+__device__ __forceinline__ uint2 quantize8_fast(const Raw8<DT>& r, float s) {
+    uint32_t h[4];  // pairs of bytes
+    if constexpr (DT == WF_F32) {
+        float f[8];
+        values8<DT>(r, f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) h[i] = two_bytes(fminf(__fmul_rn(f[2 * i], s), 127.f), fminf(__fmul_rn(f[2 * i + 1], s), 127.f));
+    } else {
+        const uint32_t w[4] = {r.v[0].x, r.v[0].y, r.v[0].z, r.v[0].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if constexpr (DT == WF_BF16) {
+                const __nv_bfloat162 v = __hmin2(__hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&w[i]), __float2bfloat162_rn(s)), __float2bfloat162_rn(127.f));
+                const uint32_t u = *reinterpret_cast<const uint32_t*>(&v);
+                h[i] = two_bytes(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+            } else {
+                const float2 v = __half22float2(__hmin2(__hmul2_rn(*reinterpret_cast<const __half2*>(&w[i]), __float2half2_rn(s)), __float2half2_rn(127.f)));
+                h[i] = two_bytes(v.x, v.y);
+            }
+        }
+    }
+    return make_uint2(__byte_perm(h[0], h[1], 0x5410), __byte_perm(h[2], h[3], 0x5410));
+}
+template <int DT>
+__device__ __noinline__ uint2 quantize8_any(const Raw8<DT> r, float s) {
+    float f[8];
+    values8<DT>(r, f);
+    uint32_t w[2] = {0, 0};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) w[e >> 2] |= static_cast<uint32_t>(quantize_one<DT>(f[e], s) & 0xff) << (8 * (e & 3));
+    return make_uint2(w[0], w[1]);
+}
+template <int DT>
+__device__ __forceinline__ float max_abs8(const Raw8<DT>& r, float mx) {  // a NaN counts for nothing
+    float f[8];
+    values8<DT>(r, f);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) mx = fmaxf(mx, fabsf(f[e]));
+    return mx;
+}
+__device__ __forceinline__ int sum_bytes(uint2 w, int sum) {
+    return __dp4a(static_cast<int>(w.x), 0x01010101, __dp4a(static_cast<int>(w.y), 0x01010101, sum));
+}
+
+// One token quantized by one block, the row held in registers between the two passes (K <= 8 * AQ_THREADS * CHUNKS): x is
+// read once, and all of a thread's loads are in flight together.
+template <int DT, int CHUNKS>
+__device__ __forceinline__ void quant_token_reg(const void* x, int64_t m, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q,
+                                                float* __restrict__ scale, int32_t* __restrict__ rowsum, float* shf, int* shi) {
+    const int chunks = static_cast<int>(K >> 3);
+    Raw8<DT> r[CHUNKS];
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+        const int i = threadIdx.x + c * AQ_THREADS;
+        load_raw8<DT>(x, m * ldx + 8 * static_cast<int64_t>(i), i < chunks, r[c]);
+    }
+    uint32_t bits = 0;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) bits = max_bits8<DT>(r[c], bits);
+    bits = warp_max_bits<DT>(bits);
+    if ((threadIdx.x & 31) == 0) shi[threadIdx.x >> 5] = static_cast<int>(bits);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < AQ_THREADS / 32; ++i) bits = max(bits, static_cast<uint32_t>(shi[i]));
+    bool fast = finite_bits<DT>(bits);
+    float mx = bits_value<DT>(bits);
+    if (!fast) {  // uniform over the block
+        mx = 0.f;
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) mx = max_abs8<DT>(r[c], mx);
+        mx = block_max(mx, shf);
+    }
+    const float s = act_scale_from_absmax<DT>(mx, eps);
+    fast = fast && s < INFINITY;
+    int sum = 0;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+        const int i = threadIdx.x + c * AQ_THREADS;
+        if (i < chunks) {
+            const uint2 w = fast ? quantize8_fast<DT>(r[c], s) : quantize8_any<DT>(r[c], s);
+            sum = sum_bytes(w, sum);
+            *reinterpret_cast<uint2*>(q + m * K + 8 * static_cast<int64_t>(i)) = w;
+        }
+    }
+    if (rowsum) {
+        __syncthreads();  // shi has been read
+        sum = block_sum_int(sum, shi);
+    }
+    if (threadIdx.x == 0) {
+        scale[m] = s;
+        if (rowsum) rowsum[m] = sum;
+    }
+}
+
 template <int DT, int CHUNKS>
 __global__ void __launch_bounds__(AQ_THREADS)
     act_quant_token_reg_kernel(const void* x, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q,
@@ -139,57 +315,144 @@ __global__ void __launch_bounds__(AQ_THREADS)
     __shared__ int shi[AQ_THREADS / 32];
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     if (!x_ready) asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    const int64_t m = blockIdx.x;
-    const int chunks = static_cast<int>(K >> 3);
-    float f[CHUNKS][8];
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) {
-        const int i = threadIdx.x + c * AQ_THREADS;
-        if (i < chunks) {
-            load8<DT>(x, m * ldx + 8 * static_cast<int64_t>(i), f[c]);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[c][e] = 0.f;
-        }
-    }
-    float mx = 0.f;
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) mx = fmaxf(mx, fabsf(f[c][e]));
-    mx = block_max(mx, shf);
-    const float s = act_scale_from_absmax<DT>(mx, eps);
-    int sum = 0;
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) {
-        const int i = threadIdx.x + c * AQ_THREADS;
-        if (i < chunks) {
-            uint32_t w0 = 0, w1 = 0;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int a = quantize_one<DT>(f[c][e], s), b = quantize_one<DT>(f[c][4 + e], s);
-                sum += a + b;
-                w0 |= static_cast<uint32_t>(a & 0xff) << (8 * e);
-                w1 |= static_cast<uint32_t>(b & 0xff) << (8 * e);
-            }
-            *reinterpret_cast<uint2*>(q + m * K + 8 * static_cast<int64_t>(i)) = make_uint2(w0, w1);
-        }
-    }
-    sum = block_sum_int(sum, shi);
-    if (threadIdx.x == 0) {
-        scale[m] = s;
-        if (rowsum) rowsum[m] = sum;
-    }
+    quant_token_reg<DT, CHUNKS>(x, blockIdx.x, K, ldx, eps, q, scale, rowsum, shf, shi);
     // one block stays until the predecessor has completed, so that this grid does not end before it; the others leave
     if (x_ready && blockIdx.x == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
+// Chunks of 8 per lane where one warp per token is the better split, else 0.  A block per token spends most of a short row on
+// its barrier and leaves threads without a chunk; a warp per token has neither, but takes its time for the row serially, so it
+// needs enough tokens to fill the chip: the two cross between 300 tokens of 576 values and 3000 of 2560 (8192 tokens: 4.0
+// against 11.1 us at K = 576, 8.4 against 13.9 at 2560; 22 against 19 at 4096; 1920 tokens of 2560: 5.0 against 4.4).
+static int warp_form_chunks(int64_t M, int64_t K) {
+    const int64_t per_lane = ((K >> 3) + 31) / 32;
+    return per_lane <= 10 && M >= 32 * per_lane * per_lane ? static_cast<int>(per_lane) : 0;
+}
+
+// One token quantized by one warp (K <= 256 * NCH): no barrier between the two passes, and NCH loads of a lane in flight.
+template <int DT, int NCH>
+__device__ __forceinline__ void quant_token_warp(const void* x, int64_t m, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q,
+                                                 float* __restrict__ scale, int32_t* __restrict__ rowsum) {
+    const int chunks = static_cast<int>(K >> 3), lane = threadIdx.x & 31;
+    Raw8<DT> r[NCH];
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) load_raw8<DT>(x, m * ldx + 8 * static_cast<int64_t>(lane + 32 * c), lane + 32 * c < chunks, r[c]);
+    uint32_t bits = 0;
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) bits = max_bits8<DT>(r[c], bits);
+    bits = warp_max_bits<DT>(bits);
+    bool fast = finite_bits<DT>(bits);
+    float mx = bits_value<DT>(bits);
+    if (!fast) {  // uniform over the warp
+        mx = 0.f;
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) mx = max_abs8<DT>(r[c], mx);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    const float s = act_scale_from_absmax<DT>(mx, eps);
+    fast = fast && s < INFINITY;
+    int sum = 0;
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) {
+        const int i = lane + 32 * c;
+        if (i < chunks) {
+            const uint2 w = fast ? quantize8_fast<DT>(r[c], s) : quantize8_any<DT>(r[c], s);
+            sum = sum_bytes(w, sum);
+            *reinterpret_cast<uint2*>(q + m * K + 8 * static_cast<int64_t>(i)) = w;
+        }
+    }
+    if (rowsum) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    }
+    if (lane == 0) {
+        scale[m] = s;
+        if (rowsum) rowsum[m] = sum;
+    }
+}
+
+template <int DT, int NCH>
+__global__ void __launch_bounds__(AQ_THREADS)
+    act_quant_warp_kernel(const void* x, int M, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q, float* __restrict__ scale,
+                          int32_t* __restrict__ rowsum, int x_ready) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    if (!x_ready) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    const int m = blockIdx.x * (AQ_THREADS / 32) + (threadIdx.x >> 5);
+    if (m < M) quant_token_warp<DT, NCH>(x, m, K, ldx, eps, q, scale, rowsum);
+    if (x_ready && blockIdx.x == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
+// ---- what the contraction for many tokens needs in front of it, in one launch: every weight as one signed byte, and the
+// quantized tokens.  Both are bound by memory and neither fills the chip alone for a thousand tokens, so they share it.
+
+// byte-wise code - 1 of four codes: the borrow of a byte never leaves it, its top bit is set first
+__device__ __forceinline__ uint32_t codes_to_s8(uint32_t v) { return ((v | 0x80808080u) - 0x01010101u) ^ 0x80808080u; }
+
+// Packed word i (16 codes) of an [N, K/4] matrix to int8 [N, K]; a warp reads 128 bytes and writes 512.
+__device__ __forceinline__ void expand_word(uint32_t w, int64_t i, int layout, int8_t* __restrict__ w8) {
+    const uint32_t m = 0x03030303u;
+    if (layout == WF_LAYOUT_WF16) {  // bit pairs j of the four bytes: weights 16 i + 4 j .. + 3
+        *reinterpret_cast<uint4*>(w8 + 16 * i) =
+            make_uint4(codes_to_s8(w & m), codes_to_s8((w >> 2) & m), codes_to_s8((w >> 4) & m), codes_to_s8((w >> 6) & m));
+    } else {  // I2_S: byte b of a block of 32 holds weights b, b + 32, b + 64, b + 96 at bits 7:6, 5:4, 3:2, 1:0
+        int8_t* d = w8 + (i >> 3) * 128 + (i & 7) * 4;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) *reinterpret_cast<uint32_t*>(d + 32 * g) = codes_to_s8((w >> (6 - 2 * g)) & m);
+    }
+}
+
+// Blocks 0 .. expand_blocks - 1 expand the weights, the others quantize: one token each, the row in CHUNKS chunks per thread
+// or read twice (0), or one token per warp of -CHUNKS chunks per lane.  DT = WF_I8: the tokens are int8 already and every
+// block expands.
+template <int DT, int CHUNKS>
+__global__ void __launch_bounds__(AQ_THREADS)
+    quantize_expand_kernel(const void* x, int M, int64_t K, int64_t ldx, float eps, int8_t* __restrict__ q, float* __restrict__ scale,
+                           const uint32_t* codes, int layout, int64_t words, int8_t* __restrict__ w8, int expand_blocks) {
+    __shared__ float shf[AQ_THREADS / 32];
+    __shared__ int shi[AQ_THREADS / 32];
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // x, and the workspace that the previous call may still read
+    if (static_cast<int>(blockIdx.x) < expand_blocks) {
+        constexpr int U = 4;  // words in flight per thread
+        const int64_t stride = static_cast<int64_t>(expand_blocks) * AQ_THREADS;
+        for (int64_t i = static_cast<int64_t>(blockIdx.x) * AQ_THREADS + threadIdx.x; i < words; i += U * stride) {
+            uint32_t w[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i + u * stride < words) w[u] = codes[i + u * stride];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i + u * stride < words) expand_word(w[u], i + u * stride, layout, w8);
+        }
+    } else if constexpr (DT != WF_I8) {
+        const int64_t m = static_cast<int64_t>(blockIdx.x) - expand_blocks;
+        if constexpr (CHUNKS > 0) {
+            quant_token_reg<DT, CHUNKS>(x, m, K, ldx, eps, q, scale, nullptr, shf, shi);
+        } else if constexpr (CHUNKS < 0) {
+            const int64_t tok = m * (AQ_THREADS / 32) + (threadIdx.x >> 5);
+            if (tok < M) quant_token_warp<DT, -CHUNKS>(x, tok, K, ldx, eps, q, scale, nullptr);
+        } else {
+            quant_token<DT>(x, m, K, ldx, eps, q, scale, nullptr, shf, shi);
+        }
+    }
+}
+
 template <int DT>
-static cudaError_t launch_token_quant(const cudaLaunchConfig_t& lc, const void* x, int64_t K, int64_t ldx, float eps, int8_t* q,
+static cudaError_t launch_token_quant(cudaLaunchConfig_t& lc, const void* x, int64_t M, int64_t K, int64_t ldx, float eps, int8_t* q,
                                       float* scale, int32_t* rowsum, int x_ready) {
+    const int per_lane = warp_form_chunks(M, K);
+    if (per_lane) {
+        lc.gridDim = dim3(static_cast<unsigned>((M + AQ_THREADS / 32 - 1) / (AQ_THREADS / 32)));
+        const int mm = static_cast<int>(M);
+        if (per_lane <= 3) return cudaLaunchKernelEx(&lc, act_quant_warp_kernel<DT, 3>, x, mm, K, ldx, eps, q, scale, rowsum, x_ready);
+        if (per_lane <= 6) return cudaLaunchKernelEx(&lc, act_quant_warp_kernel<DT, 6>, x, mm, K, ldx, eps, q, scale, rowsum, x_ready);
+        return cudaLaunchKernelEx(&lc, act_quant_warp_kernel<DT, 10>, x, mm, K, ldx, eps, q, scale, rowsum, x_ready);
+    }
     const int64_t per_thread = ((K >> 3) + AQ_THREADS - 1) / AQ_THREADS;
     if (per_thread <= 2) return cudaLaunchKernelEx(&lc, act_quant_token_reg_kernel<DT, 2>, x, K, ldx, eps, q, scale, rowsum, x_ready);
     if (per_thread <= 4) return cudaLaunchKernelEx(&lc, act_quant_token_reg_kernel<DT, 4>, x, K, ldx, eps, q, scale, rowsum, x_ready);
+    if (per_thread <= 7) return cudaLaunchKernelEx(&lc, act_quant_token_reg_kernel<DT, 7>, x, K, ldx, eps, q, scale, rowsum, x_ready);
     return cudaLaunchKernelEx(&lc, act_quant_token_kernel<DT>, x, K, ldx, eps, q, scale, rowsum, x_ready);
 }
 
@@ -203,6 +466,55 @@ extern "C" int wf_act_quant_i8(const void* x, int x_dtype, int64_t M, int64_t K,
 int wf_act_quant_token_ready(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, float eps, int8_t* q, float* scale,
                              int32_t* rowsum, int x_ready, void* stream) {
     return act_quant_impl(x, x_dtype, M, K, ldx, WF_ACT_PER_TOKEN, eps, q, scale, rowsum, x_ready, stream);
+}
+
+template <int DT>
+static cudaError_t launch_quantize_expand(cudaLaunchConfig_t& lc, const void* x, int64_t M, int64_t K, int64_t ldx, float eps, int8_t* q,
+                                          float* scale, const uint32_t* codes, int layout, int64_t words, int8_t* w8) {
+    // four words per thread and pass; at most eight blocks per SM, so that the first tokens start beside them
+    const int64_t most = 8 * static_cast<int64_t>(num_sms()), want = (words + 4 * AQ_THREADS - 1) / (4 * AQ_THREADS);
+    const int blocks = static_cast<int>(want < most ? want : most);
+    const int mm = static_cast<int>(M);
+    lc.gridDim = dim3(static_cast<unsigned>(blocks + (DT == WF_I8 ? 0 : M)));
+    if constexpr (DT == WF_I8) {
+        return cudaLaunchKernelEx(&lc, quantize_expand_kernel<DT, 0>, x, mm, K, ldx, eps, q, scale, codes, layout, words, w8, blocks);
+    } else {
+        const int per_lane = warp_form_chunks(M, K);
+        if (per_lane) {
+            lc.gridDim = dim3(static_cast<unsigned>(blocks + (M + AQ_THREADS / 32 - 1) / (AQ_THREADS / 32)));
+            if (per_lane <= 3) return cudaLaunchKernelEx(&lc, quantize_expand_kernel<DT, -3>, x, mm, K, ldx, eps, q, scale, codes, layout, words, w8, blocks);
+            if (per_lane <= 6) return cudaLaunchKernelEx(&lc, quantize_expand_kernel<DT, -6>, x, mm, K, ldx, eps, q, scale, codes, layout, words, w8, blocks);
+            return cudaLaunchKernelEx(&lc, quantize_expand_kernel<DT, -10>, x, mm, K, ldx, eps, q, scale, codes, layout, words, w8, blocks);
+        }
+        const int64_t per_thread = ((K >> 3) + AQ_THREADS - 1) / AQ_THREADS;
+        if (per_thread <= 2) return cudaLaunchKernelEx(&lc, quantize_expand_kernel<DT, 2>, x, mm, K, ldx, eps, q, scale, codes, layout, words, w8, blocks);
+        if (per_thread <= 4) return cudaLaunchKernelEx(&lc, quantize_expand_kernel<DT, 4>, x, mm, K, ldx, eps, q, scale, codes, layout, words, w8, blocks);
+        if (per_thread <= 7) return cudaLaunchKernelEx(&lc, quantize_expand_kernel<DT, 7>, x, mm, K, ldx, eps, q, scale, codes, layout, words, w8, blocks);
+        return cudaLaunchKernelEx(&lc, quantize_expand_kernel<DT, 0>, x, mm, K, ldx, eps, q, scale, codes, layout, words, w8, blocks);
+    }
+}
+
+// The launch in front of the contraction for many tokens: w8 [N, K] int8 from the packed weights and, unless x is int8
+// already, q [M, K] and scale [M] (the bits of wf_act_quant_i8 per token).  Arguments as checked by wf_bitlinear_prefill.
+int wf_quantize_expand(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, float eps, int8_t* q, float* scale, const uint8_t* codes,
+                       int layout, int64_t N, int8_t* w8, void* stream) {
+    cudaLaunchConfig_t lc = {};
+    lc.blockDim = dim3(AQ_THREADS);
+    lc.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(codes);
+    const int64_t n = N * (K / 16);
+    switch (x_dtype) {
+        case WF_F32: WF_CUDA(launch_quantize_expand<WF_F32>(lc, x, M, K, ldx, eps, q, scale, words, layout, n, w8)); break;
+        case WF_BF16: WF_CUDA(launch_quantize_expand<WF_BF16>(lc, x, M, K, ldx, eps, q, scale, words, layout, n, w8)); break;
+        case WF_F16: WF_CUDA(launch_quantize_expand<WF_F16>(lc, x, M, K, ldx, eps, q, scale, words, layout, n, w8)); break;
+        default: WF_CUDA(launch_quantize_expand<WF_I8>(lc, x, M, K, ldx, eps, q, scale, words, layout, n, w8)); break;
+    }
+    return WF_OK;
 }
 
 static int act_quant_impl(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, int mode, float eps, int8_t* q, float* scale,
@@ -228,9 +540,9 @@ static int act_quant_impl(const void* x, int x_dtype, int64_t M, int64_t K, int6
         lc.attrs = attr;
         lc.numAttrs = 1;
         switch (x_dtype) {
-            case WF_F32: WF_CUDA(launch_token_quant<WF_F32>(lc, x, K, ldx, eps, q, scale, rowsum, x_ready)); break;
-            case WF_BF16: WF_CUDA(launch_token_quant<WF_BF16>(lc, x, K, ldx, eps, q, scale, rowsum, x_ready)); break;
-            default: WF_CUDA(launch_token_quant<WF_F16>(lc, x, K, ldx, eps, q, scale, rowsum, x_ready)); break;
+            case WF_F32: WF_CUDA(launch_token_quant<WF_F32>(lc, x, M, K, ldx, eps, q, scale, rowsum, x_ready)); break;
+            case WF_BF16: WF_CUDA(launch_token_quant<WF_BF16>(lc, x, M, K, ldx, eps, q, scale, rowsum, x_ready)); break;
+            default: WF_CUDA(launch_token_quant<WF_F16>(lc, x, M, K, ldx, eps, q, scale, rowsum, x_ready)); break;
         }
     } else if (mode == WF_ACT_PER_TENSOR) {
         WF_REQUIRE(x_dtype == WF_F32, "wf_act_quant_i8: per-tensor mode takes fp32 input (as the operator it replaces)");

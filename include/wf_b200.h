@@ -277,7 +277,11 @@ int wf_bitlinear_decode_grouped(const wf_problem* dev_problems, const wf_problem
  * Synchronizes the device. */
 int wf_device_status(void);
 
+/* wf_prefill_workspace_bytes: what every call below needs.  wf_prefill_workspace_bytes_for: with this much,
+ * wf_bitlinear_prefill may run the form for many tokens, which expands the weights of the call to one byte each behind the
+ * quantized tokens; for sizes where that form does not pay it is the same number.  Results are the same bits. */
 size_t wf_prefill_workspace_bytes(int64_t M, int64_t K);
+size_t wf_prefill_workspace_bytes_for(int64_t M, int64_t N, int64_t K);
 int wf_bitlinear_prefill(const void* x, int x_dtype, int64_t ldx, const float* x_scale, const uint8_t* codes,
                          int layout, const float* w_scale, float w_scale_host, const void* bias, int bias_dtype,
                          void* y, int y_dtype, int64_t ldy, int32_t* acc_out, int64_t M, int64_t N, int64_t K,

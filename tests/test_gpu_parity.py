@@ -745,3 +745,38 @@ def test_contraction_forms_on_a_long_stack(wf, m):
     wf.device_status()
     for i in picks:
         assert torch.equal(ref[i], y[i]), i
+
+
+@pytest.mark.parametrize("m,n,k", [(65, 8, 64), (255, 264, 192), (257, 513, 256), (300, 1000, 256), (1024, 257, 576), (120, 4104, 128),
+                                   (1024, 1537, 576), (1100, 2050, 8256), (1021, 4605, 512)])
+def test_contraction_for_many_tokens_bit_exact(wf, oracle_c, m, n, k):
+    """The form that expands the weights once per call and multiplies tiles of 256 tokens: edges of token and weight tiles,
+    remainders of the 256-wide K stages, rows of y that TMA can and cannot write, every type, both layouts, a bias,
+    strided int8 input.  Integers and the fp32 rescale are exact: no tolerance."""
+    L, lib = wf._lib, wf._lib.lib()
+    assert lib.wf_prefill_workspace_bytes_for(m, n, k) > lib.wf_prefill_workspace_bytes(m, k)  # this form is the one chosen
+    rng = np.random.default_rng(m * 7919 + n * 31 + k)
+    t = rng.integers(-1, 2, size=(n, k)).astype(np.int8)
+    x = gi.with_outliers(torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)), seed=m + n + k)
+    bias = torch.from_numpy(rng.standard_normal(n).astype(np.float32))
+    codes = wf.pack_codes(torch.from_numpy(t).to(DEV))
+    for dt in ("bf16", "f16", "f32"):
+        xd = x.to(TDT[dt])
+        q, s = O.act_quant_per_token(xd.float().numpy(), dt)
+        acc = oracle_c.int_gemm(q, t)
+        y = torch.from_numpy(oracle_c.rescale(acc, s.reshape(-1), 0.0173))
+        got = wf.bitlinear(xd.to(DEV), codes, 0.0173, out_dtype=torch.float32, path="prefill")
+        assert torch.equal(got.cpu(), y), dt
+        got = wf.bitlinear(xd.to(DEV), codes, 0.0173, bias=bias.to(DEV), path="prefill")
+        assert torch.equal(got.cpu(), (y + bias).to(TDT[dt])), dt
+        if k % 128 == 0:
+            i2s = wf.pack_codes(torch.from_numpy(t).to(DEV), L.LAYOUT_I2S)
+            assert torch.equal(wf.bitlinear(xd.to(DEV), i2s, 0.0173, layout=L.LAYOUT_I2S, path="prefill").cpu(), y.to(TDT[dt])), dt
+    rows = torch.zeros(m, k + 64, dtype=torch.int8, device=DEV)
+    rows[:, :k] = torch.from_numpy(q).to(DEV)
+    got = wf.bitlinear(rows[:, :k], codes, 0.0173, x_scale=torch.from_numpy(s.reshape(-1)).to(DEV), path="prefill")
+    assert torch.equal(got.cpu(), y)
+    out = torch.full((m, n + 3), 7.0, device=DEV)  # a row stride of its own: nothing beyond a row is written
+    wf.bitlinear(x.to(DEV), codes, 0.0173, out=out[:, :n], path="prefill")
+    assert bool((out[:, n:] == 7.0).all())
+    wf.device_status()

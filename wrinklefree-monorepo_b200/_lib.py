@@ -70,6 +70,7 @@ _SIGNATURES = {
     "wf_bitlinear_decode_grouped": (_int, [_p, _p, _int, _u32, _p]),
     "wf_device_status": (_int, []),
     "wf_prefill_workspace_bytes": (_sz, [_i64, _i64]),
+    "wf_prefill_workspace_bytes_for": (_sz, [_i64, _i64, _i64]),
     "wf_bitlinear_prefill": (_int, [_p, _int, _i64, _p, _p, _int, _p, _f32, _p, _int, _p, _int, _i64, _p, _i64, _i64, _i64,
                                     _f32, _p, _sz, _u32, _p]),
     "wf_add_rmsnorm_bf16": (_int, [_p, _p, _p, _p, _i64, _i64, _f32, _u32, _p]),

@@ -18,8 +18,6 @@
 //   * warps 10-13 (and 15-18): epilogue, thread = weight row: tcgen05.ld (summing the partial accumulators), integer
 //     correction, fp32 rescale, store.
 // Every mbarrier wait is bounded.
-#include <cuda.h>
-
 #include "wf_common.cuh"
 
 namespace wf {
@@ -27,6 +25,7 @@ __device__ int g_prefill_status = 0;
 }
 #define WF_STATUS_WORD ::wf::g_prefill_status
 #include "wf_async.cuh"
+#include "wf_tc.cuh"
 
 int wf_check_linear_args(const char* who, const void* x, int x_dtype, int64_t ldx, const float* x_scale, const uint8_t* codes,
                          int layout, const void* bias, int bias_dtype, void* y, int y_dtype, int64_t ldy, int64_t M, int64_t N,
@@ -53,21 +52,8 @@ struct PrefillParams {
                           // one: no load or store waits for them, only the end of the grid does
 };
 
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// K-major operand tile with 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((addr & 0x3FFFF) >> 4);  // start address
-    d |= static_cast<uint64_t>(1024 >> 4) << 32;        // stride between 8-row groups
-    d |= static_cast<uint64_t>(1) << 46;                // descriptor version of sm_100
-    d |= static_cast<uint64_t>(2) << 61;                // SWIZZLE_128B
-    return d;
 }
 
 __device__ __forceinline__ uint4 lds128p(uint32_t addr) {
@@ -571,36 +557,6 @@ static_assert(PR_SMEM <= 227 * 1024, "shared memory of the pair form");
 static_assert(PR_ACC_COLS + PR_AS * PR_A_COLS <= 512 && PR_N % 32 == 0 && PR_X_ATOM % 1024 == 0 && PR_AS % PR_PARTS == 0 && PR_PARTS == 2,
               "tensor memory / tile shape of the pair form");
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-    return r;
-}
-// the address of `p` (a shared-memory location of this CTA) in the CTA of rank `rank` of the cluster
-__device__ __forceinline__ uint32_t map_to_rank(const void* p, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-    return r;
-}
-// Arrival on a barrier of another CTA of the cluster.  What the barriers of this kernel order is tensor-memory traffic
-// (tcgen05.st / tcgen05.ld completed by their own wait instructions and fenced with tcgen05.fence), not generic memory,
-// so the arrival carries no cluster-scope release: that form cost about 1.5 k cycles per arrival in the expansion warps.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
-}
-// commit of the pair's MMAs: one arrival on the barrier at this shared-memory offset in BOTH CTAs
-__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(smem_u32(bar)),
-                 "h"(static_cast<uint16_t>(3))
-                 : "memory");
-}
-// TMA copy into THIS CTA's shared memory whose bytes are counted on a barrier given as a cluster address (the leader's)
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const void* tmap, int c0, int c1, uint32_t bar_cluster_addr) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
-                     smem_u32(dst)),
-                 "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(bar_cluster_addr)
-                 : "memory");
-}
 __device__ __forceinline__ void mma_i8_ts_x4_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate_first) {
     asm volatile(
         "{\n .reg .pred p, q;\n .reg .b32 a1, a2, a3;\n .reg .b64 b1, b2, b3;\n"
@@ -899,41 +855,42 @@ __global__ void rowsum_i8_kernel(const int8_t* __restrict__ q, int64_t ldq, int 
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn pf_encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    }
-    return fn;
-}
-
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 }  // namespace wf
 
 using namespace wf;
 
+extern "C" int wf_wide_status_fetch(int* out);
+
 extern "C" int wf_prefill_status_fetch(int* out) {
+    int wide = 0;
+    if (int rc = wf_wide_status_fetch(&wide)) return rc;
     WF_CUDA(cudaMemcpyFromSymbol(out, g_prefill_status, sizeof(int)));
     if (*out) {
         int zero = 0;
         WF_CUDA(cudaMemcpyToSymbol(g_prefill_status, &zero, sizeof(int)));
     }
+    if (!*out) *out = wide;
     return WF_OK;
 }
+
+int wf_quantize_expand(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, float eps, int8_t* q, float* scale, const uint8_t* codes,
+                       int layout, int64_t N, int8_t* w8, void* stream);
+int wf_wide_launch(const int8_t* q, int64_t ldq, const float* x_scale, const int8_t* w8, const float* w_scale, float w_scale_host, const void* bias,
+                   int bias_dtype, void* y, int y_dtype, int64_t ldy, int64_t M, int64_t N, int64_t K, int bn, void* stream);
+int wf_wide_tile(int64_t M, int64_t N, int64_t K);
 
 // workspace: int8 activations [M, K] | multipliers [M] | row sums [M]
 extern "C" size_t wf_prefill_workspace_bytes(int64_t M, int64_t K) {
     if (M <= 0 || K <= 0) return 0;
     return align_up(static_cast<size_t>(M) * K, 256) + 2 * align_up(static_cast<size_t>(M) * 4, 256);
+}
+
+// ... and behind them, for the form for many tokens, the weights as one byte each [N, K]
+extern "C" size_t wf_prefill_workspace_bytes_for(int64_t M, int64_t N, int64_t K) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    return wf_prefill_workspace_bytes(M, K) + (wf_wide_tile(M, N, K) ? static_cast<size_t>(N) * K : 0);
 }
 
 // `batch` independent problems stacked along the rows: tokens [batch*M, K], weights [batch*N, K/4],
@@ -956,6 +913,19 @@ static int prefill_impl(const char* who, const void* x, int x_dtype, int64_t ldx
     int8_t* wq = reinterpret_cast<int8_t*>(ws);
     float* wscale = reinterpret_cast<float*>(ws + align_up(static_cast<size_t>(M) * K, 256));
     int32_t* wsum = reinterpret_cast<int32_t*>(ws + align_up(static_cast<size_t>(M) * K, 256) + align_up(static_cast<size_t>(M) * 4, 256));
+
+    // The form for many tokens: where it pays, the workspace has room for the expanded weights and nothing of the other
+    // forms is asked for.
+    const size_t base_bytes = wf_prefill_workspace_bytes(M, K);
+    const int wide_bn = batch == 1 ? wf_wide_tile(M, N, K) : 0;
+    if (wide_bn && workspace_bytes >= base_bytes + static_cast<size_t>(N) * K && acc_out == nullptr &&
+        !(flags & (WF_FLAG_WS_READY | WF_FLAG_PREFILL_PAIR | WF_FLAG_PREFILL_SINGLE))) {
+        int8_t* w8 = reinterpret_cast<int8_t*>(ws + base_bytes);
+        if (int rc = wf_quantize_expand(x, x_dtype, M, K, ldx, eps, wq, wscale, codes, layout, N, w8, stream)) return rc;
+        const bool given = x_dtype == WF_I8;
+        return wf_wide_launch(given ? static_cast<const int8_t*>(x) : wq, given ? ldx : K, given ? x_scale : wscale, w8, w_scale, w_scale_host, bias,
+                              bias_dtype, y, y_dtype, ldy, M, N, K, wide_bn, stream);
+    }
 
     const int8_t* q = nullptr;
     const float* qs = nullptr;

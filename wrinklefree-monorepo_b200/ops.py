@@ -236,12 +236,12 @@ def bitlinear(x: torch.Tensor, codes: torch.Tensor, w_scale, bias: Optional[torc
         if m == 0:
             pass
         elif use_prefill:
-            nbytes = lib.wf_prefill_workspace_bytes(m, k)
-            ws = _workspace(x.device, nbytes)
+            # a workspace of the call's own: with one that is shared, two streams of a device would write the same tokens
+            ws = torch.empty(lib.wf_prefill_workspace_bytes_for(m, n, k), dtype=torch.uint8, device=x.device)
             L.check(lib.wf_bitlinear_prefill(x2.data_ptr(), _DT[x2.dtype], x2.stride(0), _ptr(x_scale), codes.data_ptr(),
                                              layout, ws_ptr, ws_host, _ptr(bias), _DT[bias.dtype] if bias is not None else 0,
                                              y.data_ptr(), _DT[y.dtype], y.stride(0), _ptr(acc), m, n, k, eps,
-                                             _ptr(ws), ws.numel() if ws is not None else 0, flags, _stream()),
+                                             ws.data_ptr(), ws.numel(), flags, _stream()),
                     "wf_bitlinear_prefill")
         else:
             if x2.dtype != torch.int8 and _prequant(m, k):

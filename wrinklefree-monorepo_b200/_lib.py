@@ -10,6 +10,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libwf_b200.so")
+HOST_PATH = os.path.join(os.path.dirname(LIB_PATH), "wf_host.so")
 
 # constants of include/wf_b200.h
 WF_F32, WF_F16, WF_BF16, WF_I8 = 0, 1, 2, 3
@@ -120,6 +121,28 @@ def lib():
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The CPython extension of the per-call host path (csrc/wf_host.cpp)."""
+    global _host
+    if _host is None:
+        lib()  # the same message when nothing has been built
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python __graft_entry__.py build`")
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401  (the extension links against its libraries)
+
+        loader = importlib.machinery.ExtensionFileLoader("wf_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("wf_host", HOST_PATH, loader=loader))
+        loader.exec_module(mod)
+        _host = mod
+    return _host
 
 
 def check(rc: int, what: str) -> None:

@@ -8,6 +8,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libwf_b200.so")
+HOST_LIB = os.path.join(HERE, "wf_host.so")
 SOURCES = ["wf_capi.cu", "wf_pack.cu", "wf_actquant.cu", "wf_decode.cu", "wf_prefill.cu", "wf_wide.cu", "wf_elementwise.cu",
            "wf_allreduce.cu", "wf_probe.cu", "wf_attention.cu", "wf_linear.cu"]
 NVCC_FLAGS = [
@@ -70,7 +71,30 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n" + r.stdout + r.stderr)
+    build_host_extension(force)
     return LIB
+
+
+def build_host_extension(force: bool = False) -> str:
+    """Compiles the CPython extension of the per-call host path (csrc/wf_host.cpp) against this interpreter and torch."""
+    src = os.path.join(CSRC, "wf_host.cpp")
+    if not force and not _newer(HOST_LIB, [src, os.path.join(HERE, "..", "include", "wf_b200.h")]):
+        return HOST_LIB
+    import sysconfig
+
+    import torch
+
+    troot = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))) if os.path.sep in _nvcc() else os.path.join(os.sep, "usr", "local", "cuda")
+    cmd = [_host_compiler(), "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", HOST_LIB,
+           "-I" + os.path.join(troot, "include"), "-I" + os.path.join(troot, "include", "torch", "csrc", "api", "include"),
+           "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(cuda, "include"),
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-L" + os.path.join(troot, "lib"),
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-L" + HERE, "-lwf_b200", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("host extension failed:\n" + r.stdout + r.stderr)
+    return HOST_LIB
 
 
 if __name__ == "__main__":

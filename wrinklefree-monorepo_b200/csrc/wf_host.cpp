@@ -1,0 +1,239 @@
+// The per-call host path of the two operators that every projection goes through, as a CPython extension over the C ABI:
+// argument checks, allocation of results and workspace, the choice of the kernel family, the launches.
+//
+// What bounds a small call is this path and not the GPU: written in Python over ctypes, a projection of one token took 20 us
+// of host time (device guard 1.5, stream look-up 3.2, three allocations, twenty converted arguments) around a kernel of
+// five; here it takes about seven, of which the launch itself is three.
+#include <torch/csrc/python_headers.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include "../../include/wf_b200.h"
+
+namespace {
+
+struct PyFailure {};  // a Python exception is set
+
+[[noreturn]] void raise(PyObject* type, const std::string& msg) {
+    PyErr_SetString(type, msg.c_str());
+    throw PyFailure();
+}
+
+int dtype_code(at::ScalarType t) {
+    switch (t) {
+        case at::kFloat: return WF_F32;
+        case at::kHalf: return WF_F16;
+        case at::kBFloat16: return WF_BF16;
+        case at::kChar: return WF_I8;
+        default: raise(PyExc_KeyError, c10::str("unsupported dtype ", t));
+    }
+}
+
+const at::Tensor* optional_tensor(PyObject* o) {
+    if (o == Py_None) return nullptr;
+    if (!THPVariable_Check(o)) raise(PyExc_TypeError, "expected a tensor or None");
+    return &THPVariable_Unpack(o);
+}
+const at::Tensor& tensor(PyObject* o) {
+    const at::Tensor* t = optional_tensor(o);
+    if (!t) raise(PyExc_TypeError, "expected a tensor, got None");
+    return *t;
+}
+void need_cuda(std::initializer_list<const at::Tensor*> ts) {
+    for (const at::Tensor* t : ts)
+        if (t && !t->is_cuda()) raise(PyExc_RuntimeError, "wf_b200 operators need CUDA tensors (there is no CPU path)");
+}
+long long_arg(PyObject* o) {
+    const long v = PyLong_AsLong(o);
+    if (v == -1 && PyErr_Occurred()) throw PyFailure();
+    return v;
+}
+double float_arg(PyObject* o) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) throw PyFailure();
+    return v;
+}
+bool truth(PyObject* o) {
+    const int v = PyObject_IsTrue(o);
+    if (v < 0) throw PyFailure();
+    return v != 0;
+}
+void check(int rc, const char* what) {
+    if (rc) raise(PyExc_RuntimeError, c10::str(what, " failed (code ", rc, "): ", wf_last_error()));
+}
+
+// x as [tokens, K] with unit inner stride
+at::Tensor as_rows(const at::Tensor& x) {
+    if (x.dim() == 0) raise(PyExc_IndexError, "expected a tensor with at least one dimension");
+    at::Tensor r = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
+    return r.stride(1) == 1 ? r : r.contiguous();
+}
+void* ptr(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+
+struct Quantized {
+    at::Tensor q, scale, rowsum;
+};
+Quantized quantize(const at::Tensor& rows, bool per_tensor, double eps, bool want_rowsum, void* stream) {
+    const int64_t m = rows.size(0), k = rows.size(1);
+    Quantized r;
+    r.q = at::empty({m, k}, rows.options().dtype(at::kChar));
+    r.scale = at::empty({per_tensor ? 1 : m}, rows.options().dtype(at::kFloat));
+    if (want_rowsum) r.rowsum = at::empty({m}, rows.options().dtype(at::kInt));
+    const int dt = dtype_code(rows.scalar_type());
+    const int64_t ldx = rows.stride(0);
+    int rc;
+    {
+        pybind11::gil_scoped_release nogil;
+        rc = wf_act_quant_i8(rows.data_ptr(), dt, m, k, ldx, per_tensor ? WF_ACT_PER_TENSOR : WF_ACT_PER_TOKEN, static_cast<float>(eps),
+                             static_cast<int8_t*>(r.q.data_ptr()), static_cast<float*>(r.scale.data_ptr()), static_cast<int32_t*>(ptr(r.rowsum)), stream);
+    }
+    check(rc, "wf_act_quant_i8");
+    return r;
+}
+
+PyObject* wrap(const at::Tensor& t) {
+    PyObject* o = THPVariable_Wrap(t);
+    if (!o) throw PyFailure();
+    return o;
+}
+PyObject* wrap_all(std::initializer_list<at::Tensor> ts) {
+    PyObject* out = PyTuple_New(static_cast<Py_ssize_t>(ts.size()));
+    if (!out) throw PyFailure();
+    Py_ssize_t i = 0;
+    for (const at::Tensor& t : ts) {
+        PyObject* o = THPVariable_Wrap(t);
+        if (!o) {
+            Py_DECREF(out);
+            throw PyFailure();
+        }
+        PyTuple_SET_ITEM(out, i++, o);
+    }
+    return out;
+}
+
+// act_quant_i8(x, per_tensor, eps, want_rowsum) -> (q, scale[, rowsum])
+PyObject* act_quant_i8(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    try {
+        if (n != 4) raise(PyExc_TypeError, "act_quant_i8 takes 4 arguments");
+        const at::Tensor& x = tensor(a[0]);
+        need_cuda({&x});
+        const at::Tensor rows = as_rows(x);
+        c10::cuda::CUDAGuard guard(x.device());
+        const Quantized r = quantize(rows, truth(a[1]), float_arg(a[2]), truth(a[3]), c10::cuda::getCurrentCUDAStream().stream());
+        const at::Tensor q = x.dim() == 2 ? r.q : r.q.reshape(x.sizes());
+        return r.rowsum.defined() ? wrap_all({q, r.scale, r.rowsum}) : wrap_all({q, r.scale});
+    } catch (const PyFailure&) {
+        return nullptr;
+    }
+    END_HANDLE_TH_ERRORS
+}
+
+// bitlinear(x, codes, w_scale, bias, out_dtype, layout, x_scale, eps, want_acc, flags, path, out, decode_max_tokens,
+//           prequant_min_tokens, prequant_min_elems) -> y | (y, acc);   path: 0 auto, 1 decode, 2 prefill
+PyObject* bitlinear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    try {
+        if (n_args != 15) raise(PyExc_TypeError, "bitlinear takes 15 arguments");
+        const at::Tensor& x = tensor(a[0]);
+        at::Tensor codes = tensor(a[1]);
+        const at::Tensor* bias = optional_tensor(a[3]);
+        const at::Tensor* x_scale = optional_tensor(a[6]);
+        const at::Tensor* out = optional_tensor(a[11]);
+        need_cuda({&x, &codes, bias, x_scale});
+        if (x.dim() == 0) raise(PyExc_IndexError, "bitlinear: x needs at least one dimension");
+        const int64_t k = x.size(-1);
+        if (codes.scalar_type() != at::kByte || codes.dim() != 2 || codes.size(1) * 4 != k)
+            raise(PyExc_ValueError, c10::str("codes must be uint8 [N, K/4] with K=", k, ", got ", codes.sizes(), " ", codes.scalar_type()));
+        const int64_t n = codes.size(0);
+        at::Tensor rows = as_rows(x);
+        const int64_t m = rows.size(0);
+        c10::cuda::CUDAGuard guard(x.device());
+        at::ScalarType y_type = x.scalar_type() == at::kChar ? at::kFloat : x.scalar_type();
+        if (a[4] != Py_None) {
+            if (!THPDtype_Check(a[4])) raise(PyExc_TypeError, "out_dtype must be a torch.dtype");
+            y_type = reinterpret_cast<THPDtype*>(a[4])->scalar_type;
+        }
+        const at::Tensor y = out ? *out : at::empty({m, n}, x.options().dtype(y_type));
+        at::Tensor acc;
+        if (truth(a[8])) acc = at::empty({m, n}, x.options().dtype(at::kInt));
+        const float* ws_dev = nullptr;
+        float ws_host = 0.f;
+        if (THPVariable_Check(a[2])) {
+            const at::Tensor& s = THPVariable_Unpack(a[2]);
+            if (s.scalar_type() != at::kFloat || !s.is_cuda()) raise(PyExc_ValueError, "w_scale tensor must be float32 on the GPU");
+            ws_dev = static_cast<const float*>(s.data_ptr());
+        } else {
+            ws_host = static_cast<float>(float_arg(a[2]));
+        }
+        if (!codes.is_contiguous()) codes = codes.contiguous();
+        const int layout = static_cast<int>(long_arg(a[5]));
+        const double eps = float_arg(a[7]);
+        const unsigned flags = static_cast<unsigned>(long_arg(a[9]));
+        const long path = long_arg(a[10]);
+        void* const stream = c10::cuda::getCurrentCUDAStream().stream();
+        const int bias_type = bias ? dtype_code(bias->scalar_type()) : 0;
+        const void* const bias_ptr = bias ? bias->data_ptr() : nullptr;
+        const float* xs_ptr = x_scale ? static_cast<const float*>(x_scale->data_ptr()) : nullptr;
+        // auto: the tensor-core contraction above decode_max_tokens tokens, and from 16 tokens on for matrices of at least 4 Mi
+        // weights (measured: 4096 x 4096 at 32 tokens 14 us against 20 us on the decode kernel; small layers the reverse)
+        const bool contraction = path == 2 || (path == 0 && (m > long_arg(a[12]) || (m >= 16 && n * k >= (1 << 22))));
+        if (m > 0) {
+            const int64_t ldy = y.stride(0);
+            const int y_code = dtype_code(y.scalar_type());
+            int32_t* const acc_ptr = static_cast<int32_t*>(ptr(acc));
+            const uint8_t* const codes_ptr = static_cast<const uint8_t*>(codes.data_ptr());
+            int rc;
+            if (contraction) {
+                // a workspace of the call's own: two streams of a device never write the same tokens
+                const size_t bytes = wf_prefill_workspace_bytes_for(m, n, k);
+                const at::Tensor ws = at::empty({static_cast<int64_t>(bytes)}, x.options().dtype(at::kByte));
+                const int x_code = dtype_code(rows.scalar_type());
+                pybind11::gil_scoped_release nogil;
+                rc = wf_bitlinear_prefill(rows.data_ptr(), x_code, rows.stride(0), xs_ptr, codes_ptr, layout, ws_dev, ws_host, bias_ptr, bias_type,
+                                          y.data_ptr(), y_code, ldy, acc_ptr, m, n, k, static_cast<float>(eps), ws.data_ptr(), bytes, flags, stream);
+            } else {
+                Quantized pre;  // alive until the launch: its memory goes back to this stream's pool
+                if (rows.scalar_type() != at::kChar && (m >= long_arg(a[13]) || m * k >= long_arg(a[14]))) {
+                    // every CTA of the decode kernel quantizes the tokens of its problem: from this many tokens on one
+                    // quantization kernel in front of it is cheaper (same arithmetic, same bits)
+                    pre = quantize(rows, false, eps, false, stream);
+                    rows = pre.q;
+                    xs_ptr = static_cast<const float*>(pre.scale.data_ptr());
+                }
+                const int x_code = dtype_code(rows.scalar_type());
+                pybind11::gil_scoped_release nogil;
+                rc = wf_bitlinear_decode(rows.data_ptr(), x_code, rows.stride(0), xs_ptr, codes_ptr, layout, ws_dev, ws_host, bias_ptr, bias_type,
+                                         y.data_ptr(), y_code, ldy, acc_ptr, m, n, k, static_cast<float>(eps), flags, stream);
+            }
+            check(rc, contraction ? "wf_bitlinear_prefill" : "wf_bitlinear_decode");
+        }
+        at::Tensor shaped = y;
+        if (x.dim() != 2 || y.dim() != 2 || y.size(0) != m || y.size(1) != n) {
+            std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end() - 1);
+            shape.push_back(n);
+            shaped = y.reshape(shape);
+        }
+        return acc.defined() ? wrap_all({shaped, acc}) : wrap(shaped);
+    } catch (const PyFailure&) {
+        return nullptr;
+    }
+    END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"act_quant_i8", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(act_quant_i8)), METH_FASTCALL, nullptr},
+    {"bitlinear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(bitlinear)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "wf_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_wf_host() { return PyModule_Create(&module); }

@@ -30,7 +30,7 @@ def stack_uses_contraction(m: int, k: int) -> bool:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())  # a tenth of the time of torch.cuda.current_stream()
 
 
 def _need_cuda(*ts):
@@ -147,28 +147,13 @@ def act_quant_i8(x: torch.Tensor, per_tensor: bool = False, eps: float = 1e-5, w
     """int8 activation quantization.  Per token (default) follows BitLinear.activation_quant
     in the arithmetic of x.dtype; per_tensor follows bitnet_quantize_activations_cpu (fp32).
     Returns (q int8 same shape, scale fp32 [M] or [1][, rowsum int32 [M]])."""
-    _need_cuda(x)
-    k = x.shape[-1]
-    x2 = x.reshape(-1, k)
-    if x2.stride(1) != 1:
-        x2 = x2.contiguous()
-    m = x2.shape[0]
-    q = torch.empty((m, k), dtype=torch.int8, device=x.device)
-    scale = torch.empty(1 if per_tensor else m, dtype=torch.float32, device=x.device)
-    rowsum = torch.empty(m, dtype=torch.int32, device=x.device) if want_rowsum else None
-    with torch.cuda.device(x.device):
-        L.check(L.lib().wf_act_quant_i8(x2.data_ptr(), _DT[x2.dtype], m, k, x2.stride(0),
-                                        L.ACT_PER_TENSOR if per_tensor else L.ACT_PER_TOKEN, eps, q.data_ptr(),
-                                        scale.data_ptr(), _ptr(rowsum), _stream()), "wf_act_quant_i8")
-    q = q.reshape(x.shape)
-    return (q, scale, rowsum) if want_rowsum else (q, scale)
+    return L.host().act_quant_i8(x, per_tensor, eps, want_rowsum)
 
 
 # --------------------------------------------------------------------------
 # the contraction
 # --------------------------------------------------------------------------
 
-_workspaces = {}
 # Decode path: every CTA of the decode kernel quantizes the tokens of its problem itself.  That is the right trade for a
 # stack of many small problems (a CTA meets one or two of them), not for one projection that all CTAs share: there a
 # quantization kernel in front (same arithmetic, same bits) takes the absmax reduction and its barriers off the critical
@@ -181,14 +166,6 @@ PREQUANT_MAX_PROBLEMS = 4
 
 def _prequant(m: int, k: int, problems: int = 1) -> bool:
     return m >= PREQUANT_MIN_TOKENS or (problems <= PREQUANT_MAX_PROBLEMS and m * k >= PREQUANT_MIN_ELEMS)
-
-
-def _workspace(device, nbytes: int) -> torch.Tensor:
-    ws = _workspaces.get(device)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[device] = ws
-    return ws
 
 
 def bitlinear(x: torch.Tensor, codes: torch.Tensor, w_scale, bias: Optional[torch.Tensor] = None,
@@ -205,55 +182,9 @@ def bitlinear(x: torch.Tensor, codes: torch.Tensor, w_scale, bias: Optional[torc
     prefill_form: "auto", or "pair" / "single" to force the two-SM or the one-SM tile form of the contraction.
     Returns y [..., N] (and the int32 accumulators [M, N] when want_acc).
     """
-    _need_cuda(x, codes, bias, x_scale)
-    k = x.shape[-1]
-    n = codes.shape[0]
-    if codes.dtype != torch.uint8 or codes.dim() != 2 or codes.shape[1] * 4 != k:
-        raise ValueError(f"codes must be uint8 [N, K/4] with K={k}, got {tuple(codes.shape)} {codes.dtype}")
-    x2 = x.reshape(-1, k)
-    if x2.stride(1) != 1:
-        x2 = x2.contiguous()
-    m = x2.shape[0]
-    if out_dtype is None:
-        out_dtype = torch.float32 if x.dtype == torch.int8 else x.dtype
-    y = out if out is not None else torch.empty((m, n), dtype=out_dtype, device=x.device)
-    acc = torch.empty((m, n), dtype=torch.int32, device=x.device) if want_acc else None
-    if isinstance(w_scale, torch.Tensor):
-        ws_ptr, ws_host = w_scale.data_ptr(), 0.0
-        if w_scale.dtype != torch.float32 or not w_scale.is_cuda:
-            raise ValueError("w_scale tensor must be float32 on the GPU")
-    else:
-        ws_ptr, ws_host = None, float(w_scale)
-    if not codes.is_contiguous():
-        codes = codes.contiguous()
-    lib = L.lib()
-    flags = L.FLAG_PDL if pdl else 0
-    flags |= {"auto": 0, "pair": L.FLAG_PREFILL_PAIR, "single": L.FLAG_PREFILL_SINGLE}[prefill_form]
-    # auto: the tensor-core contraction above DECODE_MAX_TOKENS tokens, and from 16 tokens on for matrices of at least
-    # 4 Mi weights (measured: 4096 x 4096 at 32 tokens 14 us against 20 us on the decode kernel; small layers the reverse)
-    use_prefill = path == "prefill" or (path == "auto" and (m > DECODE_MAX_TOKENS or (m >= 16 and n * k >= (1 << 22))))
-    with torch.cuda.device(x.device):
-        if m == 0:
-            pass
-        elif use_prefill:
-            # a workspace of the call's own: with one that is shared, two streams of a device would write the same tokens
-            ws = torch.empty(lib.wf_prefill_workspace_bytes_for(m, n, k), dtype=torch.uint8, device=x.device)
-            L.check(lib.wf_bitlinear_prefill(x2.data_ptr(), _DT[x2.dtype], x2.stride(0), _ptr(x_scale), codes.data_ptr(),
-                                             layout, ws_ptr, ws_host, _ptr(bias), _DT[bias.dtype] if bias is not None else 0,
-                                             y.data_ptr(), _DT[y.dtype], y.stride(0), _ptr(acc), m, n, k, eps,
-                                             ws.data_ptr(), ws.numel(), flags, _stream()),
-                    "wf_bitlinear_prefill")
-        else:
-            if x2.dtype != torch.int8 and _prequant(m, k):
-                # every CTA of the decode kernel quantizes the tokens of its problem: from this many tokens on one
-                # quantization kernel in front of it is cheaper (same arithmetic, same bits)
-                x2, x_scale = act_quant_i8(x2, eps=eps)
-            L.check(lib.wf_bitlinear_decode(x2.data_ptr(), _DT[x2.dtype], x2.stride(0), _ptr(x_scale), codes.data_ptr(),
-                                            layout, ws_ptr, ws_host, _ptr(bias), _DT[bias.dtype] if bias is not None else 0,
-                                            y.data_ptr(), _DT[y.dtype], y.stride(0), _ptr(acc), m, n, k, eps, flags,
-                                            _stream()), "wf_bitlinear_decode")
-    y = y.reshape(*x.shape[:-1], n)
-    return (y, acc) if want_acc else y
+    flags = (L.FLAG_PDL if pdl else 0) | {"auto": 0, "pair": L.FLAG_PREFILL_PAIR, "single": L.FLAG_PREFILL_SINGLE}[prefill_form]
+    return L.host().bitlinear(x, codes, w_scale, bias, out_dtype, layout, x_scale, eps, want_acc, flags,
+                              {"auto": 0, "decode": 1, "prefill": 2}.get(path, 1), out, DECODE_MAX_TOKENS, PREQUANT_MIN_TOKENS, PREQUANT_MIN_ELEMS)
 
 
 def prefill_workspace(m_rows: int, k: int, device) -> torch.Tensor:
@@ -286,7 +217,7 @@ def bitlinear_batched(x: torch.Tensor, codes: torch.Tensor, w_scales: torch.Tens
     x [B, M, K] (contiguous), codes uint8 [B, N, K/4] (contiguous), w_scales float32 [B] or [B, 2] (first column used).
     Returns y [B, M, N] (and the int32 accumulators when want_acc).
 
-    `workspace` (default: one shared per device) with `quantized=True`: `prefill_quantize(x, workspace)` ran earlier in
+    `workspace` (default: one of the call's own) with `quantized=True`: `prefill_quantize(x, workspace)` ran earlier in
     the stream and x is not read again.  `independent=True` in addition: the workspace and the output have nothing to do
     with the launches since the last contraction that was not marked so (the quantizations went first, then one
     unmarked contraction): the launch does not wait for its predecessor and fills the SMs its tail leaves idle.
@@ -308,7 +239,7 @@ def bitlinear_batched(x: torch.Tensor, codes: torch.Tensor, w_scales: torch.Tens
     acc = torch.empty((b * m, n), dtype=torch.int32, device=x.device) if want_acc else None
     lib = L.lib()
     nbytes = lib.wf_prefill_workspace_bytes(b * m, k)
-    ws = workspace if workspace is not None else _workspace(x.device, nbytes)
+    ws = workspace if workspace is not None else torch.empty(nbytes, dtype=torch.uint8, device=x.device)
     flags = (L.FLAG_WS_READY if quantized else 0) | (L.FLAG_X_READY if independent else 0)
     with torch.cuda.device(x.device):
         L.check(lib.wf_bitlinear_prefill_batched(x.data_ptr(), _DT[x.dtype], k, codes.data_ptr(), layout, w_scales.data_ptr(),

@@ -164,6 +164,41 @@ def test_act_quant_many_tokens(wf, k, dt):
 
 
 # ---------------------------------------------------------------- contraction
+@pytest.mark.parametrize("n,k", [(1, 64), (5, 192), (3, 1024), (7, 1088), (130, 960), (64, 4160)])
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+def test_pack_ternary_edges_of_its_units(wf, n, k, dt):
+    """Matrices that end inside a warp's 1024 weights, contiguous (one run) and strided (row by row), weights on the rounding
+    boundary of the scale, zeros, and a NaN or an infinity among them: codes and scales equal the oracle's exactly."""
+    rng = np.random.default_rng(n * 977 + k)
+    base = (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
+    ties = (rng.integers(-4, 5, (n, k)) * 0.25).astype(np.float32)  # the mean is not far from 0.5 and 1
+    ties.reshape(-1)[:8] = [0.5, -0.5, 1.0, -1.0, 0.25, -0.25, 0.0, -0.0]
+    for w in (base, ties, np.zeros_like(base), base * 1e-7):
+        wt = torch.from_numpy(w).to(TDT[dt])
+        wide = torch.zeros(n, k + 64, dtype=TDT[dt], device=DEV)
+        wide[:, :k] = wt.to(DEV)
+        for view in (wt.to(DEV), wide[:, :k]):
+            codes, scale = wf.pack_ternary(view)
+            t, s = O.ternarize_absmean(wt.float().numpy())
+            assert np.array_equal(codes.cpu().numpy(), O.pack_wf16(t)) and scale[0].item() == s
+            for mode in ("bf16", "f16"):
+                with np.errstate(all="ignore"):
+                    t, dq, mul = O.ternarize_cast_first(wt.float().numpy(), mode)
+                if np.isfinite([dq, mul]).all():
+                    codes, scale = wf.pack_ternary(view, mode=TDT[mode])
+                    assert np.array_equal(codes.cpu().numpy(), O.pack_wf16(t)) and scale[0].item() == dq and scale[1].item() == mul
+    for bad in (np.nan, np.inf):  # a NaN ternarizes to -1 with the scale clamped to eps, an infinity makes the scale infinite
+        w = base.copy()
+        w[n // 2, k // 2] = bad
+        wt = torch.from_numpy(w).to(TDT[dt]).to(DEV)
+        codes, scale = wf.pack_ternary(wt)
+        mean = wt.float().abs().double().mean().float()
+        mean = torch.where(mean.isnan(), torch.full_like(mean, 1e-5), mean)
+        t = (wt.float() / mean).round().clamp(-1, 1)
+        t = torch.where(t.isnan(), torch.full_like(t, -1.0), t)
+        assert torch.equal(wf.unpack_codes(codes, n, k), t.to(torch.int8)) and scale[0].item() == mean.item()
+
+
 @pytest.mark.parametrize("m,k", [(1, 8), (288, 8), (287, 768), (300, 776), (1153, 1536), (3201, 2560), (9, 2568), (5, 8200), (3, 14336), (2, 14344)])
 @pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
 def test_act_quant_every_split_of_a_row(wf, m, k, dt):

@@ -13,8 +13,7 @@
 namespace wf {
 
 constexpr int PACK_THREADS = 256;
-constexpr int WORDS_PER_THREAD = 4;                                      // 64 weights per thread
-constexpr int PACK_WEIGHTS_PER_BLOCK = PACK_THREADS * WORDS_PER_THREAD * 16;  // 16384
+constexpr int PACK_WEIGHTS_PER_BLOCK = 16384;  // sizes the grid: weights per block and pass, at least
 
 __device__ __forceinline__ double block_sum(double v, double* sh) {
 #pragma unroll
@@ -33,40 +32,144 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return t;
 }
 
+// Ternarization is two passes over the weights, both bound by memory: 14336 x 4096 fp32 weights (235 MB) took 117 us when a
+// thread read 64 consecutive weights (256 bytes apart from its neighbour's) and divided each by the scale.  Now a warp reads
+// 1024 consecutive weights at a time, eight per lane and load, and compares with a threshold; the second pass walks
+// them from the end, where the first one has left the last 100 MB or so in L2: 71 us (first pass 40, 5.9 TB/s).  6912 x 2560:
+// 34.8 -> 20.8 us, 1536 x 576: 10.9 -> 7.2.
+constexpr int PACK_UNIT = 1024;  // weights per warp and step: four loads of 8 per lane
+
+// 8 consecutive weights
+template <int WDT>
+struct Weights8 {
+    uint4 v[WDT == WF_F32 ? 2 : 1];
+};
+template <int WDT>
+__device__ __forceinline__ void load_weights8(const void* w, int64_t elem, bool ok, Weights8<WDT>& r) {
+    const uint4* p = reinterpret_cast<const uint4*>(static_cast<const char*>(w) + elem * (WDT == WF_F32 ? 4 : 2));
+#pragma unroll
+    for (int j = 0; j < (WDT == WF_F32 ? 2 : 1); ++j) r.v[j] = ok ? __ldg(p + j) : make_uint4(0, 0, 0, 0);
+}
+template <int WDT>
+__device__ __forceinline__ void weight_values(const Weights8<WDT>& r, float (&f)[8]) {
+    const uint32_t w[4] = {r.v[0].x, r.v[0].y, r.v[0].z, r.v[0].w};
+    if constexpr (WDT == WF_F32) {
+        const uint32_t u[4] = {r.v[1].x, r.v[1].y, r.v[1].z, r.v[1].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            f[i] = __uint_as_float(w[i]);
+            f[4 + i] = __uint_as_float(u[i]);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if constexpr (WDT == WF_BF16) {
+                f[2 * i] = __uint_as_float(w[i] << 16);
+                f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+            } else {
+                const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                f[2 * i] = v.x;
+                f[2 * i + 1] = v.y;
+            }
+        }
+    }
+}
+
+// The matrix as `rows` rows of `len` weights, ldw apart (one row when the matrix is contiguous); units of PACK_UNIT weights.
+struct PackShape {
+    const void* w;
+    int64_t len, ldw;
+    int rows;
+    int segs;       // units per row
+    int64_t units;  // rows * segs
+};
+
 // Pass 1: per-block sum of |w| (after the optional cast) in fp64, fixed order.
 template <int WDT, int MODE>
-__global__ void __launch_bounds__(PACK_THREADS) abs_sum_kernel(const void* __restrict__ w, int64_t N, int64_t K,
-                                                               int64_t ldw, double* __restrict__ partial) {
+__global__ void __launch_bounds__(PACK_THREADS) abs_sum_kernel(const PackShape s, double* __restrict__ partial) {
     __shared__ double sh[PACK_THREADS / 32];
-    const int64_t total_vec = N * (K / 8);  // units of 8 weights
-    double s = 0.0;
-    for (int64_t v = static_cast<int64_t>(blockIdx.x) * PACK_THREADS + threadIdx.x; v < total_vec;
-         v += static_cast<int64_t>(gridDim.x) * PACK_THREADS) {
-        int64_t row = v / (K / 8), col = (v % (K / 8)) * 8;
-        float f[8];
-        load8<WDT>(w, row * ldw + col, f);
-        double a = 0.0;
+    const int lane = threadIdx.x & 31;
+    double sum = 0.0;
+    for (int64_t unit = static_cast<int64_t>(blockIdx.x) * (PACK_THREADS / 32) + (threadIdx.x >> 5); unit < s.units;
+         unit += static_cast<int64_t>(gridDim.x) * (PACK_THREADS / 32)) {
+        const int64_t row = s.rows == 1 ? 0 : unit / s.segs, at = (unit - row * s.segs) * PACK_UNIT + 8 * lane;
+        Weights8<WDT> r[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) a += static_cast<double>(fabsf(rnd<MODE>(f[i])));
-        s += a;
+        for (int u = 0; u < 4; ++u) load_weights8<WDT>(s.w, row * s.ldw + at + 256 * u, at + 256 * u < s.len, r[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            float f[8];
+            weight_values<WDT>(r[u], f);
+            double a = 0.0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a += static_cast<double>(fabsf(rnd<MODE>(f[i])));
+            sum += a;
+        }
     }
-    double t = block_sum(s, sh);
+    const double t = block_sum(sum, sh);
     if (threadIdx.x == 0) partial[blockIdx.x] = t;
 }
 
-// Pass 2: every block re-reduces the partials in the same order, derives the
-// scale, ternarizes and packs.  One thread produces four output words from 64
-// consecutive weights.
+// Pass 2: every block re-reduces the partials in the same order, derives the scale, ternarizes and packs.
+//
+// FP32 mode: the code of w is clamp(rint(w / mean), -1, 1) + 1.  The fp32 quotient exceeds 1/2 exactly when w > mean / 2: the
+// next float above mean / 2 is at least half an ulp of 1/2 further in the quotient, and the tie itself rounds to zero.
+// So two comparisons with mean / 2 (exact) stand for the division (which a matrix with a NaN or an infinity keeps).  Cast
+// modes: the same two comparisons on the rounded product; a NaN compares false with both, the code 0 that the clamp gives it.
+//
+// The comparisons of four weights as masks of four bytes (code = [v > h] + [v >= -h]): six instructions per weight that take
+// a predicate, a select and an addition each were what bounded this pass.
+// the sign bits of four floats as four bytes of ones or zeros (a selector with its top bit set replicates the byte's sign)
+__device__ __forceinline__ uint32_t signs4(float a, float b, float c, float d) {
+    uint32_t lo, hi;
+    asm("prmt.b32 %0, %1, %2, 0xfbfb;" : "=r"(lo) : "r"(__float_as_uint(a)), "r"(__float_as_uint(b)));
+    asm("prmt.b32 %0, %1, %2, 0xfbfb;" : "=r"(hi) : "r"(__float_as_uint(c)), "r"(__float_as_uint(d)));
+    return __byte_perm(lo, hi, 0x5410);
+}
+// codes of the weights 4 g .. 4 g + 3 of a lane's eight as four bytes.  h = mean / 2 (FP32) or 1/2; `finite`: the sum of all
+// weights is finite, so there is no NaN and no infinity among them and signs of differences decide (FP32 mode).
+template <int WDT, int MODE>
+__device__ __forceinline__ uint32_t codes4(const Weights8<WDT>& r, int g, float q_mul, float h, bool finite) {
+    const uint32_t ones = 0x01010101u;
+    float f[8];
+    weight_values<WDT>(r, f);
+    if constexpr (MODE == WF_F32) {
+        if (finite) {
+            const uint32_t above = signs4(h - f[4 * g], h - f[4 * g + 1], h - f[4 * g + 2], h - f[4 * g + 3]);
+            const uint32_t below = signs4(f[4 * g] + h, f[4 * g + 1] + h, f[4 * g + 2] + h, f[4 * g + 3] + h);
+            return ones + (above & ones) - (below & ones);
+        }
+        uint32_t c = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            c |= static_cast<uint32_t>(static_cast<int>(fminf(fmaxf(rintf(__fdiv_rn(f[4 * g + i], q_mul)), -1.f), 1.f)) + 1) << (8 * i);
+        return c;
+    } else if constexpr (MODE == WF_BF16) {
+        __nv_bfloat162 v[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) v[i] = __hmul2_rn(__floats2bfloat162_rn(f[4 * g + 2 * i], f[4 * g + 2 * i + 1]), __float2bfloat162_rn(q_mul));
+        const __nv_bfloat162 hi = __float2bfloat162_rn(0.5f), lo = __float2bfloat162_rn(-0.5f);
+        return (__byte_perm(__hgt2_mask(v[0], hi), __hgt2_mask(v[1], hi), 0x6420) & ones) + (__byte_perm(__hge2_mask(v[0], lo), __hge2_mask(v[1], lo), 0x6420) & ones);
+    } else {
+        __half2 v[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) v[i] = __hmul2_rn(__floats2half2_rn(f[4 * g + 2 * i], f[4 * g + 2 * i + 1]), __float2half2_rn(q_mul));
+        const __half2 hi = __float2half2_rn(0.5f), lo = __float2half2_rn(-0.5f);
+        return (__byte_perm(__hgt2_mask(v[0], hi), __hgt2_mask(v[1], hi), 0x6420) & ones) + (__byte_perm(__hge2_mask(v[0], lo), __hge2_mask(v[1], lo), 0x6420) & ones);
+    }
+}
+
 template <int WDT, int MODE>
 __global__ void __launch_bounds__(PACK_THREADS)
-    ternarize_pack_kernel(const void* __restrict__ w, int64_t N, int64_t K, int64_t ldw, const double* __restrict__ partial,
-                          int npartial, float eps, uint8_t* __restrict__ codes, float* __restrict__ scale_out) {
+    ternarize_pack_kernel(const PackShape s, int64_t weights, const double* partial, int npartial, float eps, uint8_t* __restrict__ codes,
+                          float* __restrict__ scale_out) {
     __shared__ double sh[PACK_THREADS / 32];
-    double s = 0.0;
-    for (int i = threadIdx.x; i < npartial; i += PACK_THREADS) s += partial[i];
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the partial sums
+    double sum = 0.0;
+    for (int i = threadIdx.x; i < npartial; i += PACK_THREADS) sum += *static_cast<const volatile double*>(partial + i);
     // the per-thread strided sums depend only on npartial and the block size: identical in every block
-    double total = block_sum(s, sh);
-    float mean = static_cast<float>(total / static_cast<double>(N * K));
+    const double total = block_sum(sum, sh);
+    float mean = static_cast<float>(total / static_cast<double>(weights));
     float q_mul, dq;
     if constexpr (MODE == WF_F32) {
         mean = fmaxf(mean, eps);
@@ -81,34 +184,31 @@ __global__ void __launch_bounds__(PACK_THREADS)
         scale_out[0] = dq;
         scale_out[1] = q_mul;
     }
-    const int64_t chunks_per_row = K / 64;
-    const int64_t total_chunks = N * chunks_per_row;
-    for (int64_t c = static_cast<int64_t>(blockIdx.x) * PACK_THREADS + threadIdx.x; c < total_chunks;
-         c += static_cast<int64_t>(gridDim.x) * PACK_THREADS) {
-        int64_t row = c / chunks_per_row, col = (c % chunks_per_row) * 64;
-        uint32_t words[4];
+    const float half = MODE == WF_F32 ? 0.5f * q_mul : 0.5f;
+    const bool finite = total < 1e300;  // also false for a NaN
+    const int lane = threadIdx.x & 31;
+    const int64_t code_row = s.len / 4;  // bytes
+    for (int64_t back = static_cast<int64_t>(blockIdx.x) * (PACK_THREADS / 32) + (threadIdx.x >> 5); back < s.units;
+         back += static_cast<int64_t>(gridDim.x) * (PACK_THREADS / 32)) {
+        const int64_t unit = s.units - 1 - back;
+        const int64_t row = s.rows == 1 ? 0 : unit / s.segs, at = (unit - row * s.segs) * PACK_UNIT + 8 * lane;
+        Weights8<WDT> r[4];
 #pragma unroll
-        for (int wd = 0; wd < 4; ++wd) {
-            float f[16];
-            float(&lo)[8] = *reinterpret_cast<float(*)[8]>(&f[0]);
-            float(&hi)[8] = *reinterpret_cast<float(*)[8]>(&f[8]);
-            load8<WDT>(w, row * ldw + col + wd * 16, lo);
-            load8<WDT>(w, row * ldw + col + wd * 16 + 8, hi);
-            uint32_t word = 0;
+        for (int u = 0; u < 4; ++u) load_weights8<WDT>(s.w, row * s.ldw + at + 256 * u, at + 256 * u < s.len, r[u]);
+        uint32_t word[4];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float t;
-                if constexpr (MODE == WF_F32)
-                    t = rintf(__fdiv_rn(f[i], q_mul));
-                else
-                    t = rintf(rnd<MODE>(__fmul_rn(rnd<MODE>(f[i]), q_mul)));
-                int code = static_cast<int>(fminf(fmaxf(t, -1.f), 1.f)) + 1;
-                int j = i >> 2, b = i & 3;  // weight 4j + b -> byte b, bit pair j
-                word |= static_cast<uint32_t>(code) << (8 * b + 2 * j);
-            }
-            words[wd] = word;
+        for (int u = 0; u < 4; ++u) {
+            // weights 0-3 in bit pair 0 of the four bytes, 4-7 in bit pair 1
+            uint32_t c = codes4<WDT, MODE>(r[u], 0, q_mul, half, finite) | (codes4<WDT, MODE>(r[u], 1, q_mul, half, finite) << 2);
+            c <<= 4 * (lane & 1);  // an odd lane holds the upper half of its word: bit pairs 2 and 3
+            word[u] = c | __shfl_xor_sync(0xffffffffu, c, 1);
         }
-        *reinterpret_cast<uint4*>(codes + row * (K / 4) + col / 4) = make_uint4(words[0], words[1], words[2], words[3]);
+        // lane l of loads 2h and 2h + 1: the even lanes store the words of one, the odd lanes of the other
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t first = (unit - row * s.segs) * PACK_UNIT + 256 * (2 * h + (lane & 1)) + 16 * (lane >> 1);  // its first weight
+            if (first < s.len) *reinterpret_cast<uint32_t*>(codes + row * code_row + first / 4) = (lane & 1) ? word[2 * h + 1] : word[2 * h];
+        }
     }
 }
 
@@ -226,26 +326,40 @@ static int pack_grid(int64_t N, int64_t K) {
     return static_cast<int>(blocks);
 }
 
+template <int WDT, int MODE>
+static int launch_pack_mode(const PackShape& s, int64_t weights, int grid, float eps, uint8_t* codes, float* scale, double* partial, cudaStream_t st) {
+    abs_sum_kernel<WDT, MODE><<<grid, PACK_THREADS, 0, st>>>(s, partial);
+    WF_CUDA(cudaGetLastError());
+    cudaLaunchConfig_t lc = {};  // its blocks take the places that the first pass leaves and wait there for its sums
+    lc.gridDim = dim3(static_cast<unsigned>(grid));
+    lc.blockDim = dim3(PACK_THREADS);
+    lc.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    WF_CUDA(cudaLaunchKernelEx(&lc, ternarize_pack_kernel<WDT, MODE>, s, weights, static_cast<const double*>(partial), grid, eps, codes, scale));
+    return WF_OK;
+}
+
 template <int WDT>
 static int launch_pack(const void* w, int64_t N, int64_t K, int64_t ldw, int mode, float eps, uint8_t* codes, float* scale,
                        double* partial, cudaStream_t st) {
-    int grid = pack_grid(N, K);
+    const int grid = pack_grid(N, K);
+    PackShape s;
+    s.w = w;
+    s.rows = ldw == K ? 1 : static_cast<int>(N);
+    s.len = ldw == K ? N * K : K;
+    s.ldw = ldw;
+    const int64_t segs = (s.len + PACK_UNIT - 1) / PACK_UNIT;
+    s.segs = static_cast<int>(segs);
+    s.units = s.rows * segs;
     switch (mode) {
-        case WF_PACK_FP32:
-            abs_sum_kernel<WDT, WF_F32><<<grid, PACK_THREADS, 0, st>>>(w, N, K, ldw, partial);
-            ternarize_pack_kernel<WDT, WF_F32><<<grid, PACK_THREADS, 0, st>>>(w, N, K, ldw, partial, grid, eps, codes, scale);
-            break;
-        case WF_PACK_CAST_BF16:
-            abs_sum_kernel<WDT, WF_BF16><<<grid, PACK_THREADS, 0, st>>>(w, N, K, ldw, partial);
-            ternarize_pack_kernel<WDT, WF_BF16><<<grid, PACK_THREADS, 0, st>>>(w, N, K, ldw, partial, grid, eps, codes, scale);
-            break;
-        default:
-            abs_sum_kernel<WDT, WF_F16><<<grid, PACK_THREADS, 0, st>>>(w, N, K, ldw, partial);
-            ternarize_pack_kernel<WDT, WF_F16><<<grid, PACK_THREADS, 0, st>>>(w, N, K, ldw, partial, grid, eps, codes, scale);
-            break;
+        case WF_PACK_FP32: return launch_pack_mode<WDT, WF_F32>(s, N * K, grid, eps, codes, scale, partial, st);
+        case WF_PACK_CAST_BF16: return launch_pack_mode<WDT, WF_BF16>(s, N * K, grid, eps, codes, scale, partial, st);
+        default: return launch_pack_mode<WDT, WF_F16>(s, N * K, grid, eps, codes, scale, partial, st);
     }
-    WF_CUDA(cudaGetLastError());
-    return WF_OK;
 }
 
 }  // namespace wf

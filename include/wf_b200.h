@@ -312,6 +312,15 @@ int wf_prefill_quantize(const void* x, int x_dtype, int64_t ldx, int64_t M, int6
                         size_t workspace_bytes, unsigned flags, void* stream);
 
 /*
+ * The operands of the straight-through backward pass, as the values the reference's fake-quantized tensors hold
+ * (BitLinear.weight_quant and activation_quant, packages/training/src/wrinklefree/models/bitlinear.py:46-84):
+ * wf_dequant_weights: out [N, K] = (code - 1) * scale[0], rounded to `dtype` (codes in WF_LAYOUT_WF16, scale a device pointer).
+ * wf_dequant_tokens:  out [M, K] = q / scale[m], rounded to x_dtype, stored as `dtype`.  All contiguous.
+ */
+int wf_dequant_weights(const uint8_t* codes, const float* scale, void* out, int dtype, int64_t N, int64_t K, void* stream);
+int wf_dequant_tokens(const int8_t* q, const float* scale, int x_dtype, void* out, int dtype, int64_t M, int64_t K, void* stream);
+
+/*
  * Fused elementwise kernels around the projections of a decoder layer (bf16 tensors, contiguous rows).
  * They replace operator chains of the callers of BitLinear in the reference model
  * (packages/training/src/wrinklefree/models/subln.py / transformer.py:80-117 for residual + RMSNorm,

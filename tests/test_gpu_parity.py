@@ -815,3 +815,20 @@ def test_contraction_for_many_tokens_bit_exact(wf, oracle_c, m, n, k):
     wf.bitlinear(x.to(DEV), codes, 0.0173, out=out[:, :n], path="prefill")
     assert bool((out[:, n:] == 7.0).all())
     wf.device_status()
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 64), (3, 5, 192), (40, 33, 2560), (2, 3, 4160)])
+@pytest.mark.parametrize("xdt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+def test_dequantized_operands_of_the_backward_pass(wf, m, n, k, xdt, dt):
+    """One kernel each for the quantized weights and the quantized tokens as values: equal to the chain of torch operators
+    that they stand for, bit for bit."""
+    g = torch.Generator().manual_seed(m + n + k)
+    t = torch.randint(-1, 2, (n, k), generator=g).to(torch.int8)
+    scale = torch.tensor([0.0173, 3.0], device=DEV)
+    want = t.to(DEV).to(TDT[dt]) * scale[0].to(TDT[dt])
+    assert torch.equal(wf.ops.dequant_weights(wf.pack_codes(t.to(DEV)), scale, TDT[dt]), want)
+    q = torch.randint(-128, 128, (m, k), generator=g).to(torch.int8).to(DEV)
+    s = (torch.rand(m, generator=g) * 60 + 0.01).to(TDT[xdt]).float().to(DEV)
+    want = (q.to(TDT[xdt]) / s.to(TDT[xdt]).unsqueeze(1)).to(TDT[dt])
+    assert torch.equal(wf.ops.dequant_tokens(q, s, TDT[xdt], TDT[dt]), want)

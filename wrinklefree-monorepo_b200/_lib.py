@@ -64,6 +64,8 @@ _SIGNATURES = {
     "wf_quantize_maxabs": (_int, [_p, _int, _i64, _i64, _i64, _int, _int, _p, _p, _p]),
     "wf_pack_codes": (_int, [_p, _p, _int, _i64, _i64, _p]),
     "wf_unpack_codes": (_int, [_p, _int, _p, _i64, _i64, _p]),
+    "wf_dequant_weights": (_int, [_p, _p, _p, _int, _i64, _i64, _p]),
+    "wf_dequant_tokens": (_int, [_p, _p, _int, _p, _int, _i64, _i64, _p]),
     "wf_act_quant_i8": (_int, [_p, _int, _i64, _i64, _i64, _int, _f32, _p, _p, _p, _p]),
     "wf_bitlinear_decode": (_int, [_p, _int, _i64, _p, _p, _int, _p, _f32, _p, _int, _p, _int, _i64, _p, _i64, _i64, _i64,
                                    _f32, _u32, _p]),

@@ -31,7 +31,7 @@ class _PackedSTE(torch.autograd.Function):
     the value of ``F.linear(activation_quant(x), weight_quant(w), bias)`` without re-ternarizing the latent weight or
     running a float GEMM over integer-valued operands (wrinklefree/models/bitlinear.py:99-113).
     Backward: the gradients autograd derives from the reference's ``v + (quant(v) - v).detach()`` form:
-    dX = dY @ weight_quant(w)  (the ternary codes times their scale, unpacked on the GPU for this one product),
+    dX = dY @ weight_quant(w)  (the ternary codes times their scale, written out on the GPU for this one product),
     dW = dY^T @ activation_quant(x)  (rebuilt from the saved int8 codes and per-token scales, 1 byte per element saved
     instead of the activation itself), dbias = sum(dY)."""
 
@@ -53,11 +53,13 @@ class _PackedSTE(torch.autograd.Function):
         dy2 = dy.reshape(-1, n)
         dx = dw = db = None
         if ctx.needs_input_grad[0]:
-            w_q = ops.unpack_codes(codes, n, k).to(dy2.dtype) * scale[0].to(dy2.dtype)
-            dx = (dy2 @ w_q).reshape(ctx.in_shape)
+            dx = (dy2 @ ops.dequant_weights(codes, scale, dy2.dtype)).reshape(ctx.in_shape)
         if ctx.needs_input_grad[1]:
-            x_q = q.to(ctx.x_dtype) / s.to(ctx.x_dtype).unsqueeze(1)  # the values activation_quant(x) holds
-            dw = (dy2.t() @ x_q.to(dy2.dtype)).to(ctx.w_dtype)
+            x_q = ops.dequant_tokens(q, s, ctx.x_dtype, dy2.dtype)  # the values activation_quant(x) holds
+            if ctx.w_dtype == torch.float32 and dy2.dtype != torch.float32 and not torch.is_grad_enabled():
+                dw = torch.mm(dy2.t(), x_q, out_dtype=torch.float32)  # the fp32 sums as they are, without a pass that widens them
+            else:
+                dw = (dy2.t() @ x_q).to(ctx.w_dtype)
         if ctx.has_bias and ctx.needs_input_grad[2]:
             db = dy2.sum(0)
         return dx, dw, db, None

@@ -150,6 +150,26 @@ def act_quant_i8(x: torch.Tensor, per_tensor: bool = False, eps: float = 1e-5, w
     return L.host().act_quant_i8(x, per_tensor, eps, want_rowsum)
 
 
+def dequant_weights(codes: torch.Tensor, scale: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """The quantized weights [N, K] of packed WF16 codes as values of `dtype`: (code - 1) * scale[0]."""
+    _need_cuda(codes, scale)
+    n, k = codes.shape[0], codes.shape[1] * 4
+    out = torch.empty((n, k), dtype=dtype, device=codes.device)
+    with torch.cuda.device(codes.device):
+        L.check(L.lib().wf_dequant_weights(codes.data_ptr(), scale.data_ptr(), out.data_ptr(), _DT[dtype], n, k, _stream()), "wf_dequant_weights")
+    return out
+
+
+def dequant_tokens(q: torch.Tensor, scale: torch.Tensor, x_dtype: torch.dtype, dtype: torch.dtype) -> torch.Tensor:
+    """The quantized activations [M, K] that activation_quant holds for an input of `x_dtype`: q / scale[m], as `dtype`."""
+    _need_cuda(q, scale)
+    m, k = q.shape
+    out = torch.empty((m, k), dtype=dtype, device=q.device)
+    with torch.cuda.device(q.device):
+        L.check(L.lib().wf_dequant_tokens(q.data_ptr(), scale.data_ptr(), _DT[x_dtype], out.data_ptr(), _DT[dtype], m, k, _stream()), "wf_dequant_tokens")
+    return out
+
+
 # --------------------------------------------------------------------------
 # the contraction
 # --------------------------------------------------------------------------

@@ -272,6 +272,11 @@ int wf_bitlinear_decode_plan(wf_problem* host_problems, int P);
 int wf_bitlinear_decode_grouped(const wf_problem* dev_problems, const wf_problem* host_problems, int P, unsigned flags,
                                 void* stream);
 
+/* 1 when wf_bitlinear_decode(_grouped) with up to `problems` projections of the same M tokens of width K, `weights` weights in
+ * all, quantizes floating-point tokens inside the launch at no cost worth a launch of its own; 0 when a caller does well
+ * to quantize larger inputs first (wf_act_quant_i8) and pass int8. */
+int wf_decode_fuses_quant(int64_t M, int64_t K, int64_t weights, int problems);
+
 /* Last device-side status of the decode kernels on the current device: 0, or WF_E_LIMIT when a bounded
  * wait inside a kernel ran out (the kernel then finished without hanging; its outputs are invalid).
  * Synchronizes the device. */

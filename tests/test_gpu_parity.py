@@ -832,3 +832,40 @@ def test_dequantized_operands_of_the_backward_pass(wf, m, n, k, xdt, dt):
     s = (torch.rand(m, generator=g) * 60 + 0.01).to(TDT[xdt]).float().to(DEV)
     want = (q.to(TDT[xdt]) / s.to(TDT[xdt]).unsqueeze(1)).to(TDT[dt])
     assert torch.equal(wf.ops.dequant_tokens(q, s, TDT[xdt], TDT[dt]), want)
+
+
+@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("n,k", [(1, 64), (33, 192), (1500, 576), (70, 2304), (2561, 2560), (9, 16384), (300, 8320)])
+def test_projection_of_one_or_two_tokens(wf, m, n, k):
+    """The launch for one or two tokens: rows that no warp's share divides, every count of chunks per lane and more than one
+    segment of them, each type, both layouts, a bias, int8 input, up to four projections of the same tokens, tokens with an
+    infinity or a NaN.  Integers and the fp32 rescale are exact: no tolerance."""
+    L = wf._lib
+    assert wf._lib.lib().wf_decode_fuses_quant(1, 64, 64, 1) == 1
+    rng = np.random.default_rng(m * 31 + n * 7 + k)
+    t = rng.integers(-1, 2, size=(n, k)).astype(np.int8)
+    x = gi.with_outliers(torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)), seed=m + n + k)
+    bias = torch.from_numpy(rng.standard_normal(n).astype(np.float32))
+    lays = (L.LAYOUT_WF16, L.LAYOUT_I2S) if k % 128 == 0 else (L.LAYOUT_WF16,)
+    packed = {lay: wf.pack_codes(torch.from_numpy(t).to(DEV), lay) for lay in lays}
+    for dt in ("bf16", "f16", "f32"):
+        xd = x.to(TDT[dt])
+        q, s = O.act_quant_per_token(xd.float().numpy(), dt)
+        acc = O.int_gemm(q, t)
+        y = torch.from_numpy(O.rescale(acc, s.reshape(-1), 0.0173))
+        for lay, codes in packed.items():
+            got, a = wf.bitlinear(xd.to(DEV), codes, 0.0173, bias=bias.to(DEV), layout=lay, out_dtype=torch.float32, want_acc=True, path="decode")
+            assert np.array_equal(a.cpu().numpy(), acc) and torch.equal(got.cpu(), y + bias), (dt, lay)
+            got = wf.bitlinear(torch.from_numpy(q).to(DEV), codes, 0.0173, layout=lay, x_scale=torch.from_numpy(s.reshape(-1)).to(DEV), path="decode")
+            assert torch.equal(got.cpu(), y), (dt, lay)
+    codes = packed[L.LAYOUT_WF16]
+    xd = x.to(torch.bfloat16).to(DEV)
+    want = wf.bitlinear(xd, codes, 0.0173, path="prefill")
+    group = wf.DecodeGroup([dict(x=xd, codes=codes[: max(1, n // d)], w_scale=0.0173) for d in (1, 2, 3, 5)])
+    for d, got in zip((1, 2, 3, 5), group.run()):
+        assert torch.equal(got, want[:, : max(1, n // d)]), d
+    for bad in (float("inf"), float("nan")):
+        xb = xd.clone()
+        xb[m - 1, k // 2] = bad
+        (y1, a1), (y2, a2) = (wf.bitlinear(xb, codes, 0.0173, out_dtype=torch.float32, want_acc=True, path=path) for path in ("decode", "prefill"))
+        assert torch.equal(a1, a2) and torch.equal(y1.nan_to_num(nan=1e30), y2.nan_to_num(nan=1e30)), bad

@@ -71,6 +71,7 @@ _SIGNATURES = {
                                    _f32, _u32, _p]),
     "wf_bitlinear_decode_plan": (_int, [_p, _int]),
     "wf_bitlinear_decode_grouped": (_int, [_p, _p, _int, _u32, _p]),
+    "wf_decode_fuses_quant": (_int, [_i64, _i64, _i64, _int]),
     "wf_device_status": (_int, []),
     "wf_prefill_workspace_bytes": (_sz, [_i64, _i64]),
     "wf_prefill_workspace_bytes_for": (_sz, [_i64, _i64, _i64]),

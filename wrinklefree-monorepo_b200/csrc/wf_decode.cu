@@ -1456,12 +1456,20 @@ static int dispatch_nt(const wf_problem* dev, const wf_problem& single, const De
 
 static int check_problem(const char* who, const wf_problem& q);
 
+}  // namespace wf
+// few tokens through one projection or a few that share them (wf_gemv.cu)
+bool wf_gemv_takes(const wf_problem* q, int P);
+int wf_gemv_launch(const wf_problem* q, int P, unsigned flags, void* stream);
+namespace wf {
+
 static int run_group(const char* who, const wf_problem* dev, wf_problem* host, int P, bool planned, unsigned flags, void* stream) {
     for (int i = 0; i < P; ++i) {
         if (int rc = check_problem(who, host[i])) return rc;
         WF_REQUIRE(host[i].x_dtype == host[0].x_dtype, "%s: all problems of a group must share x_dtype", who);
     }
     if (int rc = require_device()) return rc;
+    const bool few = wf_gemv_takes(host, P);
+    if (few && !planned) return wf_gemv_launch(host, P, flags, stream);
     GroupPlan g;
     if (planned) {
         // the caller's copy on the device was planned earlier: recompute and compare
@@ -1479,6 +1487,7 @@ static int run_group(const char* who, const wf_problem* dev, wf_problem* host, i
     } else {
         if (int rc = plan_group(host, P, g, true)) return rc;
     }
+    if (few) return wf_gemv_launch(host, P, flags, stream);
     DecodeCfg cfg;
     cfg.P = P; cfg.total_items = g.total_items; cfg.RI = g.RI; cfg.KBmax = g.KBmax; cfg.MTA = g.MTA; cfg.stages = g.stages;
     cfg.stage_bytes = g.stage_bytes; cfg.act_off = g.act_off; cfg.stage_off = g.stage_off; cfg.decoupled = g.decoupled; cfg.cpp = g.cpp; cfg.nbuf = g.nbuf;

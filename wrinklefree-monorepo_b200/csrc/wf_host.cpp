@@ -200,9 +200,10 @@ PyObject* bitlinear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
                                           y.data_ptr(), y_code, ldy, acc_ptr, m, n, k, static_cast<float>(eps), ws.data_ptr(), bytes, flags, stream);
             } else {
                 Quantized pre;  // alive until the launch: its memory goes back to this stream's pool
-                if (rows.scalar_type() != at::kChar && (m >= long_arg(a[13]) || m * k >= long_arg(a[14]))) {
+                if (rows.scalar_type() != at::kChar && (m >= long_arg(a[13]) || m * k >= long_arg(a[14])) && !wf_decode_fuses_quant(m, k, n * k, 1)) {
                     // every CTA of the decode kernel quantizes the tokens of its problem: from this many tokens on one
-                    // quantization kernel in front of it is cheaper (same arithmetic, same bits)
+                    // quantization kernel in front of it is cheaper (same arithmetic, same bits), unless the launch is of
+                    // the kind that does it on the way
                     pre = quantize(rows, false, eps, false, stream);
                     rows = pre.q;
                     xs_ptr = static_cast<const float*>(pre.scale.data_ptr());

@@ -184,7 +184,10 @@ PREQUANT_MIN_ELEMS = 4096   # launches of at most PREQUANT_MAX_PROBLEMS problems
 PREQUANT_MAX_PROBLEMS = 4
 
 
-def _prequant(m: int, k: int, problems: int = 1) -> bool:
+def _prequant(m: int, k: int, problems: int = 1, weights: int = 0) -> bool:
+    """`weights`: weights of all problems, when they read the same tokens: few of them quantize those on the way."""
+    if weights and L.lib().wf_decode_fuses_quant(m, k, weights, problems):
+        return False
     return m >= PREQUANT_MIN_TOKENS or (problems <= PREQUANT_MAX_PROBLEMS and m * k >= PREQUANT_MIN_ELEMS)
 
 
@@ -303,7 +306,10 @@ class DecodeGroup:
         dev = problems[0]["x"].device
         # With many tokens per problem x is quantized once per distinct input by a kernel of its own in run(), and
         # the problems read the int8 copy (otherwise every CTA quantizes the tokens of its problem again).
-        prequant = all(pr["x"].dtype != torch.int8 and _prequant(pr["x"].reshape(-1, pr["x"].shape[-1]).shape[0], pr["x"].shape[-1], len(problems))
+        one_x = all(pr["x"].data_ptr() == problems[0]["x"].data_ptr() and pr["x"].shape == problems[0]["x"].shape for pr in problems)
+        weights = 0 if any(pr.get("xchg") or pr.get("prefetch") is not None for pr in problems) or not one_x else 4 * sum(pr["codes"].numel() for pr in problems)
+        prequant = all(pr["x"].dtype != torch.int8
+                       and _prequant(pr["x"].reshape(-1, pr["x"].shape[-1]).shape[0], pr["x"].shape[-1], len(problems), weights)
                        and not pr.get("x_mode") for pr in problems)
         self._quant = {}  # data_ptr of x -> (x2, q, scale, eps)
         for i, pr in enumerate(problems):

@@ -342,6 +342,11 @@ int wf_add_rmsnorm_bf16(void* h, const void* delta, const void* weight, void* y,
                         void* stream);
 int wf_rope_kv_bf16(void* q, const void* k, const void* v, const float* cos, const float* sin, const int64_t* pos, void* kcache,
                     void* vcache, int64_t B, int nq, int nkv, int D, int T, unsigned flags, void* stream);
+/* wf_rope_kv_bf16 for a whole prompt: q [B, S, nq*D] (rotated in place), k, v [B, S, nkv*D]; token s of a sequence is at position
+ * s, S <= T; D a multiple of 16, tensors 16-byte aligned (apply_rotary_emb over a prompt,
+ * packages/training/src/wrinklefree/models/attention.py:41-64). */
+int wf_rope_kv_prompt_bf16(void* q, const void* k, const void* v, const float* cos, const float* sin, void* kcache, void* vcache, int64_t B,
+                           int64_t S, int nq, int nkv, int D, int64_t T, unsigned flags, void* stream);
 int wf_act_mul_bf16(const void* gate, const void* up, void* out, int64_t n, int mode, unsigned flags, void* stream);
 /*
  * The same two kernels with the per-token int8 quantization of the projection that follows fused in (the reference's

@@ -70,6 +70,26 @@ def test_graphed_step_reads_what_its_predecessor_wrote(wf, B):
     wf.device_status()
 
 
+@pytest.mark.parametrize("B,S,nq,nkv,D,T", [(1, 1, 1, 1, 16, 1), (2, 7, 9, 3, 64, 11), (1, 130, 32, 8, 128, 130), (3, 33, 4, 4, 48, 40)])
+def test_rope_and_cache_write_of_a_prompt(wf, B, S, nq, nkv, D, T):
+    """One launch for the rotation of q and k and the cache write of a prompt: bit for bit the operator chain it stands for;
+    positions behind the prompt stay as they were."""
+    from wrinklefree_monorepo_b200 import ops
+    from wrinklefree_monorepo_b200.decoder import _rope
+
+    dev = torch.device("cuda", 0)
+    g = torch.Generator().manual_seed(B * 100 + S)
+    q, k, v = (torch.randn(B * S, n * D, generator=g).bfloat16().to(dev) for n in (nq, nkv, nkv))
+    ang = torch.rand(T, D // 2, generator=g).to(dev) * 6
+    cos, sin = ang.cos(), ang.sin()
+    kc, vc = (torch.full((B, nkv, T, D), 3.0, dtype=torch.bfloat16, device=dev) for _ in range(2))
+    want_q, want_k = (_rope(t.view(B, S, n, D).transpose(1, 2), cos[:S], sin[:S]) for t, n in ((q, nq), (k, nkv)))
+    ops.rope_kv_prompt_(q, k, v, cos, sin, kc, vc, S)
+    assert torch.equal(q.view(B, S, nq, D).transpose(1, 2), want_q) and torch.equal(kc[:, :, :S], want_k)
+    assert torch.equal(vc[:, :, :S], v.view(B, S, nkv, D).transpose(1, 2))
+    assert bool((kc[:, :, S:] == 3.0).all()) and bool((vc[:, :, S:] == 3.0).all())
+
+
 def test_fused_elementwise_kernels(wf):
     from wrinklefree_monorepo_b200 import ops
 

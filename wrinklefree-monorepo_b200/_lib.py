@@ -79,6 +79,7 @@ _SIGNATURES = {
                                     _f32, _p, _sz, _u32, _p]),
     "wf_add_rmsnorm_bf16": (_int, [_p, _p, _p, _p, _i64, _i64, _f32, _u32, _p]),
     "wf_rope_kv_bf16": (_int, [_p, _p, _p, _p, _p, _p, _p, _p, _i64, _int, _int, _int, _int, _u32, _p]),
+    "wf_rope_kv_prompt_bf16": (_int, [_p, _p, _p, _p, _p, _p, _p, _i64, _i64, _int, _int, _int, _i64, _u32, _p]),
     "wf_act_mul_bf16": (_int, [_p, _p, _p, _i64, _int, _u32, _p]),
     "wf_attn_decode_workspace_bytes": (_sz, [_i64, _int, _int, _int, _int]),
     "wf_attn_decode_bf16": (_int, [_p, _p, _p, _p, _p, _i64, _int, _int, _int, _int, _f32, _p, _sz, _u32, _p]),

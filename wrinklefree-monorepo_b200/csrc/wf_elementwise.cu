@@ -165,6 +165,60 @@ __global__ void rope_kv_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat1
     }
 }
 
+// RoPE + cache write of a whole prompt: token (b, s) at position s.  Query heads are rotated in place, key heads rotated into
+// kcache[b, head, s, :], value heads copied to vcache[b, head, s, :].  One thread per 8 + 8 values of a head (the two halves that
+// rotate into each other).  Every product and difference is rounded by itself, as the operator chain it stands for does (two
+// slices, four products, a difference, a sum, a concatenation, a conversion, for q and for k, and two copies into the
+// cache: 20 launches of about 4 us each on the host).
+__global__ void __launch_bounds__(256) rope_kv_prompt_kernel(__nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v,
+                                                             const float* __restrict__ cosv, const float* __restrict__ sinv,
+                                                             __nv_bfloat16* __restrict__ kcache, __nv_bfloat16* __restrict__ vcache, int S, int nq, int nkv,
+                                                             int D, int T, int64_t total) {
+    pdl_trigger();
+    pdl_wait();
+    const int half = D / 2, parts = half / 8, heads = nq + nkv;
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
+        const int part = static_cast<int>(i % parts);
+        const int64_t hr = i / parts;
+        const int head = static_cast<int>(hr % heads);
+        const int64_t row = hr / heads;  // b * S + s
+        const int s = static_cast<int>(row % S);
+        const int64_t b = row / S;
+        const bool is_q = head < nq;
+        const int hk = head - nq;
+        const __nv_bfloat16* src = is_q ? q + (row * nq + head) * D : k + (row * nkv + hk) * D;
+        __nv_bfloat16* dst = is_q ? q + (row * nq + head) * D : kcache + ((b * nkv + hk) * T + s) * D;
+        const uint4 lo = ld16_chained(src + part * 8), hi = ld16_chained(src + half + part * 8);
+        const uint32_t a[4] = {lo.x, lo.y, lo.z, lo.w}, c[4] = {hi.x, hi.y, hi.z, hi.w};
+        const float4* cp = reinterpret_cast<const float4*>(cosv + static_cast<int64_t>(s) * half + part * 8);
+        const float4* sp = reinterpret_cast<const float4*>(sinv + static_cast<int64_t>(s) * half + part * 8);
+        const float4 c0 = __ldg(cp), c1 = __ldg(cp + 1), s0 = __ldg(sp), s1 = __ldg(sp + 1);
+        const float cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        uint32_t o0[4], o1[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float r0[2], r1[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float x1 = u ? bf_hi(a[e]) : bf_lo(a[e]), x2 = u ? bf_hi(c[e]) : bf_lo(c[e]);
+                r0[u] = __fsub_rn(__fmul_rn(x1, cs[2 * e + u]), __fmul_rn(x2, sn[2 * e + u]));
+                r1[u] = __fadd_rn(__fmul_rn(x2, cs[2 * e + u]), __fmul_rn(x1, sn[2 * e + u]));
+            }
+            o0[e] = pack_bf(r0[0], r0[1]);
+            o1[e] = pack_bf(r1[0], r1[1]);
+        }
+        *reinterpret_cast<uint4*>(dst + part * 8) = make_uint4(o0[0], o0[1], o0[2], o0[3]);
+        *reinterpret_cast<uint4*>(dst + half + part * 8) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
+        if (!is_q) {
+            const __nv_bfloat16* pv = v + (row * nkv + hk) * D;
+            __nv_bfloat16* dv = vcache + ((b * nkv + hk) * T + s) * D;
+            *reinterpret_cast<uint4*>(dv + part * 8) = ld16_chained(pv + part * 8);
+            *reinterpret_cast<uint4*>(dv + half + part * 8) = ld16_chained(pv + half + part * 8);
+        }
+    }
+}
+
 // out = act(g) * u, act = SiLU (mode 0) or ReLU^2 (mode 1); intermediate rounded to bf16 like the unfused chain.
 __device__ __forceinline__ float act_one(float a, int mode) {
     float t;
@@ -301,6 +355,22 @@ extern "C" int wf_rope_kv_bf16(void* q, const void* k, const void* v, const floa
     WF_CUDA(launch(rope_kv_kernel, static_cast<unsigned>(B * (nq + nkv)), static_cast<unsigned>(threads), flags, stream,
                    static_cast<__nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), cos, sin, pos,
                    static_cast<__nv_bfloat16*>(kcache), static_cast<__nv_bfloat16*>(vcache), nq, nkv, D, T));
+    return WF_OK;
+}
+
+extern "C" int wf_rope_kv_prompt_bf16(void* q, const void* k, const void* v, const float* cos, const float* sin, void* kcache, void* vcache,
+                                      int64_t B, int64_t S, int nq, int nkv, int D, int64_t T, unsigned flags, void* stream) {
+    WF_REQUIRE(q && k && v && cos && sin && kcache && vcache, "wf_rope_kv_prompt_bf16: null pointer");
+    WF_REQUIRE(B > 0 && S > 0 && S <= T && T < (1LL << 31) && nq > 0 && nkv > 0 && D > 0 && D % 16 == 0, "wf_rope_kv_prompt_bf16: need S <= T and a head dimension that is a multiple of 16");
+    WF_REQUIRE(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(cos) |
+                 reinterpret_cast<uintptr_t>(sin) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 15) == 0,
+               "wf_rope_kv_prompt_bf16: tensors must be 16-byte aligned");
+    if (int rc = require_device()) return rc;
+    const int64_t total = B * S * (nq + nkv) * (D / 16);
+    const int64_t blocks = (total + 255) / 256, most = 16 * static_cast<int64_t>(num_sms());
+    WF_CUDA(launch(rope_kv_prompt_kernel, static_cast<unsigned>(blocks < most ? blocks : most), 256, flags, stream, static_cast<__nv_bfloat16*>(q),
+                   static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), cos, sin, static_cast<__nv_bfloat16*>(kcache),
+                   static_cast<__nv_bfloat16*>(vcache), static_cast<int>(S), nq, nkv, D, static_cast<int>(T), total));
     return WF_OK;
 }
 

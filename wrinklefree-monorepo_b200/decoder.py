@@ -410,6 +410,10 @@ class TernaryDecoder:
         S = ids.shape[1]
         if S > self.T:
             raise ValueError(f"prompt of {S} tokens exceeds the cache of {self.T}")
+        i_loc = self.i_hi - self.i_lo
+        if (self.dtype == torch.bfloat16 and d % 16 == 0 and cfg.hidden % 8 == 0 and max(cfg.hidden, i_loc, self.nq * d) <= 16384
+                and i_loc % 8 == 0):
+            return self._prefill_done(self._prefill_kernels(ids, all_logits), all_logits, S)
         x = self.embed[ids]  # [B, S, hidden]
         cos, sin = self.cos[:S], self.sin[:S]
         for L in self.layers:
@@ -433,7 +437,46 @@ class TernaryDecoder:
                 act = _rms_norm(act, L["sf"], cfg.subln_eps)
             dn = self._allreduce(ops.bitlinear(act, *L["down"]))
             x = x + dn.view(B, S, cfg.hidden)
-        logits = self._head(_rms_norm(x if all_logits else x[:, -1], self.norm_f, cfg.eps))
+        return self._prefill_done(self._head(_rms_norm(x if all_logits else x[:, -1], self.norm_f, cfg.eps)), all_logits, S)
+
+    def _prefill_kernels(self, ids, all_logits):
+        """The prompt pass on this library's kernels (bf16): residual add + RMSNorm with the quantization that q/k/v resp. gate/up
+        share, RoPE with the cache write, gate activation with the quantization of down.  Only the attention itself is the
+        framework's.  A layer is 11 launches; as a chain of torch operators around the projections it was 50."""
+        cfg, B, d, S = self.cfg, self.B, self.cfg.head_dim, ids.shape[1]
+        M, dev = B * S, self.dev
+
+        def quantized(k):
+            return torch.empty(M, k, dtype=torch.int8, device=dev), torch.empty(M, dtype=torch.float32, device=dev)
+
+        h, delta = self.embed[ids].reshape(M, cfg.hidden), None
+        for L in self.layers:
+            xq, xs = ops.add_rmsnorm_quant_(h, delta, L["n1"], *quantized(cfg.hidden), cfg.eps)
+            q, k, v = (ops.bitlinear(xq, *L[n], x_scale=xs, out_dtype=self.dtype) for n in ("q", "k", "v"))
+            ops.rope_kv_prompt_(q, k, v, self.cos, self.sin, L["kc"], L["vc"], S)
+            a = _causal_attention(q.view(B, S, self.nq, d).transpose(1, 2), L["kc"][:, :, :S], L["vc"][:, :, :S])
+            a = a.transpose(1, 2).reshape(M, self.nq * d)
+            if cfg.subln:
+                aq, as_ = ops.add_rmsnorm_quant_(a, None, L["sa"], *quantized(self.nq * d), cfg.subln_eps)
+                o = ops.bitlinear(aq, *L["o"], x_scale=as_, out_dtype=self.dtype)
+            else:
+                o = ops.bitlinear(a, *L["o"])
+            hq, hs = ops.add_rmsnorm_quant_(h, self._allreduce(o), L["n2"], *quantized(cfg.hidden), cfg.eps)
+            g, u = (ops.bitlinear(hq, *L[n], x_scale=hs, out_dtype=self.dtype) for n in ("gate", "up"))
+            if cfg.subln:
+                act = ops.act_mul(g, u, torch.empty_like(g), cfg.act)
+                actq, acts = ops.add_rmsnorm_quant_(act, None, L["sf"], *quantized(act.shape[1]), cfg.subln_eps)
+            else:
+                actq, acts = ops.act_mul_quant(g, u, *quantized(g.shape[1]), mode=cfg.act)
+            delta = self._allreduce(ops.bitlinear(actq, *L["down"], x_scale=acts, out_dtype=self.dtype))
+        if not all_logits:
+            h, delta = (t.view(B, S, cfg.hidden)[:, -1].contiguous() for t in (h, delta))
+        xf = ops.add_rmsnorm_(h, delta, self.norm_f, torch.empty_like(h), cfg.eps)
+        return self._head(xf.view(B, S, cfg.hidden) if all_logits else xf)
+
+    def _prefill_done(self, logits, all_logits, S):
+        """Full rows of the logits, the greedy next token, the position behind the prompt."""
+        cfg = self.cfg
         if self.tp > 1:  # the prompt pass returns the full rows
             parts = [torch.empty(*logits.shape[:-1], hi - lo, dtype=logits.dtype, device=logits.device)
                      for lo, hi in tpmod.shard_bounds(cfg.vocab, self.tp, 1)]

@@ -414,6 +414,17 @@ def rope_kv_(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tenso
                 "wf_rope_kv_bf16")
 
 
+def rope_kv_prompt_(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, kcache: torch.Tensor,
+                    vcache: torch.Tensor, s: int, pdl: bool = False):
+    """`rope_kv_` for a prompt of `s` tokens per sequence: q [B*s, nq*D] (rotated in place), k, v [B*s, nkv*D]; positions 0 .. s - 1
+    of the caches [B, nkv, T, D] receive the rotated keys and the values."""
+    _need_cuda(q, k, v, cos, sin, kcache, vcache)
+    b, nkv, t, d = kcache.shape
+    with torch.cuda.device(q.device):
+        L.check(L.lib().wf_rope_kv_prompt_bf16(q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), kcache.data_ptr(), vcache.data_ptr(),
+                                               b, s, q.numel() // (b * s * d), nkv, d, t, L.FLAG_PDL if pdl else 0, _stream()), "wf_rope_kv_prompt_bf16")
+
+
 _attn_ws = {}
 
 

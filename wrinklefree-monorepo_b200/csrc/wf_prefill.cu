@@ -68,6 +68,10 @@ __device__ __forceinline__ uint4 lds128p(uint32_t addr) {
 // ~260 cycles even when it succeeds at once (hence the non-blocking first test in mbar_wait); and for few tokens the
 // MMA issue rate (~29 ns per instruction of K = 32 whatever N <= 64) is the floor, so a barrier round trip per
 // 128-wide K block doubled the time: stages of 512 amortise it over sixteen MMAs.
+// A code is expanded to the top bit pair of its byte (factor 64, taken out of the sums at the end: |sum| <= 128 * 128 * 65536 <
+// 2^31).  The left shifts that takes run on the multiplier pipe beside the masks on the logic pipe; right shifts into the
+// bottom bit pair shared the logic pipe with the masks, and the eight expansion warps were what bounded the forms for few tokens.
+constexpr int EXPAND_SHIFT = 6;
 constexpr int SM_BM = 128;   // weight rows per tile
 constexpr int SM_BK = 128;   // K per swizzle atom (128 bytes of int8)
 constexpr int SM_PK = 4;     // atoms per stage: a stage is 512 weights of every row = one 128-byte packed row segment
@@ -170,7 +174,7 @@ __device__ __forceinline__ void epilogue16(const uint32_t (&v)[16], const int* s
     float o[16];
 #pragma unroll
     for (int jt = 0; jt < 16; ++jt) {
-        o[jt] = rescale(static_cast<int>(v[jt]) - rs[jt], iv[jt], s_w);
+        o[jt] = rescale((static_cast<int>(v[jt]) >> EXPAND_SHIFT) - rs[jt], iv[jt], s_w);
         if (has_bias) o[jt] = __fadd_rn(o[jt], bias);
     }
     if (valid >= 16) {
@@ -381,7 +385,7 @@ __global__ void __launch_bounds__(sm_threads<NTOK>(), 1)
         const int grp = (warp - 2) >> 2;
         const int quarter = warp & 3;           // the TMEM lanes this warp may access
         const int r = quarter * 32 + lane;      // weight row inside the tile
-        const uint32_t m = 0x03030303u;
+        const uint32_t m = 0xc0c0c0c0u;
         int sit = 0;
         for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
             for (int g = 0; g < stages; ++g, ++sit) {
@@ -404,16 +408,16 @@ __global__ void __launch_bounds__(sm_threads<NTOK>(), 1)
                     if (p.layout == WF_LAYOUT_WF16) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            v[4 * i] = w[i] & m;
-                            v[4 * i + 1] = (w[i] >> 2) & m;
-                            v[4 * i + 2] = (w[i] >> 4) & m;
-                            v[4 * i + 3] = (w[i] >> 6) & m;
+                            v[4 * i] = (w[i] << 6) & m;
+                            v[4 * i + 1] = (w[i] << 4) & m;
+                            v[4 * i + 2] = (w[i] << 2) & m;
+                            v[4 * i + 3] = w[i] & m;
                         }
                     } else {  // I2_S: byte b of the 32 holds weights b, b + 32, b + 64, b + 96 at bits 7:6, 5:4, 3:2, 1:0
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) v[8 * q + i] = (w[i] >> (6 - 2 * q)) & m;
+                            for (int i = 0; i < 8; ++i) v[8 * q + i] = (w[i] << (2 * q)) & m;
                     }
                     tmem_st32_nowait(dst + jj * 32, v);
                     if (jj == 1) {  // every packed byte of this warp's share is in registers or on its way to tensor memory
@@ -498,7 +502,7 @@ __global__ void __launch_bounds__(sm_threads<NTOK>(), 1)
                         const int tok_in = c0 + jt;
                         if (tok_in < mtok) {
                             const int64_t tok = tok0 + tok_in;
-                            const int acc = static_cast<int>(v[jt]) - s_rowsum[tok_in];
+                            const int acc = (static_cast<int>(v[jt]) >> EXPAND_SHIFT) - s_rowsum[tok_in];
                             float o = rescale(acc, s_inv[tok_in], s_w);
                             if (has_bias) o = __fadd_rn(o, bias);
                             store1_rt(p.y, p.y_dtype, tok * p.ldy + nrow, o);
@@ -713,7 +717,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1)
         const int grp = (warp - 2) >> 2;
         const int quarter = warp & 3;
         const int r = quarter * 32 + lane;
-        const uint32_t m = 0x03030303u;
+        const uint32_t m = 0xc0c0c0c0u;
         int sit = grp;  // this group's tensor-memory stages: grp, grp + 2, ...
         for (int t = cluster_id; t < total_tiles; t += n_clusters) {
             for (int g = grp; g < astages; g += 2, sit += 2) {
@@ -733,16 +737,16 @@ __global__ void __launch_bounds__(SM_THREADS, 1)
                     if (p.layout == WF_LAYOUT_WF16) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            v[jj][4 * i] = w[i] & m;
-                            v[jj][4 * i + 1] = (w[i] >> 2) & m;
-                            v[jj][4 * i + 2] = (w[i] >> 4) & m;
-                            v[jj][4 * i + 3] = (w[i] >> 6) & m;
+                            v[jj][4 * i] = (w[i] << 6) & m;
+                            v[jj][4 * i + 1] = (w[i] << 4) & m;
+                            v[jj][4 * i + 2] = (w[i] << 2) & m;
+                            v[jj][4 * i + 3] = w[i] & m;
                         }
                     } else {
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) v[jj][8 * q + i] = (w[i] >> (6 - 2 * q)) & m;
+                            for (int i = 0; i < 8; ++i) v[jj][8 * q + i] = (w[i] << (2 * q)) & m;
                     }
                 }
                 __syncwarp();
@@ -813,7 +817,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1)
                         const int tok_in = c0 + jt;
                         if (tok_in < mtok) {
                             const int64_t tok = tok0 + tok_in;
-                            const int acc = static_cast<int>(v[jt]) - s_rowsum[tok_in];
+                            const int acc = (static_cast<int>(v[jt]) >> EXPAND_SHIFT) - s_rowsum[tok_in];
                             float o = rescale(acc, s_inv[tok_in], s_w);
                             if (has_bias) o = __fadd_rn(o, bias);
                             store1_rt(p.y, p.y_dtype, tok * p.ldy + nrow, o);

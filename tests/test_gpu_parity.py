@@ -163,6 +163,25 @@ def test_act_quant_many_tokens(wf, k, dt):
     assert torch.equal(q2, q) and torch.equal(s2, s)
 
 
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("eps", [1e-5, 1e-38])
+def test_act_quant_of_every_absolute_maximum(wf, dt, eps):
+    """Every positive finite value of a 16-bit type as the absolute maximum of a token, with both signs: the multiplier is
+    rounded twice (its reciprocal is subnormal for the largest maxima), and no product may leave the range of int8 unclamped.
+    One warp per token, one block per token, and the launch that quantizes a single token itself."""
+    top = torch.arange(1, 0x7F80 if dt == "bf16" else 0x7C00, dtype=torch.int32).to(torch.int16).view(TDT[dt])
+    x = torch.zeros(len(top), 64, dtype=TDT[dt])
+    x[:, 0], x[:, 9], x[:, 18], x[:, 63] = -top, top, -(top / 2), top / 3
+    q, s = O.act_quant_per_token(x.float().numpy(), dt, eps)
+    for rows in (slice(None), slice(len(top) - 20, None)):  # many short rows: a warp each; a few: a block each
+        got, scale = wf.act_quant_i8(x[rows].to(DEV), eps=eps)
+        assert np.array_equal(scale.cpu().numpy(), s[rows]) and np.array_equal(got.cpu().numpy(), q[rows])
+    codes = wf.pack_codes(torch.ones(1, 64, dtype=torch.int8, device=DEV))
+    for i in range(len(top) - 200, len(top), 3):  # the acc of weights that are all 1 is the sum of the codes
+        _, acc = wf.bitlinear(x[i : i + 1].to(DEV), codes, 1.0, eps=eps, want_acc=True, path="decode")
+        assert int(acc) == int(q[i].astype(np.int32).sum()), float(top[i])
+
+
 # ---------------------------------------------------------------- contraction
 @pytest.mark.parametrize("n,k", [(1, 64), (5, 192), (3, 1024), (7, 1088), (130, 960), (64, 4160)])
 @pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])

@@ -155,7 +155,7 @@ __device__ __forceinline__ void quant_token_reg(const void* x, int64_t m, int64_
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < AQ_THREADS / 32; ++i) bits = max(bits, static_cast<uint32_t>(shi[i]));
-    bool fast = finite_bits<DT>(bits);
+    bool fast = fast_bits<DT>(bits);
     float mx = bits_value<DT>(bits);
     if (!fast) {  // uniform over the block
         mx = 0.f;
@@ -219,7 +219,7 @@ __device__ __forceinline__ void quant_token_warp(const void* x, int64_t m, int64
 #pragma unroll
     for (int c = 0; c < NCH; ++c) bits = max_bits8<DT>(r[c], bits);
     bits = warp_max_bits<DT>(bits);
-    bool fast = finite_bits<DT>(bits);
+    bool fast = fast_bits<DT>(bits);
     float mx = bits_value<DT>(bits);
     if (!fast) {  // uniform over the warp
         mx = 0.f;

@@ -160,8 +160,8 @@ __device__ __forceinline__ void gemv_quantize(const GemvParams& p, uint8_t* s_x,
 #pragma unroll
     for (int i = 0; i < WPT; ++i) bits = max(bits, s_red[w0 + i]);
     float mx = bits_value<DT>(bits);
-    bool fast = finite_bits<DT>(bits);
-    if (__syncthreads_or(!fast)) {  // an infinity or a NaN among the tokens
+    bool fast = fast_bits<DT>(bits);
+    if (__syncthreads_or(!fast)) {  // an infinity, a NaN or a maximum out of range among the tokens
         mx = 0.f;
 #pragma unroll
         for (int c = 0; c < GV_XCH; ++c)

@@ -50,9 +50,12 @@ __device__ __forceinline__ void values8(const Raw8<DT>& r, float (&f)[8]) {
 //   * the absolute maximum over bit patterns (non-negative values order like theirs), two 16-bit elements at a time;
 //   * the product with the multiplier as one packed multiplication, which rounds once like the fp32 product of two 16-bit
 //     values (exact) rounded to the type;
-//   * the rounding to an integer as an addition of 1.5 * 2^23 (half to even), whose lowest byte is the int8.  |x * s| stays
-//     below 128.5 (three roundings of at most 2^-9 on top of 127), so only the upper bound of the clamp is needed.
-// A row with an infinity or a NaN, and a multiplier that is not finite, take quantize_one instead.
+//   * the rounding to an integer as an addition of 1.5 * 2^23 (half to even), whose lowest byte is the int8.  Only the upper
+//     bound of the clamp is applied: the multiplier is 127 / max with two roundings of at most 2^-8 each, so |x * s| is below
+//     127 * (1 + 2^-8)^2 = 127.995 and its own rounding ends at 128 at most, which is in range with a minus sign.
+// That needs a maximum whose reciprocal is a normal number of the type: bf16 reciprocals of more than 2^126 are off by up to
+// 1.6 %, x * s reaches -129 there and would wrap to +127.  (fp16 reciprocals of more than 2^14 are off by 2^-9: 127.4.)  Rows
+// with such a maximum, an infinity or a NaN, and a multiplier that is not finite, take quantize_one instead.
 template <int DT>
 __device__ __forceinline__ uint32_t max_bits8(const Raw8<DT>& r, uint32_t mx) {
 #pragma unroll
@@ -70,8 +73,8 @@ __device__ __forceinline__ uint32_t warp_max_bits(uint32_t mx) {
     return __reduce_max_sync(0xffffffffu, mx);
 }
 template <int DT>
-__device__ __forceinline__ bool finite_bits(uint32_t bits) {
-    return bits < (DT == WF_F32 ? 0x7f800000u : (DT == WF_BF16 ? 0x7f80u : 0x7c00u));
+__device__ __forceinline__ bool fast_bits(uint32_t bits) {  // the absolute maximum is one that quantize8_fast takes
+    return bits < (DT == WF_F32 ? 0x7f800000u : (DT == WF_BF16 ? 0x7e81u : 0x7c00u));
 }
 template <int DT>
 __device__ __forceinline__ float bits_value(uint32_t bits) {

@@ -243,8 +243,8 @@ typedef struct WF_ALIGN64 wf_problem {
      *     same way, packages/inference/extern/sglang-bitnet/sgl-kernel/csrc/cpu/bitnet_fused_layer.cpp:150-375);
      *   WF_X_NORM: h = x (+ x2), then h * rsqrt(mean(h^2) + norm_eps) * norm_w (wf_add_rmsnorm_bf16) - the residual add and
      *     RMSNorm in front of q/k/v or gate/up (the A100 stack fuses the quantization into its norm,
-     *     packages/inference/extern/BitNet/gpu/model.py:54-76); h_out (nullable) receives h, written once per launch.
-     * x2 and h_out have the row stride of x. */
+     *     packages/inference/extern/BitNet/gpu/model.py:54-76); h_out (nullable) receives h; problems of a group
+     * may share one or have their own, and every one is written.  x2 and h_out have the row stride of x. */
     const void* x2;
     const void* norm_w;
     void* h_out;

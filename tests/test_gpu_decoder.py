@@ -316,6 +316,29 @@ def test_fused_inputs_of_grouped_projections(wf, oracle_c):
     wf.device_status()
 
 
+@pytest.mark.parametrize("m,k,ns", [(1, 576, (64, 64)), (2, 2560, (640, 200, 640)), (1, 576, (6912, 6000)), (3, 576, (6912, 6000)), (5, 2560, (6912, 6016)),
+                                    (2, 256, (40000, 40000)), (1, 192, (64000, 64000)), (2, 256, (40000, 30000)), (3, 256, (17000,) * 5), (9, 640, (512, 512))])
+def test_every_residual_output_of_a_group_is_written(wf, m, k, ns):
+    """Problems of one group with a residual output of their own: the launch for one or two tokens, the forms where warps share
+    an item or take whole ones, the streaming form with equal and with unequal problems.  The sum of two bf16 tensors rounded once:
+    exact."""
+    from wrinklefree_monorepo_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + k)
+    h, d = (torch.randn(m, k, generator=g, device="cuda").bfloat16() for _ in range(2))
+    w = torch.ones(k, device="cuda").bfloat16()
+    codes = [torch.randint(0, 3, (n, k // 4), generator=g, device="cuda", dtype=torch.uint8) for n in ns]
+    for which in (range(len(ns)), (0,), (len(ns) - 1,), (0, len(ns) - 1)):
+        outs = {i: torch.zeros_like(h) for i in which}
+        grp = ops.DecodeGroup([dict(x=h, x2=d, x_mode="norm", norm_w=w, codes=c, w_scale=0.01, h_out=outs.get(i)) for i, c in enumerate(codes)])
+        for kw in (dict(), dict(pdl=True), dict(pdl=True, x_ready=True)):
+            for o in outs.values():
+                o.zero_()
+            grp.run(**kw)
+            assert all(torch.equal(o, h + d) for o in outs.values()), (list(which), kw)
+    wf.device_status()
+
+
 def test_fused_decode_step_equals_unfused(wf):
     """The six-launch decode step (fused inputs) against the ten-launch step of the same model."""
     from wrinklefree_monorepo_b200.decoder import DecoderConfig, TernaryDecoder

@@ -1055,8 +1055,8 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2)
     const int mvalid0 = uni > 0 ? mv0 : min(cfg.MTA, h0->M - m00);
     const int mvalid1 = npre > 1 ? min(cfg.MTA, (uni > 0 ? single.M : h1->M) - m01) : 0;
     // fused input modes: the CTA that owns the first row item of a (problem, token pass) writes the residual stream
-    const bool wh0 = !early && uni == 0 && h0->h_out != nullptr && (local0 % h0->_row_items) == 0;
-    const bool wh1 = npre > 1 && !early && uni == 0 && h1->h_out != nullptr && (local1 % h1->_row_items) == 0;
+    const bool wh0 = !early && h0->h_out != nullptr && (local0 % h0->_row_items) == 0;
+    const bool wh1 = npre > 1 && !early && h1->h_out != nullptr && (local1 % h1->_row_items) == 0;
     quantize_phase<XDT, STREAM_THREADS, Q_ISSUE>(q0, x0, xs0, cfg.MTA, m00, mvalid0, s_act, s_inv, s_rowsum, s_maxbits, xcache0, s_ss, wh0);
     if (npre > 1)
         quantize_phase<XDT, STREAM_THREADS, Q_ISSUE>(q1, x1, xs1, cfg.MTA, m01, mvalid1, s_act + act_bytes, s_inv + MT, s_rowsum + MT,
@@ -1315,14 +1315,15 @@ static int encode_maps(wf_problem& q) {
     return WF_OK;
 }
 
-// All problems read the same tokens in one pass (q/k/v, gate/up, or a single problem): one quantization serves them all.
+// All problems read the same tokens in one pass (q/k/v, gate/up, or a single problem): one quantization serves them all, and
+// the residual output that goes with it is the first problem's.
 static bool shares_x(const wf_problem* probs, int P, int MTA) {
     if (probs[0].M > MTA || probs[0].M > 8) return false;  // measured with up to 8 tokens (one token tile)
     for (int i = 1; i < P; ++i)
         if (probs[i].x != probs[0].x || probs[i].x_scale != probs[0].x_scale || probs[i].ldx != probs[0].ldx || probs[i].M != probs[0].M ||
             probs[i].K != probs[0].K || probs[i].layout != probs[0].layout || probs[i].eps != probs[0].eps ||
             probs[i].x_mode != probs[0].x_mode || probs[i].x2 != probs[0].x2 || probs[i].norm_w != probs[0].norm_w ||
-            probs[i].norm_eps != probs[0].norm_eps)
+            probs[i].norm_eps != probs[0].norm_eps || (probs[i].h_out && probs[i].h_out != probs[0].h_out))
             return false;
     return true;
 }
@@ -1502,7 +1503,9 @@ static int run_group(const char* who, const wf_problem* dev, wf_problem* host, i
     cfg.prefetch = 0;
     if (P <= 8)
         for (int i = 0; i < P; ++i) cfg.prefetch |= (host[i].prefetch != nullptr && host[i].prefetch_bytes > 0) ? 1 : 0;
-    cfg.x_ready = ((flags & WF_FLAG_X_READY) && !cfg.xchg) ? 1 : 0;  // a pushing launch reads the exchange's step after its predecessors
+    bool waits = cfg.xchg != nullptr;  // a pushing launch reads the exchange's step after its predecessors
+    for (int i = 0; i < P; ++i) waits = waits || host[i].h_out;  // and a residual output is written before the wait of a launch whose x is ready
+    cfg.x_ready = ((flags & WF_FLAG_X_READY) && !waits) ? 1 : 0;
     cfg.wide = (!g.decoupled && g.RI == 1 && g.total_items >= 3LL * g.grid && shares_x(host, P, g.MTA)) ? 1 : 0;
     cfg.items_q = g.total_items / g.grid; cfg.items_r = g.total_items % g.grid;
     cfg.uniform_items = 0;

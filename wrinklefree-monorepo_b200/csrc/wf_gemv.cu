@@ -346,12 +346,16 @@ extern "C" int wf_decode_fuses_quant(int64_t M, int64_t K, int64_t weights, int 
     return gemv_pays(M, K, weights, problems) && gemv_quantizes(M, K) ? 1 : 0;
 }
 
-// Whether it runs the group: worth it, the same tokens for every problem, nothing of what only the kernel for stacks does.
+// Whether it runs the group: worth it, the same tokens for every problem, nothing of what only the kernel for stacks does
+// (an exchange, a prefetch, several residual outputs).
 bool wf_gemv_takes(const wf_problem* q, int P) {
     int64_t weights = 0;
     for (int i = 0; i < P && i < GV_MAX_P; ++i) weights += static_cast<int64_t>(q[i].N) * q[i].K;
     if (!gemv_pays(q[0].M, q[0].K, weights, P) || (q[0].x_dtype != WF_I8 && !gemv_quantizes(q[0].M, q[0].K))) return false;
+    const void* h_out = nullptr;  // the launch writes one residual stream
     for (int i = 0; i < P; ++i) {
+        if (q[i].h_out && h_out && q[i].h_out != h_out) return false;
+        if (q[i].h_out) h_out = q[i].h_out;
         if (q[i].xchg || (q[i].prefetch && q[i].prefetch_bytes > 0)) return false;
         if (q[i].M != q[0].M || q[i].K != q[0].K || q[i].layout != q[0].layout || q[i].x != q[0].x || q[i].ldx != q[0].ldx || q[i].x_scale != q[0].x_scale ||
             q[i].eps != q[0].eps || q[i].x_mode != q[0].x_mode || q[i].x2 != q[0].x2 || q[i].norm_w != q[0].norm_w || q[i].norm_eps != q[0].norm_eps)

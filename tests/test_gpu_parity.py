@@ -182,6 +182,26 @@ def test_act_quant_of_every_absolute_maximum(wf, dt, eps):
         assert int(acc) == int(q[i].astype(np.int32).sum()), float(top[i])
 
 
+@pytest.mark.parametrize("ulps", [0, 1, 2, 3, 5, 7, 1001, (1 << 23) - 1, 1 << 23, (1 << 24) - 1, 1 << 24, (1 << 24) + 2])
+def test_pack_ternary_of_a_tiny_mean(wf, ulps):
+    """eps = 0 lets the mean be zero or subnormal, where half of it is not a number of the type: the codes are those of the
+    quotient w / mean for means up to the smallest with an exact half and beyond.  0 / 0 is a NaN, which the clamp takes to -1."""
+    tiny = 2.0 ** -149  # the smallest positive float
+    for around in (0, 1, max(ulps // 2, 1)):  # +-, so that the mean stays what it is
+        steps = torch.full((4, 64), float(ulps), dtype=torch.float64)
+        steps[:, 0::4] = ulps // 2 + 1
+        steps[:, 1::4] = ulps + (ulps - ulps // 2 - 1)
+        steps[:, 2::8] = ulps - min(around, ulps)
+        steps[:, 6::8] = ulps + min(around, ulps)
+        w = (steps * tiny * torch.where(torch.arange(64) % 3 == 0, -1.0, 1.0)).float()
+        codes, scale = wf.pack_ternary(w.to(DEV), eps=0.0)
+        mean = w.abs().double().mean().float()
+        with np.errstate(invalid="ignore"):
+            want = np.clip(np.nan_to_num(np.rint(w.numpy() / np.float32(mean)), nan=-1.0), -1, 1).astype(np.int8)
+        assert scale[0].item() == mean.item()
+        assert np.array_equal(wf.unpack_codes(codes, 4, 64).cpu().numpy(), want), (ulps, around)
+
+
 # ---------------------------------------------------------------- contraction
 @pytest.mark.parametrize("n,k", [(1, 64), (5, 192), (3, 1024), (7, 1088), (130, 960), (64, 4160)])
 @pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])

@@ -114,7 +114,8 @@ __global__ void __launch_bounds__(PACK_THREADS) abs_sum_kernel(const PackShape s
 //
 // FP32 mode: the code of w is clamp(rint(w / mean), -1, 1) + 1.  The fp32 quotient exceeds 1/2 exactly when w > mean / 2: the
 // next float above mean / 2 is at least half an ulp of 1/2 further in the quotient, and the tie itself rounds to zero.
-// So two comparisons with mean / 2 (exact) stand for the division (which a matrix with a NaN or an infinity keeps).  Cast
+// So two comparisons with mean / 2 stand for the division, wherever mean / 2 is exact: a mean that is subnormal or zero (eps = 0)
+// keeps the division, and so does a matrix with a NaN or an infinity.  Cast
 // modes: the same two comparisons on the rounded product; a NaN compares false with both, the code 0 that the clamp gives it.
 //
 // The comparisons of four weights as masks of four bytes (code = [v > h] + [v >= -h]): six instructions per weight that take
@@ -126,15 +127,15 @@ __device__ __forceinline__ uint32_t signs4(float a, float b, float c, float d) {
     asm("prmt.b32 %0, %1, %2, 0xfbfb;" : "=r"(hi) : "r"(__float_as_uint(c)), "r"(__float_as_uint(d)));
     return __byte_perm(lo, hi, 0x5410);
 }
-// codes of the weights 4 g .. 4 g + 3 of a lane's eight as four bytes.  h = mean / 2 (FP32) or 1/2; `finite`: the sum of all
-// weights is finite, so there is no NaN and no infinity among them and signs of differences decide (FP32 mode).
+// codes of the weights 4 g .. 4 g + 3 of a lane's eight as four bytes.  h = mean / 2 (FP32) or 1/2; `by_sign` (FP32 mode): there is
+// no NaN and no infinity among the weights and h is exact, so the signs of differences decide.
 template <int WDT, int MODE>
-__device__ __forceinline__ uint32_t codes4(const Weights8<WDT>& r, int g, float q_mul, float h, bool finite) {
+__device__ __forceinline__ uint32_t codes4(const Weights8<WDT>& r, int g, float q_mul, float h, bool by_sign) {
     const uint32_t ones = 0x01010101u;
     float f[8];
     weight_values<WDT>(r, f);
     if constexpr (MODE == WF_F32) {
-        if (finite) {
+        if (by_sign) {
             const uint32_t above = signs4(h - f[4 * g], h - f[4 * g + 1], h - f[4 * g + 2], h - f[4 * g + 3]);
             const uint32_t below = signs4(f[4 * g] + h, f[4 * g + 1] + h, f[4 * g + 2] + h, f[4 * g + 3] + h);
             return ones + (above & ones) - (below & ones);
@@ -185,7 +186,8 @@ __global__ void __launch_bounds__(PACK_THREADS)
         scale_out[1] = q_mul;
     }
     const float half = MODE == WF_F32 ? 0.5f * q_mul : 0.5f;
-    const bool finite = total < 1e300;  // also false for a NaN
+    // the sum of all weights is finite (also false for a NaN) and half of the mean is a normal number
+    const bool by_sign = total < 1e300 && half >= 1.17549435e-38f;
     const int lane = threadIdx.x & 31;
     const int64_t code_row = s.len / 4;  // bytes
     for (int64_t back = static_cast<int64_t>(blockIdx.x) * (PACK_THREADS / 32) + (threadIdx.x >> 5); back < s.units;
@@ -199,7 +201,7 @@ __global__ void __launch_bounds__(PACK_THREADS)
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             // weights 0-3 in bit pair 0 of the four bytes, 4-7 in bit pair 1
-            uint32_t c = codes4<WDT, MODE>(r[u], 0, q_mul, half, finite) | (codes4<WDT, MODE>(r[u], 1, q_mul, half, finite) << 2);
+            uint32_t c = codes4<WDT, MODE>(r[u], 0, q_mul, half, by_sign) | (codes4<WDT, MODE>(r[u], 1, q_mul, half, by_sign) << 2);
             c <<= 4 * (lane & 1);  // an odd lane holds the upper half of its word: bit pairs 2 and 3
             word[u] = c | __shfl_xor_sync(0xffffffffu, c, 1);
         }

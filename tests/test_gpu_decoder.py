@@ -364,6 +364,21 @@ def test_fused_decode_step_equals_unfused(wf):
     wf.device_status()
 
 
+def test_prefetch_that_was_asked_for_is_used(wf):
+    """A model whose default is the fused step, which has no prefetch: asking for one selects the separate launches, and their
+    descriptors carry the ranges."""
+    from wrinklefree_monorepo_b200.decoder import DecoderConfig, TernaryDecoder
+
+    cfg = DecoderConfig(layers=2, hidden=576, n_q=9, n_kv=3, head_dim=64, intermediate=1536, vocab=500)
+    dev = torch.device("cuda", 0)
+    assert TernaryDecoder(cfg, 1, 8, dev, seed=2).fused
+    m = TernaryDecoder(cfg, 1, 8, dev, seed=2, prefetch=True)
+    assert not m.fused
+    got = [p.prefetch_bytes for p in m.layers[0]["g_qkv"]._host] + [p.prefetch_bytes for p in m.layers[0]["g_gu"]._host]
+    want = [m.layers[0][n][0].numel() for n in ("o", "gate", "up", "down")] + [m.layers[1]["q"][0].numel()]
+    assert got == want
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 1000, 576), (3, 130, 72), (32, 5000, 4096), (256, 3000, 4096), (300, 1100, 1024), (17, 128, 8)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 def test_linear_bf16_output_head(wf, m, n, k, out_dtype):

@@ -84,8 +84,9 @@ class TernaryDecoder:
         projections (six launches per layer instead of ten), False never.  Every CTA of a projection then repeats the norm
         or the activation, so it pays only for short rows and few of them; measured on B200 per layer: one sequence 27.5 -> 25.1 us
         (576 wide), 45.2 -> 43.3 (2560), 58.8 -> 69.7 (4096); two 29.3 -> 26.9 (576), 47 -> 54 (2560).  By default it is on where it
-        pays: up to 2560 wide for one sequence, up to 1024 for two.  `fuse_exchange` (tensor parallel, up to 8 sequences, bf16): the row-parallel projections push their partial
-        outputs to every rank inside their own launch and the residual add + RMSNorm that follows sums them (default: from two
+        pays: up to 2560 wide for one sequence, up to 1024 for two, and no `prefetch` asked for (the fused
+        step has none).
+        `fuse_exchange` (tensor parallel, up to 8 sequences, bf16): the row-parallel projections push their partial outputs to every rank inside their own launch and the residual add + RMSNorm that follows sums them (default: from two
         sequences on; True / False force it)."""
         self._fuse_opt = fuse
         # tensor parallel, few tokens: False keeps the exchange after o_proj / down_proj a kernel of its own
@@ -194,7 +195,8 @@ class TernaryDecoder:
         alternates between two buffers (a fused launch reads one and writes the other)."""
         cfg, B, d, dev, dt = self.cfg, self.B, self.cfg.head_dim, self.dev, self.dtype
         self.big = B >= 16 and cfg.hidden >= 2048  # projections on the tensor-core contraction for few tokens
-        fuse = self._fuse_opt is True or (self._fuse_opt is None and self.tp == 1 and B <= 2 and cfg.hidden <= (2560 if B == 1 else 1024))
+        fuse = self._fuse_opt is True or (self._fuse_opt is None and not self.prefetch and self.tp == 1 and B <= 2
+                                              and cfg.hidden <= (2560 if B == 1 else 1024))
         self.fused = dt == torch.bfloat16 and not self.big and not cfg.subln and cfg.hidden % 8 == 0 and fuse
         self.h = torch.empty(B, cfg.hidden, dtype=dt, device=dev)
         self.h2 = torch.empty(B, cfg.hidden, dtype=dt, device=dev)

@@ -873,6 +873,25 @@ def test_dequantized_operands_of_the_backward_pass(wf, m, n, k, xdt, dt):
     assert torch.equal(wf.ops.dequant_tokens(q, s, TDT[xdt], TDT[dt]), want)
 
 
+@pytest.mark.parametrize("other", [dict(eps=2e-5), dict(layout=1), dict(prefetch=True), dict()])
+def test_group_that_is_not_one_launch_is_quantized_in_front(wf, other):
+    """Two projections of the same token: one launch quantizes it on the way when both ask for the same; where they differ in
+    what that launch has once, the kernel for stacks runs, and the token is quantized in front of it as for any such group."""
+    k = 4096
+    x = torch.randn(1, k, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1)).bfloat16()
+    t = torch.randint(-1, 2, (300, k), device=DEV, generator=torch.Generator(device=DEV).manual_seed(2)).to(torch.int8)
+    kw = {n: v for n, v in other.items() if n != "prefetch"}
+    first = dict(x=x, codes=wf.pack_codes(t), w_scale=0.5, want_acc=True)
+    second = dict(x=x, codes=wf.pack_codes(t, kw.get("layout", 0)), w_scale=0.5, want_acc=True, **kw)
+    if "prefetch" in other:
+        second["prefetch"] = first["codes"]
+    grp = wf.DecodeGroup([first, second])
+    assert len(grp._quant) == (0 if not other else 2 if "eps" in other else 1)
+    grp.run()
+    want = O.int_gemm(O.act_quant_per_token(x.float().cpu().numpy(), "bf16")[0], t.cpu().numpy())
+    assert all(np.array_equal(a.cpu().numpy(), want) for a in grp.accs)
+
+
 @pytest.mark.parametrize("m", [1, 2])
 @pytest.mark.parametrize("n,k", [(1, 64), (33, 192), (1500, 576), (70, 2304), (2561, 2560), (9, 16384), (300, 8320)])
 def test_projection_of_one_or_two_tokens(wf, m, n, k):

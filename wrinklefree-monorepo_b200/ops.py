@@ -306,8 +306,12 @@ class DecodeGroup:
         dev = problems[0]["x"].device
         # With many tokens per problem x is quantized once per distinct input by a kernel of its own in run(), and
         # the problems read the int8 copy (otherwise every CTA quantizes the tokens of its problem again).
-        one_x = all(pr["x"].data_ptr() == problems[0]["x"].data_ptr() and pr["x"].shape == problems[0]["x"].shape for pr in problems)
-        weights = 0 if any(pr.get("xchg") or pr.get("prefetch") is not None for pr in problems) or not one_x else 4 * sum(pr["codes"].numel() for pr in problems)
+        # A few problems that quantize the same tokens alike, and ask for nothing else, may be one launch that does it on the way.
+        def tokens(pr):
+            return pr["x"].data_ptr(), pr["x"].shape, pr["x"].stride(), pr["x"].dtype, pr.get("layout", L.LAYOUT_WF16), pr.get("eps", 1e-5)
+
+        alike = all(tokens(pr) == tokens(problems[0]) and not pr.get("xchg") and pr.get("prefetch") is None for pr in problems)
+        weights = 4 * sum(pr["codes"].numel() for pr in problems) if alike else 0
         prequant = all(pr["x"].dtype != torch.int8
                        and _prequant(pr["x"].reshape(-1, pr["x"].shape[-1]).shape[0], pr["x"].shape[-1], len(problems), weights)
                        and not pr.get("x_mode") for pr in problems)

@@ -259,6 +259,76 @@ def test_decode_attention_kernel(wf, B, nq, nkv, D, T, pos):
         assert err <= 1e-2, err
 
 
+def test_attention_workspace_of_a_captured_step(wf):
+    """A captured step keeps its own attention workspace: a later, larger attention call and tensors allocated after it leave
+    the replays what the same steps are without a graph."""
+    from wrinklefree_monorepo_b200 import ops
+    from wrinklefree_monorepo_b200.decoder import DecoderConfig, TernaryDecoder
+
+    cfg = DecoderConfig(layers=2, hidden=256, n_q=4, n_kv=2, head_dim=64, intermediate=512, vocab=1000)
+    dev = torch.device("cuda", 0)
+    T = 520  # several tiles per unit: partial results that CTAs merge through the workspace
+    ids = torch.randint(0, cfg.vocab, (1, T), generator=torch.Generator().manual_seed(4)).to(dev)
+    want = []
+    for graphed in (False, True):
+        m = TernaryDecoder(cfg, 1, T, dev, seed=3)
+        if graphed:
+            m.capture()
+            big = torch.zeros(64, 8, 1024, 128, dtype=torch.bfloat16, device=dev)
+            q = torch.zeros(64, 32 * 128, dtype=torch.bfloat16, device=dev)
+            ops.attn_decode(q, big, big, None, torch.empty_like(q))
+            filled = [torch.full((1 << 18,), 255, dtype=torch.uint8, device=dev) for _ in range(64)]
+        m.prefill(ids[:, : T - 6])
+        for t in range(T - 6, T):
+            m.tok.copy_(ids[:, t])
+            m.graph.replay() if graphed else m._decode_step()
+            torch.cuda.synchronize()
+            if graphed:
+                assert torch.equal(m.logits, want[t - T + 6]), t
+            else:
+                want.append(m.logits.clone())
+    assert all(bool((f == 255).all()) for f in filled)
+    wf.device_status()
+
+
+def test_attention_calls_without_a_workspace(wf):
+    """Calls on two streams never share partial results or tickets, a captured call owns its workspace, the kept ones are
+    bounded, and a growing context replaces only its own stream's."""
+    from wrinklefree_monorepo_b200 import ops
+
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(1)
+    ins = []
+    for t in (640, 2048, 320, 4096):
+        kc, vc = (torch.randn(1, 2, t, 64, generator=g, device=dev).bfloat16() for _ in range(2))
+        ins.append((torch.randn(1, 4 * 64, generator=g, device=dev).bfloat16(), kc, vc))
+
+    def call(i):
+        q, kc, vc = ins[i % len(ins)]
+        return ops.attn_decode(q, kc, vc, None, torch.empty_like(q))
+
+    want = [call(i) for i in range(len(ins))]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(ops.ATTN_WORKSPACES + 4)]
+    got = []
+    for i in range(12 * len(streams)):
+        with torch.cuda.stream(streams[i % len(streams)]):
+            got.append((i, call(i + i // len(streams))))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want[(i + i // len(streams)) % len(ins)]) for i, o in got)
+    assert len(ops._attn_ws) <= ops.ATTN_WORKSPACES
+    assert len({ws.data_ptr() for ws in ops._attn_ws.values()}) == len(ops._attn_ws)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = [call(i) for i in range(len(ins))]
+    ops._attn_ws.clear()
+    torch.cuda.empty_cache()
+    for _ in range(2):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(out, want))
+
+
 def test_fused_inputs_of_grouped_projections(wf, oracle_c):
     """The fused input modes of the grouped decode kernel against the unfused kernels of the library: rmsnorm(x + x2)
     in front of a q/k/v-like group (all three forms of the kernel: shared tokens, a single matrix, a streaming

@@ -202,6 +202,7 @@ class TernaryDecoder:
         self.h2 = torch.empty(B, cfg.hidden, dtype=dt, device=dev)
         self.xf = torch.empty(B, cfg.hidden, dtype=dt, device=dev)
         self.head_out = torch.empty(B, self.lm_head.shape[0], dtype=dt, device=dev) if dt == torch.bfloat16 else None
+        self.attn_ws = ops.attn_workspace(B, self.nq, self.nkv, d, self.T, dev)  # captured steps hold its address
         # Tensor parallel, few tokens: the exchange after o_proj / down_proj is fused into those launches (they push their
         # partial outputs to every rank) and into the residual add + RMSNorm that follows (it sums what was pushed).
         self.fuse_exchange = False
@@ -311,7 +312,7 @@ class TernaryDecoder:
             if self.attention == "library":  # the framework's fused kernel, kept as a comparison for the benchmark
                 a = F.scaled_dot_product_attention(q.view(B, self.nq, 1, d), L["kc"], L["vc"], attn_mask=valid, enable_gqa=True)
             else:
-                a = ops.attn_decode(q, L["kc"], L["vc"], self.pos if self.masked else None, L["attn"], pdl=True)
+                a = ops.attn_decode(q, L["kc"], L["vc"], self.pos if self.masked else None, L["attn"], pdl=True, workspace=self.attn_ws)
             # from 16 sequences on the single projections of a wide model run on the tensor-core contraction for few
             # tokens (measured: 14 vs 20 us for 4096 x 4096 at 32 tokens; narrow layers stay faster on the decode kernel)
             big = self.big
@@ -394,7 +395,7 @@ class TernaryDecoder:
                 L["attn"].copy_(F.scaled_dot_product_attention(q.view(self.B, self.nq, 1, cfg.head_dim), L["kc"], L["vc"], attn_mask=valid,
                                                                enable_gqa=True).reshape(self.B, -1))
             else:
-                ops.attn_decode(q, L["kc"], L["vc"], self.pos if self.masked else None, L["attn"], pdl=True)
+                ops.attn_decode(q, L["kc"], L["vc"], self.pos if self.masked else None, L["attn"], pdl=True, workspace=self.attn_ws)
             L["g_o"].run(pdl=True)
             self._allreduce(L["ob"])
             L["g_gu"].run(pdl=True)

@@ -429,27 +429,48 @@ def rope_kv_prompt_(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torc
                                                b, s, q.numel() // (b * s * d), nkv, d, t, L.FLAG_PDL if pdl else 0, _stream()), "wf_rope_kv_prompt_bf16")
 
 
+# Workspaces of attn_decode calls that bring none, by (device, stream): launches of one stream may share one, for they run one
+# after the other, and its memory goes back to that stream.  At most ATTN_WORKSPACES streams keep one.
 _attn_ws = {}
+ATTN_WORKSPACES = 16
+
+
+def attn_workspace(b: int, nq: int, nkv: int, d: int, t: int, device) -> torch.Tensor:
+    """Workspace for `attn_decode` on caches [b, nkv, t, d] with nq query heads: partial results, and tickets that are zero
+    between launches.  Launches that run one after the other may share it, also in other shapes that need no more."""
+    with torch.cuda.device(device):
+        nbytes = L.lib().wf_attn_decode_workspace_bytes(b, nq, nkv, d, t)
+        return torch.zeros(nbytes, dtype=torch.uint8, device=device)
+
+
+def _attn_workspace(b: int, nq: int, nkv: int, d: int, t: int, device) -> torch.Tensor:
+    if torch.cuda.is_current_stream_capturing():  # the graph owns it (and clears its tickets on every replay)
+        return attn_workspace(b, nq, nkv, d, t, device)
+    key = (torch.cuda.current_device(), _stream())
+    ws = _attn_ws.get(key)
+    if ws is None or ws.numel() < L.lib().wf_attn_decode_workspace_bytes(b, nq, nkv, d, t):
+        ws = attn_workspace(b, nq, nkv, d, t, device)
+        _attn_ws.pop(key, None)
+        if len(_attn_ws) >= ATTN_WORKSPACES:
+            _attn_ws.pop(next(iter(_attn_ws), None), None)
+        _attn_ws[key] = ws
+    return ws
 
 
 def attn_decode(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, pos: Optional[torch.Tensor], out: torch.Tensor,
-                scale: Optional[float] = None, pdl: bool = False):
+                scale: Optional[float] = None, pdl: bool = False, workspace: Optional[torch.Tensor] = None):
     """Decode-step attention over the bf16 KV cache: q [B, nq*D] (rotated), caches [B, nkv, T, D], `pos` a device
     scalar (positions 0..pos are attended to; None: all T), out [B, nq*D].  Grouped-query heads share one pass over
-    their keys and values."""
-    _need_cuda(q, kcache, vcache, pos, out)
+    their keys and values.  `workspace`: from `attn_workspace`, kept by the caller (a captured call without one clears its own
+    on every replay)."""
+    _need_cuda(q, kcache, vcache, pos, out, workspace)
     b, nkv, t, d = kcache.shape
     nq = q.numel() // (b * d)
     if q.dtype != torch.bfloat16 or kcache.dtype != torch.bfloat16 or not (kcache.is_contiguous() and vcache.is_contiguous()):
         raise ValueError("attn_decode needs contiguous bf16 tensors")
-    lib = L.lib()
-    nbytes = lib.wf_attn_decode_workspace_bytes(b, nq, nkv, d, t)
-    ws = _attn_ws.get(q.device)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(max(nbytes, 1 << 16), dtype=torch.uint8, device=q.device)
-        _attn_ws[q.device] = ws
     with torch.cuda.device(q.device):
-        L.check(lib.wf_attn_decode_bf16(q.data_ptr(), kcache.data_ptr(), vcache.data_ptr(), _ptr(pos), out.data_ptr(), b, nq, nkv, d, t,
+        ws = workspace if workspace is not None else _attn_workspace(b, nq, nkv, d, t, q.device)
+        L.check(L.lib().wf_attn_decode_bf16(q.data_ptr(), kcache.data_ptr(), vcache.data_ptr(), _ptr(pos), out.data_ptr(), b, nq, nkv, d, t,
                                         float(scale if scale is not None else d ** -0.5), ws.data_ptr(), ws.numel(),
                                         L.FLAG_PDL if pdl else 0, _stream()), "wf_attn_decode_bf16")
     return out

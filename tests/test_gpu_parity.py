@@ -856,6 +856,28 @@ def test_contraction_for_many_tokens_bit_exact(wf, oracle_c, m, n, k):
     wf.device_status()
 
 
+def test_contraction_for_many_tokens_without_room_for_its_weights(wf):
+    """On a card with no room for one byte per weight the call runs in the small workspace: the same bits, no error."""
+    g = torch.Generator(device=DEV).manual_seed(5)
+    m, n, k = 1024, 14336, 4096
+    codes = wf.pack_codes(torch.randint(-1, 2, (n, k), generator=g, device=DEV).to(torch.int8))
+    x = torch.randn(m, k, generator=g, device=DEV).bfloat16()
+    want, out = wf.bitlinear(x, codes, 0.5), torch.zeros(m, n, dtype=torch.bfloat16, device=DEV)
+    assert wf._lib.lib().wf_prefill_workspace_bytes_for(m, n, k) > n * k
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (40 << 20)) / total)
+    try:
+        wf.bitlinear(x, codes, 0.5, out=out)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(out, want) and torch.cuda.max_memory_allocated() - before < n * k
+    wf.device_status()
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 1, 64), (3, 5, 192), (40, 33, 2560), (2, 3, 4160)])
 @pytest.mark.parametrize("xdt", ["f32", "bf16", "f16"])
 @pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])

@@ -97,6 +97,19 @@ Quantized quantize(const at::Tensor& rows, bool per_tensor, double eps, bool wan
     return r;
 }
 
+// The contraction's workspace, one of the call's own: two streams of a device never write the same tokens.  The form for many
+// tokens wants room for one byte per weight; on a card that has none left the call runs the packed form in the smaller one.
+at::Tensor contraction_workspace(int64_t m, int64_t n, int64_t k, const at::TensorOptions& bytes) {
+    const int64_t most = static_cast<int64_t>(wf_prefill_workspace_bytes_for(m, n, k)), least = static_cast<int64_t>(wf_prefill_workspace_bytes(m, k));
+    if (most > least) {
+        try {
+            return at::empty({most}, bytes);
+        } catch (const c10::OutOfMemoryError&) {
+        }
+    }
+    return at::empty({least}, bytes);
+}
+
 PyObject* wrap(const at::Tensor& t) {
     PyObject* o = THPVariable_Wrap(t);
     if (!o) throw PyFailure();
@@ -191,13 +204,12 @@ PyObject* bitlinear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
             const uint8_t* const codes_ptr = static_cast<const uint8_t*>(codes.data_ptr());
             int rc;
             if (contraction) {
-                // a workspace of the call's own: two streams of a device never write the same tokens
-                const size_t bytes = wf_prefill_workspace_bytes_for(m, n, k);
-                const at::Tensor ws = at::empty({static_cast<int64_t>(bytes)}, x.options().dtype(at::kByte));
+                const at::Tensor ws = contraction_workspace(m, n, k, x.options().dtype(at::kByte));
                 const int x_code = dtype_code(rows.scalar_type());
                 pybind11::gil_scoped_release nogil;
                 rc = wf_bitlinear_prefill(rows.data_ptr(), x_code, rows.stride(0), xs_ptr, codes_ptr, layout, ws_dev, ws_host, bias_ptr, bias_type,
-                                          y.data_ptr(), y_code, ldy, acc_ptr, m, n, k, static_cast<float>(eps), ws.data_ptr(), bytes, flags, stream);
+                                          y.data_ptr(), y_code, ldy, acc_ptr, m, n, k, static_cast<float>(eps), ws.data_ptr(),
+                                          static_cast<size_t>(ws.numel()), flags, stream);
             } else {
                 Quantized pre;  // alive until the launch: its memory goes back to this stream's pool
                 if (rows.scalar_type() != at::kChar && (m >= long_arg(a[13]) || m * k >= long_arg(a[14])) && !wf_decode_fuses_quant(m, k, n * k, 1)) {

@@ -268,6 +268,47 @@ def test_packed_weight_cache_invalidation(wf):
     assert not layer._packed
 
 
+def test_host_extension_belongs_to_its_torch(wf, monkeypatch, tmp_path):
+    """The extension of the per-call host path is built against torch's C++ interface: it is built again when torch is another
+    one, and one that was built for another torch is refused when it is loaded."""
+    import importlib.util
+    import subprocess
+
+    import torch
+
+    L = wf._lib
+    spec = importlib.util.spec_from_file_location("_wf_build_under_test", os.path.join(L.HERE, "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    compiled = []
+    real_run = subprocess.run
+
+    def run(cmd, **kw):
+        if not any(str(c).endswith("wf_host.cpp") for c in cmd):
+            return real_run(cmd, **kw)
+        compiled.append(cmd)
+        open(build.HOST_LIB, "w").close()
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+
+    monkeypatch.setattr(build, "HOST_LIB", str(tmp_path / "wf_host.so"))
+    monkeypatch.setattr(build.subprocess, "run", run)
+    build.build_host_extension()
+    build.build_host_extension()
+    assert len(compiled) == 1
+    assert L.host().torch_version == torch.__version__.split("+")[0]
+    monkeypatch.setattr(torch, "__version__", "99.0.0+other")
+    build.build_host_extension()
+    build.build_host_extension()
+    assert len(compiled) == 2
+    monkeypatch.setattr(L, "_host", None)
+    with pytest.raises(RuntimeError, match="build it again for torch 99.0.0"):
+        L.host()
+    (tmp_path / "broken.so").write_bytes(b"not a library")
+    monkeypatch.setattr(L, "HOST_PATH", str(tmp_path / "broken.so"))
+    with pytest.raises(RuntimeError, match="does not load; build it again"):
+        L.host()
+
+
 def test_flags_match_the_header_and_the_stack_rule(wf):
     """The flag values of the Python binding are those of include/wf_b200.h, wf_prefill_quantize validates its
     arguments without a GPU, and the rule that sends a stack of layers to the contraction is monotonic in the token

@@ -140,11 +140,17 @@ def host():
         import importlib.machinery
         import importlib.util
 
-        import torch  # noqa: F401  (the extension links against its libraries)
+        import torch  # the extension links against its libraries and takes its tensors
 
+        rebuild = f"build it again for torch {torch.__version__}: `python __graft_entry__.py build`"
         loader = importlib.machinery.ExtensionFileLoader("wf_host", HOST_PATH)
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("wf_host", HOST_PATH, loader=loader))
-        loader.exec_module(mod)
+        try:
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("wf_host", HOST_PATH, loader=loader))
+            loader.exec_module(mod)
+        except ImportError as e:
+            raise RuntimeError(f"{HOST_PATH} does not load; {rebuild}") from e
+        if getattr(mod, "torch_version", None) != torch.__version__.split("+")[0]:
+            raise RuntimeError(f"{HOST_PATH} was built for torch {getattr(mod, 'torch_version', 'of an unknown version')}; {rebuild}")
         _host = mod
     return _host
 

@@ -76,14 +76,19 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
 
 
 def build_host_extension(force: bool = False) -> str:
-    """Compiles the CPython extension of the per-call host path (csrc/wf_host.cpp) against this interpreter and torch."""
-    src = os.path.join(CSRC, "wf_host.cpp")
-    if not force and not _newer(HOST_LIB, [src, os.path.join(HERE, "..", "include", "wf_b200.h")]):
-        return HOST_LIB
+    """Compiles the CPython extension of the per-call host path (csrc/wf_host.cpp) against this interpreter and torch; again
+    when either of them is another one than that of the last time, which wf_host.built names."""
     import sysconfig
 
     import torch
 
+    src = os.path.join(CSRC, "wf_host.cpp")
+    stamp = os.path.splitext(HOST_LIB)[0] + ".built"
+    against = f"torch {torch.__version__} in {os.path.dirname(torch.__file__)}, python {sys.version}\n"
+    if not force and os.path.exists(stamp) and not _newer(HOST_LIB, [src, os.path.join(HERE, "..", "include", "wf_b200.h")]):
+        with open(stamp) as f:
+            if f.read() == against:
+                return HOST_LIB
     troot = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))) if os.path.sep in _nvcc() else os.path.join(os.sep, "usr", "local", "cuda")
     cmd = [_host_compiler(), "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", HOST_LIB,
@@ -94,6 +99,8 @@ def build_host_extension(force: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("host extension failed:\n" + r.stdout + r.stderr)
+    with open(stamp, "w") as f:
+        f.write(against)
     return HOST_LIB
 
 

@@ -13,6 +13,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
+#include <torch/version.h>
 
 #include "../../include/wf_b200.h"
 
@@ -249,4 +250,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "wf_host", nullptr, -1, methods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_wf_host() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit_wf_host() {
+    PyObject* m = PyModule_Create(&module);
+    // the tensors it takes and returns are torch's C++ objects: the loader compares this with the torch that is running
+    if (m && PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) < 0) Py_CLEAR(m);
+    return m;
+}

@@ -372,8 +372,11 @@ def test_fused_inputs_of_grouped_projections(wf, oracle_c):
     got = ops.DecodeGroup([dict(x=h, x_mode="norm", norm_w=w, norm_eps=1e-6, codes=c, w_scale=s_, out_dtype=torch.float32) for c, s_ in mats]).run(pdl=True)
     for a, b in zip(got, ref):
         assert float((a - b).abs().max() / b.abs().max()) <= 1e-2
-    # activation modes: bit-exact against act_mul + projection
-    for (m, k, n, mode) in ((1, 14336, 4096, "silu"), (4, 1536, 576, "relu2"), (9, 1024, 300, "silu"), (33, 640, 128, "relu2")):
+    # activation modes: bit-exact against act_mul + projection; `few`: on the launch for one or two tokens
+    for (m, k, n, mode, few) in ((1, 14336, 4096, "silu", False), (4, 1536, 576, "relu2", False), (9, 1024, 300, "silu", False),
+                                 (33, 640, 128, "relu2", False), (1, 1536, 576, "silu", True), (1, 6912, 2560, "relu2", True),
+                                 (1, 16384, 70, "silu", True), (2, 1536, 576, "relu2", True), (2, 4096, 2560, "silu", True), (2, 8192, 33, "relu2", True)):
+        assert wf._lib.lib().wf_decode_fuses_quant(m, k, n * k, 1) == few
         gate = torch.randn(m, k, generator=g).bfloat16().to(dev)
         up = torch.randn(m, k, generator=g).bfloat16().to(dev)
         codes, sc = wf.pack_ternary((torch.randn(n, k, generator=g) * 0.02).to(dev))
@@ -409,13 +412,16 @@ def test_every_residual_output_of_a_group_is_written(wf, m, k, ns):
     wf.device_status()
 
 
-def test_fused_decode_step_equals_unfused(wf):
-    """The six-launch decode step (fused inputs) against the ten-launch step of the same model."""
+@pytest.mark.parametrize("B", [1, 2, 3])
+def test_fused_decode_step_equals_unfused(wf, B):
+    """The six-launch decode step (fused inputs) against the ten-launch step of the same model; one and two sequences of a narrow
+    model take it by default, on the launch for so few tokens."""
     from wrinklefree_monorepo_b200.decoder import DecoderConfig, TernaryDecoder
 
     cfg = DecoderConfig(layers=3, hidden=256, n_q=4, n_kv=2, head_dim=64, intermediate=512, vocab=1000)
     dev = torch.device("cuda", 0)
-    B, S, T = 3, 7, 16
+    S, T = 7, 16
+    assert TernaryDecoder(cfg, B, T, dev, seed=2).fused == (B <= 2)
     ids = torch.randint(0, cfg.vocab, (B, S), generator=torch.Generator().manual_seed(6)).to(dev)
     outs = []
     for fuse in (True, False):

@@ -850,9 +850,13 @@ def test_contraction_for_many_tokens_bit_exact(wf, oracle_c, m, n, k):
     rows[:, :k] = torch.from_numpy(q).to(DEV)
     got = wf.bitlinear(rows[:, :k], codes, 0.0173, x_scale=torch.from_numpy(s.reshape(-1)).to(DEV), path="prefill")
     assert torch.equal(got.cpu(), y)
-    out = torch.full((m, n + 3), 7.0, device=DEV)  # a row stride of its own: nothing beyond a row is written
-    wf.bitlinear(x.to(DEV), codes, 0.0173, out=out[:, :n], path="prefill")
-    assert bool((out[:, n:] == 7.0).all())
+    # a row stride of its own, where TMA cannot and (for such n) can write the rows: the values, and nothing beyond a row
+    for dt in ("f32", "bf16"):
+        want = wf.bitlinear(x.to(TDT[dt]).to(DEV), codes, 0.0173, path="prefill")
+        for pad in (3, 16 - n % 8):
+            out = torch.full((m, n + pad), 7.0, dtype=TDT[dt], device=DEV)
+            wf.bitlinear(x.to(TDT[dt]).to(DEV), codes, 0.0173, out=out[:, :n], path="prefill")
+            assert torch.equal(out[:, :n], want) and bool((out[:, n:] == 7.0).all()), (dt, pad)
     wf.device_status()
 
 

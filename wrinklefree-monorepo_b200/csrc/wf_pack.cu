@@ -186,8 +186,8 @@ __global__ void __launch_bounds__(PACK_THREADS)
         scale_out[1] = q_mul;
     }
     const float half = MODE == WF_F32 ? 0.5f * q_mul : 0.5f;
-    // the sum of all weights is finite (also false for a NaN) and half of the mean is a normal number
-    const bool by_sign = total < 1e300 && half >= 1.17549435e-38f;
+    // the sum of all weights is finite (also false for a NaN) and half of the mean is exact: a mean of 2^-125 or more
+    const bool by_sign = total < 1e300 && q_mul >= 2.3509887e-38f;
     const int lane = threadIdx.x & 31;
     const int64_t code_row = s.len / 4;  // bytes
     for (int64_t back = static_cast<int64_t>(blockIdx.x) * (PACK_THREADS / 32) + (threadIdx.x >> 5); back < s.units;

@@ -440,6 +440,18 @@ def test_fused_decode_step_equals_unfused(wf, B):
     wf.device_status()
 
 
+@pytest.mark.parametrize("B,hidden,n_q,n_kv,d,mlp,fused", [(1, 576, 9, 3, 64, 16384, True), (1, 2560, 20, 5, 128, 9600, True), (1, 2560, 20, 5, 128, 11008, False),
+                                                           (1, 2048, 16, 4, 128, 14336, False), (1, 4096, 32, 8, 128, 4096, False), (2, 1024, 16, 4, 64, 4096, True),
+                                                           (2, 1024, 16, 4, 64, 8192, False), (2, 576, 9, 3, 64, 9600, False), (3, 576, 9, 3, 64, 1536, False)])
+def test_default_step_is_fused_only_where_its_launches_take_it(wf, B, hidden, n_q, n_kv, d, mlp, fused):
+    """The rule on widths alone chose the fused step for MLPs whose launches then ran, with the norm or the activation in every
+    block, on the kernel for stacks (up to a third slower per layer)."""
+    from wrinklefree_monorepo_b200.decoder import DecoderConfig, TernaryDecoder
+
+    cfg = DecoderConfig(layers=1, hidden=hidden, n_q=n_q, n_kv=n_kv, head_dim=d, intermediate=mlp, vocab=100)
+    assert TernaryDecoder(cfg, B, 8, torch.device("cuda", 0)).fused == fused
+
+
 def test_prefetch_that_was_asked_for_is_used(wf):
     """A model whose default is the fused step, which has no prefetch: asking for one selects the separate launches, and their
     descriptors carry the ranges."""

@@ -84,8 +84,8 @@ class TernaryDecoder:
         projections (six launches per layer instead of ten), False never.  Every CTA of a projection then repeats the norm
         or the activation, so it pays only for short rows and few of them; measured on B200 per layer: one sequence 27.5 -> 25.1 us
         (576 wide), 45.2 -> 43.3 (2560), 58.8 -> 69.7 (4096); two 29.3 -> 26.9 (576), 47 -> 54 (2560).  By default it is on where it
-        pays: up to 2560 wide for one sequence, up to 1024 for two, and no `prefetch` asked for (the fused
-        step has none).
+        pays (`_fusing_pays`: up to 2560 wide for one sequence, up to 1024 for two, MLPs that its launches take) and no `prefetch` is
+        asked for (the fused step has none).
         `fuse_exchange` (tensor parallel, up to 8 sequences, bf16): the row-parallel projections push their partial outputs to every rank inside their own launch and the residual add + RMSNorm that follows sums them (default: from two
         sequences on; True / False force it)."""
         self._fuse_opt = fuse
@@ -188,6 +188,18 @@ class TernaryDecoder:
         self.next_tok = torch.zeros(batch, dtype=torch.long, device=device)
 
     # ------------------------------------------------------------------ decode step buffers and groups
+    def _fusing_pays(self):
+        """The fused step is the faster one where every launch of it that has an input of its own to compute runs on the kernel
+        for one or two tokens: measured over widths of 576 to 2560 and MLPs of 1536 to 16384, one sequence gains up to 9 % per
+        layer (nothing at the far end of what that kernel takes) and loses 3 to 4 % from the first MLP on that it leaves to the
+        one for stacks (11008 at a width of 2560).  Two sequences gain 1 to 5 % up to an MLP of 4096, are even to 6 % slower up to
+        8192 and 22 to 34 % slower beyond."""
+        cfg, B, d, fuses = self.cfg, self.B, self.cfg.head_dim, ops.L.lib().wf_decode_fuses_quant
+        if B > 2 or cfg.hidden > (2560 if B == 1 else 1024) or (B == 2 and cfg.intermediate > 4096):
+            return False
+        return bool(fuses(B, cfg.hidden, cfg.hidden * (cfg.n_q + 2 * cfg.n_kv) * d, 3) and fuses(B, cfg.hidden, 2 * cfg.hidden * cfg.intermediate, 2)
+                    and fuses(B, cfg.intermediate, cfg.hidden * cfg.intermediate, 1))
+
     def _step_bufs(self):
         """Static buffers and launch groups of the decode step.  Small batches (the projections on the fused
         quantize-and-contract kernel) use the fused input modes: the residual add + RMSNorm runs inside the q/k/v and
@@ -195,8 +207,7 @@ class TernaryDecoder:
         alternates between two buffers (a fused launch reads one and writes the other)."""
         cfg, B, d, dev, dt = self.cfg, self.B, self.cfg.head_dim, self.dev, self.dtype
         self.big = B >= 16 and cfg.hidden >= 2048  # projections on the tensor-core contraction for few tokens
-        fuse = self._fuse_opt is True or (self._fuse_opt is None and not self.prefetch and self.tp == 1 and B <= 2
-                                              and cfg.hidden <= (2560 if B == 1 else 1024))
+        fuse = self._fuse_opt is True or (self._fuse_opt is None and not self.prefetch and self.tp == 1 and self._fusing_pays())
         self.fused = dt == torch.bfloat16 and not self.big and not cfg.subln and cfg.hidden % 8 == 0 and fuse
         self.h = torch.empty(B, cfg.hidden, dtype=dt, device=dev)
         self.h2 = torch.empty(B, cfg.hidden, dtype=dt, device=dev)

@@ -659,6 +659,33 @@ def test_batched_prefill_equals_per_layer_calls(wf, oracle_c):
     wf.device_status()
 
 
+def test_batched_gradients_of_a_training_step(wf, monkeypatch):
+    """Several gradients of one 16-bit step in one call (vmap over the backward pass): the product with fp32 results has no
+    batching rule, so the batched call takes the one that has.  Its dW is rounded to bf16 once more than the single one (half an
+    ulp is 2^-9 of a value; twice that leaves room for sums in another order)."""
+    g = torch.Generator(device=DEV).manual_seed(8)
+    layer = wf.BitLinear(576, 200, bias=True).to(DEV)
+    x = torch.randn(2, 33, 576, generator=g, device=DEV).bfloat16().requires_grad_(True)
+    dy = torch.randn(3, 2, 33, 200, generator=g, device=DEV).bfloat16()
+    y, wanted = layer(x), [x, layer.weight, layer.bias]
+    asked, mm = [], torch.mm
+
+    def counting(*a, **kw):
+        asked.append(kw.get("out_dtype"))
+        return mm(*a, **kw)
+
+    monkeypatch.setattr(torch, "mm", counting)
+    single = [torch.autograd.grad(y, wanted, d, retain_graph=True) for d in dy]
+    assert asked == [torch.float32] * 3
+    batched = torch.autograd.grad(y, wanted, dy, is_grads_batched=True, retain_graph=True)
+    assert asked == [torch.float32] * 3
+    for i in range(3):
+        for a, b in zip(batched, single[i]):
+            assert a[i].dtype == b.dtype and a[i].shape == b.shape
+            assert float((a[i].float() - b.float()).norm()) <= 2.0 ** -8 * float(b.float().norm())
+
+
+
 # ---------------------------------------------------------------- training step on the packed weights
 @pytest.mark.parametrize("dt,tol", [("f32", 1e-5), ("bf16", 2e-2)])
 def test_training_step_on_packed_weights(wf, dt, tol):

@@ -24,6 +24,11 @@ from . import ops
 from .lambda_warmup import get_current_lambda
 
 
+def _batched(t: torch.Tensor) -> bool:
+    """Whether `t` stands for a batch under vmap (`is_grads_batched`, vectorized Jacobians)."""
+    return torch._C._functorch.is_batchedtensor(t) or torch._C._functorch.is_legacy_batchedtensor(t)
+
+
 class _PackedSTE(torch.autograd.Function):
     """Training step of a BitLinear at lambda = 1 on the packed weights (straight-through estimator).
 
@@ -56,8 +61,10 @@ class _PackedSTE(torch.autograd.Function):
             dx = (dy2 @ ops.dequant_weights(codes, scale, dy2.dtype)).reshape(ctx.in_shape)
         if ctx.needs_input_grad[1]:
             x_q = ops.dequant_tokens(q, s, ctx.x_dtype, dy2.dtype)  # the values activation_quant(x) holds
-            if ctx.w_dtype == torch.float32 and dy2.dtype != torch.float32 and not torch.is_grad_enabled():
-                dw = torch.mm(dy2.t(), x_q, out_dtype=torch.float32)  # the fp32 sums as they are, without a pass that widens them
+            if ctx.w_dtype == torch.float32 and dy2.dtype != torch.float32 and not torch.is_grad_enabled() and not _batched(dy2):
+                # the fp32 sums as they are, without a pass that widens them; vmap has no rule for this product and would run
+                # it once per sample (8 gradients of 4096 x (6912 x 2560): 1832 us against 1107 for the other)
+                dw = torch.mm(dy2.t(), x_q, out_dtype=torch.float32)
             else:
                 dw = (dy2.t() @ x_q).to(ctx.w_dtype)
         if ctx.has_bias and ctx.needs_input_grad[2]:

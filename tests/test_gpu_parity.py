@@ -890,7 +890,7 @@ def test_contraction_for_many_tokens_bit_exact(wf, oracle_c, m, n, k):
 def test_contraction_for_many_tokens_without_room_for_its_weights(wf):
     """On a card with no room for one byte per weight the call runs in the small workspace: the same bits, no error."""
     g = torch.Generator(device=DEV).manual_seed(5)
-    m, n, k = 1024, 14336, 4096
+    m, n, k = 2048, 14336, 4096
     codes = wf.pack_codes(torch.randint(-1, 2, (n, k), generator=g, device=DEV).to(torch.int8))
     x = torch.randn(m, k, generator=g, device=DEV).bfloat16()
     want, out = wf.bitlinear(x, codes, 0.5), torch.zeros(m, n, dtype=torch.bfloat16, device=DEV)

@@ -84,7 +84,9 @@ extern "C" {
 #define WF_FLAG_PREFILL_PAIR 4u   /* wf_bitlinear_prefill, more than 64 tokens: use the form in which two CTAs (a cluster of two
                                      SMs, tcgen05 cta_group::2) share each 256-row x 192-token tile (half the token bytes from
                                      L2 per multiply-add; measured slower than the default on B200) */
-#define WF_FLAG_PREFILL_SINGLE 8u /* ... the form with one CTA per 128-row x 128-token tile (the default) */
+#define WF_FLAG_PREFILL_SINGLE 8u /* ... the form with one CTA per 128-row x 128-token tile on packed weights (without either flag: this
+                                     form or, with the workspace of wf_prefill_workspace_bytes_for, the one for many tokens, whichever
+                                     is the faster by the sizes) */
 
 int wf_version(void);
 const char* wf_last_error(void);
@@ -183,7 +185,8 @@ int wf_act_quant_i8(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ld
  * wf_bitlinear_decode: fused per-token activation quantization + contraction for small token counts
  * (decode); any M is accepted, the weights are re-read once per group of tokens that fits in shared memory.
  * wf_bitlinear_prefill: the tensor-core (tcgen05) contraction for large token counts; needs
- * workspace of wf_prefill_workspace_bytes(M, K) bytes when x is not WF_I8.
+ * workspace of wf_prefill_workspace_bytes(M, K) bytes when x is not WF_I8; with that of wf_prefill_workspace_bytes_for it may run
+ * the form for many tokens.
  *
  * Replace: BitLinear.forward at lambda = 1 (packages/training/src/wrinklefree/models/bitlinear.py:86-113),
  *          bitnet_gemv_cpu / bitnet_gemm_cpu (packages/inference/extern/sglang-bitnet/sgl-kernel/csrc/cpu/torch_extension_cpu.cpp:331-407),

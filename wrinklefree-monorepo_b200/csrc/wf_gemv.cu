@@ -96,7 +96,9 @@ __device__ __forceinline__ void gemv_quantize(const GemvParams& p, uint8_t* s_x,
     for (int c = 0; c < GV_XCH; ++c)
         load_raw8<DT>(p.x, base + 8 * (t + c * TPT), live && t + c * TPT < chunks8, r[c]);  // zeros where there is nothing
     if constexpr (DT == WF_BF16) {
-        if (p.x_mode != WF_X_PLAIN) {  // the arithmetic of the stand-alone norm and activation kernels
+        if (p.x_mode != WF_X_PLAIN) {
+            // the arithmetic of the stand-alone kernels: the same bits for the activations; the norm's mean of squares is summed in
+            // another order (square by square, and over other chunks), which may move its last bit and with it single int8 codes
             Raw8<DT> r2[GV_XCH];
 #pragma unroll
             for (int c = 0; c < GV_XCH; ++c)

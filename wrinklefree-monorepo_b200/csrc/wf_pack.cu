@@ -332,7 +332,9 @@ template <int WDT, int MODE>
 static int launch_pack_mode(const PackShape& s, int64_t weights, int grid, float eps, uint8_t* codes, float* scale, double* partial, cudaStream_t st) {
     abs_sum_kernel<WDT, MODE><<<grid, PACK_THREADS, 0, st>>>(s, partial);
     WF_CUDA(cudaGetLastError());
-    cudaLaunchConfig_t lc = {};  // its blocks take the places that the first pass leaves and wait there for its sums
+    // Chained, so that its launch is prepared beside the first pass.  That pass triggers nothing before its end: the blocks of this
+    // one start when all of its blocks have left, and wait for its sums to be visible.
+    cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(static_cast<unsigned>(grid));
     lc.blockDim = dim3(PACK_THREADS);
     lc.stream = st;

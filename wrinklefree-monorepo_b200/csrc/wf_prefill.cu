@@ -953,10 +953,10 @@ static int prefill_impl(const char* who, const void* x, int x_dtype, int64_t ldx
     if (!enc) return fail(WF_E_DEVICE, "cuTensorMapEncodeTiled is not available in this driver");
     const int ntok = M_one <= 16 ? 16 : (M_one <= 32 ? 32 : (M_one <= 64 ? 64 : 128));
     const int sms = num_sms();
-    // Single form (one CTA per 128 x 128 tile) unless the caller asks for the pair form (two CTAs per 256 x PR_N tile):
-    // measured on B200 at M = 512 ... 8192 on the three sweep shapes the single form is the faster one everywhere
-    // (1.41 / 1.68 / 2.13 POPS against 1.22 / 1.58 / 1.79 at M = 8192; a pair tile of 128 tokens with a ring of four
-    // tensor-memory stages was slower still), although the pair form pulls half the token bytes from L2.
+    // Of the two forms on packed weights the single one (one CTA per 128 x 128 tile) unless the caller asks for the pair form (two
+    // CTAs per 256 x PR_N tile): measured on B200 at M = 512 ... 8192 on the three sweep shapes the single form is the faster
+    // of the two everywhere (1.92 / 2.31 / 2.28 POPS at M = 8192 against 2.13 - 2.18 at best; a pair tile of 128 tokens with a ring of
+    // four tensor-memory stages was slower still), although the pair form pulls half the token bytes from L2.
     bool pair = false;
     if (ntok == 128 && (flags & WF_FLAG_PREFILL_PAIR) && !(flags & WF_FLAG_PREFILL_SINGLE)) pair = sms >= 2;
     alignas(64) CUtensorMap tmap_a, tmap_p;

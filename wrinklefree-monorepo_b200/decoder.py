@@ -6,7 +6,8 @@ act(gate) * up -> down BitLinear -> residual; bf16 embedding and lm_head.  Unlik
 KV cache, launches q/k/v and gate/up as one grouped kernel each, and replays the whole decode step as a CUDA
 graph.  With `subln=True` and weights loaded under the reference's parameter names it computes the reference
 model (BitNetLlama) itself.  In the decode step the norms, RoPE + cache write, attention over the cache and the gate
-activation are kernels of this library as well; the prompt pass uses stock torch operators around the projections.
+activation are kernels of this library as well; so they are in the prompt pass of a bf16 model, where only the attention is the
+framework's (an fp32 model, which the parity tests use, runs the prompt on torch operators around the projections).
 
 Tensor parallel: heads and the MLP width are split over the ranks of a process group; q/k/v/gate/up are
 column-parallel, o/down row-parallel with one all-reduce each (the reference's plan); the output head is sharded by

@@ -463,7 +463,8 @@ def prefill_section(wf, torch, device, peak_tops, shapes=None, ms=None):
                         "frac_of_measured_int8": round(tops / peak_tops, 4),
                         "frac_of_nominal_int8_4500": round(tops / 4500.0, 4),
                         "contraction_only": {"us": round(us_c, 2), "TOPS": round(tops_c, 1), "frac_of_measured_int8": round(tops_c / peak_tops, 4),
-                                             "input": "int8 activations + per-token scales given (the operator signature of bitnet_gemm_i2_i8)"}})
+                                             "input": "int8 activations + per-token scales given (the operator signature of bitnet_gemm_i2_i8); with many tokens "
+                                                      "the call also expands the packed weights to one byte each, which the time includes"}})
     return out
 
 

@@ -7,9 +7,10 @@
 // (wf_actquant.cu), into the caller's workspace: the form that expands inside the contraction (wf_prefill.cu) does so again
 // for every 128 tokens and holds the weights in tensor memory, which leaves room for 128 x 128 accumulators.  Here tensor
 // memory holds two accumulators of 256 tokens x 256 weight rows per pair of SMs (cta_group::2) and both operands come by
-// TMA: 32 KB per SM and 8.4 M multiply-adds.  What bounds it (8192 tokens, 6912 x 2560): the instructions alone take
-// 68 us = 4.28 POPS of the 4.58 measured for the instruction, the copies alone 48 us, all of it with the stores of y 88 us: at
-// the full rate operand reads and copies fill the shared-memory port, and every further byte is in their way.
+// TMA: 32 KB per SM and 8.4 M multiply-adds.  What bounds it (8192 tokens, 6912 x 2560): all of it takes 90.5 us = 3.20 POPS, the
+// tensor pipe active 84 % of the cycles under ncu; in one-off variants the instructions alone took 68 us = 4.28 POPS of the 4.58
+// measured for the instruction and the copies alone 48 us: at the full rate operand reads and copies fill the
+// shared-memory port, and every further byte is in their way.
 //   * warp 0 (one lane): TMA of this CTA's 128 tokens and of its half of the weight rows, counted on the leader's barrier;
 //     stages of two 128-byte atoms: with one atom per stage the barrier round trip and commit (about 220 ns per
 //     stage) were the bound of every tile narrower than 256 rows;
@@ -311,8 +312,8 @@ extern "C" int wf_wide_status_fetch(int* out) {
 
 // Weight rows per tile (256, 192, 128 or 64), or 0 where the form that keeps the weights packed (128 x 128 tiles, one per SM)
 // is the faster one.  Both times are estimated in microseconds from what was measured on B200 over M = 128 ... 8192 on seven
-// shapes of 0.9 to 59 Mi weights; over these 70 points the pick is never slower than the packed form, 1.3 % slower than the
-// fastest of the five forms on average and 20 % at worst:
+// shapes of 0.9 to 59 Mi weights; over these 70 points a pick of this form takes 0.60 to 0.93 of the packed form's time, and the
+// pick is 0.4 % slower than the fastest of the five forms on average and 14 % at worst (512 tokens, 6912 x 2560):
 //   packed: waves of 148 tiles x (0.88 per 512 of K + 0.4);
 //   here: waves of 74 tiles x (0.65 / 0.54 / 0.45 / 0.44 per 256 of K for 256 / 192 / 128 / 64 weight rows + 0.4), and the
 //   expansion, 4.2 million weights per microsecond.  (One instruction of K = 32 takes 73 ns at 256 weight rows and still

@@ -382,6 +382,40 @@ int wf_attn_decode_bf16(const void* q, const void* kcache, const void* vcache, c
                         int nkv, int D, int T, float scale, void* workspace, size_t workspace_bytes, unsigned flags, void* stream);
 
 /*
+ * All layers of a ternary decoder for one new token per sequence (bf16), in one launch: a thread-block cluster carries a sequence
+ * through residual add + RMSNorm, q/k/v, RoPE + cache write, attention over the cache, o, residual add + RMSNorm, gate/up, gate
+ * activation and down of every layer, and the final norm.  Per step what the reference's decoder layers compute for a new token
+ * (packages/training/src/wrinklefree/models/transformer.py:80-117, attention.py:126-218, ffn.py:43-87) with the arithmetic of this
+ * library's separate kernels, except the order of fp32 sums and the probabilities of the attention, which stay fp32.
+ * wf_step_layer: device pointers of one layer; codes in WF_LAYOUT_WF16, scales device scalars, norms bf16 [hidden], caches
+ * bf16 [B, nkv, T, D] (rows of 16 bytes, 16-byte aligned like every tensor here).  `layers` is an array of L of them in device memory.
+ * h [B, hidden]: the tokens' embeddings; xf [B, hidden]: the normalised output in front of the head; cos / sin fp32 [T, D/2]; pos:
+ * device scalar, the new token's position (reduced modulo T as in wf_rope_kv_bf16).  act: 0 SiLU, 1 ReLU^2.
+ * wf_decode_layers_cluster: CTAs per sequence (16 or 8) with which all B sequences run at once on this device, to be passed as
+ * `cluster`; 0 when the separate launches are faster or the kernel does not take the shape: D 64 or 128, at most four query heads per KV head, at most 16 KV heads,
+ * widths that are multiples of 64 up to 8192, buffers that fit shared memory.  Takes WF_FLAG_PDL.
+ */
+typedef struct wf_step_layer {
+    const uint8_t* codes[7]; /* q, k, v, o, gate, up, down */
+    const float* scale[7];
+    const void* norm1; /* in front of q/k/v */
+    const void* norm2; /* in front of gate/up */
+    void* kcache;
+    void* vcache;
+} wf_step_layer;
+int wf_decode_layers_cluster(int64_t B, int hidden, int nq, int nkv, int D, int inter, int64_t T);
+int wf_decode_layers_bf16(const wf_step_layer* layers, int L, const void* h, const void* norm_f, void* xf, const float* cos, const float* sin,
+                          const int64_t* pos, int64_t B, int hidden, int nq, int nkv, int D, int inter, int64_t T, int act, float eps,
+                          float quant_eps, float scale, int cluster, unsigned flags, void* stream);
+
+/*
+ * Index of the largest of V bf16 values per row (row stride ld), as torch.argmax picks it: the first of equal ones, the first NaN where
+ * there is one.  out [B].  pos (nullable): a device scalar that one block increments, the position of a decode step.  Takes
+ * WF_FLAG_PDL.
+ */
+int wf_argmax_bf16(const void* x, int64_t ld, int64_t B, int64_t V, int64_t* out, int64_t* pos, unsigned flags, void* stream);
+
+/*
  * Dense bf16 linear layer: y[M, N] = x[M, K] . w[N, K]^T, bf16 operands (row strides ldx, ldw in elements, multiples
  * of 8; x and w 16-byte aligned; K a multiple of 8), fp32 accumulation on the tensor cores, y of y_dtype (WF_F32 /
  * WF_BF16 / WF_F16, row stride ldy).  It is the output head of the ternary decoder, the one matrix the reference keeps

@@ -537,3 +537,68 @@ def test_norm_and_activation_with_fused_quantization(wf, m, k):
         out = torch.empty_like(h0)
         ops.act_mul_quant(h0, up, q, s, mode, out=out)
         assert torch.equal(out, a_ref) and torch.equal(q, q_ref) and torch.equal(s, s_ref)
+
+
+@pytest.mark.parametrize("B,hidden,n_q,n_kv,d,mlp,act,S,steps", [
+    (1, 64, 1, 1, 64, 64, "silu", 3, 4),        # one row group per CTA, one head
+    (3, 256, 4, 2, 64, 512, "relu2", 0, 20),    # from an empty cache, across the edge of a tile
+    (1, 576, 9, 3, 64, 1536, "silu", 76, 8),    # across the edge of a round of tiles (80 positions per CTA)
+    (7, 576, 9, 3, 64, 1536, "silu", 15, 4),    # every cluster that fits
+    (2, 512, 8, 2, 128, 1024, "silu", 250, 4),  # sixteen lanes per position, several rounds
+    (12, 320, 4, 4, 64, 192, "silu", 9, 3)])    # clusters of eight
+def test_all_layers_in_one_launch(wf, B, hidden, n_q, n_kv, d, mlp, act, S, steps):
+    """The step that runs all layers in one launch against the separate launches, teacher-forced: logits within the 3e-2 that int8
+    codes on a rounding edge move them (norm and softmax sums run in another order), caches of the first layer likewise, nothing
+    written behind the position."""
+    from wrinklefree_monorepo_b200.decoder import DecoderConfig, TernaryDecoder
+
+    cfg = DecoderConfig(layers=3, hidden=hidden, n_q=n_q, n_kv=n_kv, head_dim=d, intermediate=mlp, vocab=500, act=act)
+    dev = torch.device("cuda", 0)
+    T = S + steps + 2
+    ids = torch.randint(0, cfg.vocab, (B, S + steps), generator=torch.Generator().manual_seed(B + hidden)).to(dev)
+    ms = [TernaryDecoder(cfg, B, T, dev, seed=2, fuse=fuse) for fuse in (None, False)]
+    assert ms[0].resident is not None and ms[1].resident is None and ms[0].resident.cluster == (8 if B > 8 else 16)
+    outs = []
+    for m in ms:
+        m.capture()
+        for L in m.layers:  # the warm-up steps wrote position 0 and later ones
+            L["kc"].zero_()
+            L["vc"].zero_()
+        if S:
+            m.prefill(ids[:, :S])
+        got = []
+        for t in range(S, S + steps):
+            m.tok.copy_(ids[:, t])
+            m.graph.replay()
+            got.append(m.logits.float().clone())
+        assert int(m.pos) == S + steps
+        assert torch.equal(m.next_tok, m.logits.argmax(-1))
+        assert not any(bool(L[c][:, :, S + steps:].any()) for L in m.layers for c in ("kc", "vc"))
+        outs.append(torch.stack(got))
+    err = float((outs[0] - outs[1]).abs().max() / outs[1].abs().max())
+    assert err <= 3e-2, err
+    for c in ("kc", "vc"):
+        a, b = (m.layers[0][c].float() for m in ms)
+        assert float((a - b).abs().max() / b.abs().max()) <= 2e-2, c
+    wf.device_status()
+
+
+@pytest.mark.parametrize("B,V", [(1, 1), (3, 7), (2, 1000), (1, 49152), (5, 40001)])
+def test_argmax_of_the_head(wf, B, V):
+    """As torch.argmax: ties go to the first, zeros of both signs tie, a NaN is the largest; odd lengths and row strides."""
+    from wrinklefree_monorepo_b200 import ops
+
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(V)
+    rows = torch.randn(B, V + 9, generator=g, device=dev).bfloat16()
+    inputs = [rows[:, :V], rows[:, 1:V + 1], rows[:, :V].contiguous(), torch.zeros(B, V, device=dev).bfloat16() * -1, torch.full((B, V), float("-inf"), device=dev).bfloat16()]
+    inputs.append(inputs[3].clone())
+    inputs[-1][:, V // 2] = 0.0
+    for at in (V - 1, V // 3):
+        x = inputs[2].clone()
+        x[:, at:] = float("nan")
+        inputs.append(x)
+    for i, x in enumerate(inputs):
+        out, pos = torch.full((B,), -1, dtype=torch.long, device=dev), torch.tensor(41, device=dev)
+        ops.argmax_(x, out, pos)
+        assert torch.equal(out, x.argmax(-1)) and int(pos) == 42, i

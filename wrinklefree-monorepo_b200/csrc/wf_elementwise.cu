@@ -281,6 +281,66 @@ __global__ void __launch_bounds__(AMQ_THREADS) act_mul_quant_kernel(const __nv_b
     quantize_row_bf16<AMQ_THREADS, AMQ_CHUNKS>(o, mx, chunks, tid, sh, q + m * I, q_scale + m, q_eps);
 }
 
+// Greedy choice of a decode step: one block per row, 16 bytes per load, several loads in flight.  A framework reduction of 49152 values
+// took 13.6 us, this takes what reading 98 KB through one SM takes.  A value's key orders like the value (bf16 bits made
+// monotone, -0 like +0, every NaN above infinity); ties go to the lowest index.
+constexpr int AM_THREADS = 1024;
+__device__ __forceinline__ uint32_t argmax_key(uint32_t b) {
+    if ((b & 0x7fffu) > 0x7f80u) return 0x1ffffu;
+    if (b == 0x8000u) b = 0;
+    return (b & 0x8000u) ? 0xffffu - b : b + 0x8000u;
+}
+__global__ void __launch_bounds__(AM_THREADS) argmax_kernel(const __nv_bfloat16* x, int64_t ld, int V, int vec, int64_t* __restrict__ out, int64_t* pos) {
+    __shared__ unsigned long long sh[AM_THREADS / 32];
+    pdl_trigger();
+    pdl_wait();
+    const __nv_bfloat16* row = x + static_cast<int64_t>(blockIdx.x) * ld;
+    const int tid = threadIdx.x;
+    uint32_t key = 0;
+    int at = 0x7fffffff;
+    auto take = [&](uint32_t bits, int i) {  // indices of a thread ascend: only a larger key replaces
+        const uint32_t k = argmax_key(bits);
+        if (k > key || at == 0x7fffffff) {
+            key = k;
+            at = i;
+        }
+    };
+    const int n8 = vec ? V >> 3 : 0;
+    constexpr int U = 4;
+    for (int i0 = tid; i0 < n8; i0 += U * AM_THREADS) {
+        uint4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i0 + u * AM_THREADS < n8) v[u] = ld16_chained(row + 8 * static_cast<int64_t>(i0 + u * AM_THREADS));
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i0 + u * AM_THREADS < n8) {
+                const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    take(w[e] & 0xffffu, 8 * (i0 + u * AM_THREADS) + 2 * e);
+                    take(w[e] >> 16, 8 * (i0 + u * AM_THREADS) + 2 * e + 1);
+                }
+            }
+        }
+    }
+    for (int i = 8 * n8 + tid; i < V; i += AM_THREADS) take(*reinterpret_cast<const volatile unsigned short*>(row + i), i);
+    unsigned long long best = (static_cast<unsigned long long>(key) << 32) | (0xffffffffu - static_cast<uint32_t>(at));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if ((tid & 31) == 0) sh[tid >> 5] = best;
+    __syncthreads();
+    if (tid < 32) {
+        best = sh[tid];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+        if (tid == 0) {
+            out[blockIdx.x] = static_cast<int64_t>(0xffffffffu - static_cast<uint32_t>(best));
+            if (pos && blockIdx.x == 0) *pos += 1;
+        }
+    }
+}
+
 template <typename... KArgs, typename... Args>
 static cudaError_t launch(void (*kernel)(KArgs...), unsigned grid, unsigned block, unsigned flags, void* stream, Args... args) {
     cudaLaunchConfig_t lc = {};
@@ -384,5 +444,16 @@ extern "C" int wf_act_mul_bf16(const void* gate, const void* up, void* out, int6
     if (blocks > 148 * 8) blocks = 148 * 8;
     WF_CUDA(launch(act_mul_kernel, static_cast<unsigned>(blocks), 256u, flags, stream, static_cast<const __nv_bfloat16*>(gate),
                    static_cast<const __nv_bfloat16*>(up), static_cast<__nv_bfloat16*>(out), n, mode));
+    return WF_OK;
+}
+
+extern "C" int wf_argmax_bf16(const void* x, int64_t ld, int64_t B, int64_t V, int64_t* out, int64_t* pos, unsigned flags, void* stream) {
+    WF_REQUIRE(x && out, "wf_argmax_bf16: null pointer");
+    WF_REQUIRE(B > 0 && B < (1LL << 31) && V > 0 && V < (1LL << 31) - 16 * AM_THREADS && (ld >= V || B == 1), "wf_argmax_bf16: empty or oversized rows");
+    WF_REQUIRE(reinterpret_cast<uintptr_t>(x) % 2 == 0, "wf_argmax_bf16: x must be 2-byte aligned");
+    if (int rc = require_device()) return rc;
+    const int vec = reinterpret_cast<uintptr_t>(x) % 16 == 0 && (ld % 8 == 0 || B == 1);
+    WF_CUDA(launch(argmax_kernel, static_cast<unsigned>(B), static_cast<unsigned>(AM_THREADS), flags, stream, static_cast<const __nv_bfloat16*>(x), ld,
+                   static_cast<int>(V), vec, out, pos));
     return WF_OK;
 }

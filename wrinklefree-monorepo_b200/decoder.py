@@ -233,6 +233,7 @@ class TernaryDecoder:
         self.qnorm = (dt == torch.bfloat16 and not self.fused and cfg.hidden % 8 == 0 and cfg.hidden <= 16384
                       and ops._prequant(B, cfg.hidden, 2))
         self.qact = (dt == torch.bfloat16 and not self.fused and i_loc % 8 == 0 and i_loc <= 16384 and ops._prequant(B, i_loc, 1))
+        self.resident = self._resident_layers()
         mode = "silu" if cfg.act == "silu" else "relu2"
         prev_down = None
         for li, L in enumerate(self.layers):
@@ -284,6 +285,22 @@ class TernaryDecoder:
                     din = dict(x=L["act_q"], x_scale=L["act_s"]) if self.qact else dict(x=L["actn"] if cfg.subln else L["act"])
                     L["g_down"] = ops.DecodeGroup([dict(codes=L["down"][0], w_scale=L["down"][1], out=L["db"], xchg=xp, **din)])
 
+    def _resident_layers(self):
+        """The launch that runs all layers of a step, or None where it does not pay or something only the separate launches have is
+        asked for."""
+        cfg = self.cfg
+        if (self.tp > 1 or self._fuse_opt is not None or self.prefetch or self.dtype != torch.bfloat16 or cfg.subln or cfg.layers == 0
+                or cfg.n_q % cfg.n_kv):
+            return None
+        cluster = ops.L.lib().wf_decode_layers_cluster(self.B, cfg.hidden, cfg.n_q, cfg.n_kv, cfg.head_dim, cfg.intermediate, self.T)
+        if not cluster:
+            return None
+        names = ("q", "k", "v", "o", "gate", "up", "down")
+        layers = [dict(codes=[L[n][0] for n in names], scales=[L[n][1] for n in names], norms=[L["n1"], L["n2"]], caches=[L["kc"], L["vc"]]) for L in self.layers]
+        if any(t.data_ptr() % 16 for lay in layers for name in ("codes", "norms") for t in lay[name]) or self.norm_f.data_ptr() % 16:
+            return None
+        return ops.DecodeLayers(layers, cfg.hidden, cfg.n_q, cfg.n_kv, cfg.intermediate, cfg.act, cfg.eps, self.norm_f, self.cos, self.sin, cluster)
+
     def _act(self, g, u):
         return (F.silu(g) if self.cfg.act == "silu" else F.relu(g).pow(2)) * u
 
@@ -301,7 +318,10 @@ class TernaryDecoder:
         starts while its predecessor drains (the projections stream their first weights meanwhile) and waits for it
         before it reads an activation."""
         cfg, B, d = self.cfg, self.B, self.cfg.head_dim
-        self.h.copy_(self.embed[self.tok])  # residual stream [B, hidden]
+        torch.ops.aten.index.Tensor_out(self.embed, [self.tok], out=self.h)  # residual stream [B, hidden]
+        if self.resident is not None and self.masked and self.attention == "kernel":
+            self.resident.run(self.h, self.xf, self.pos, pdl=True)
+            return self._greedy(self._head(self.xf, self.head_out, pdl=True), advance=True)
         if self.fused:
             return self._decode_step_fused()
         valid = None
@@ -372,8 +392,7 @@ class TernaryDecoder:
             self._oneshot.reduce_add_rmsnorm_(self.h, self.norm_f, self.xf, cfg.eps, pdl=True)
         else:
             ops.add_rmsnorm_(self.h, delta, self.norm_f, self.xf, cfg.eps, pdl=True)
-        self._greedy(self._head(self.xf, self.head_out, pdl=True))
-        self.pos.add_(1)
+        self._greedy(self._head(self.xf, self.head_out, pdl=True), advance=True)
 
     def _head(self, x, out=None, pdl=False):
         """This rank's rows of the output head: a kernel of this library for bf16, the framework's matmul for the fp32
@@ -382,9 +401,14 @@ class TernaryDecoder:
             return ops.linear_bf16(x, self.lm_head, out=out, pdl=pdl)
         return x @ self.lm_head.t()
 
-    def _greedy(self, logits):
-        """next_tok = argmax over the vocabulary; `logits` are this rank's rows of the head."""
+    def _greedy(self, logits, advance=False):
+        """next_tok = argmax over the vocabulary; `logits` are this rank's rows of the head.  `advance`: the position moves on."""
         self.logits = logits
+        if self.tp == 1 and logits.dtype == torch.bfloat16:
+            ops.argmax_(logits, self.next_tok, self.pos if advance else None, pdl=True)
+            return
+        if advance:
+            self.pos.add_(1)
         if self.tp == 1:
             self.next_tok.copy_(logits.argmax(-1))
             return
@@ -414,8 +438,7 @@ class TernaryDecoder:
             L["g_down"].run(pdl=True)
             self._allreduce(L["db"])
         ops.add_rmsnorm_(self.h, self.layers[-1]["db"], self.norm_f, self.xf, cfg.eps, pdl=True)
-        self._greedy(self._head(self.xf, self.head_out, pdl=True))
-        self.pos.add_(1)
+        self._greedy(self._head(self.xf, self.head_out, pdl=True), advance=True)
 
     # ------------------------------------------------------------------ public
     def prefill(self, ids: torch.Tensor, all_logits: bool = False):

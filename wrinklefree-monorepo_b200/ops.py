@@ -393,6 +393,42 @@ class DecodeGroup:
         return self.outputs
 
 
+def argmax_(x: torch.Tensor, out: torch.Tensor, pos: Optional[torch.Tensor] = None, pdl: bool = False):
+    """out [B] (int64) = x.argmax(-1) of bf16 rows [B, V]; `pos`: an int64 scalar that the launch increments."""
+    _need_cuda(x, out, pos)
+    b, v = x.shape
+    if x.dtype != torch.bfloat16 or out.dtype != torch.long or x.stride(1) != 1 or out.numel() != b or not out.is_contiguous():
+        raise ValueError("argmax_ needs bf16 rows with unit inner stride and a contiguous int64 output of one element per row")
+    with torch.cuda.device(x.device):
+        L.check(L.lib().wf_argmax_bf16(x.data_ptr(), x.stride(0), b, v, out.data_ptr(), _ptr(pos), L.FLAG_PDL if pdl else 0, _stream()), "wf_argmax_bf16")
+    return out
+
+
+class DecodeLayers:
+    """The layers of a decoder for one new token per sequence as one launch (wf_decode_layers_bf16).  `layers`: per layer a dict of
+    "codes" and "scales" (q, k, v, o, gate, up, down), "norms" (two) and "caches" (keys, values); the tensors are kept."""
+
+    def __init__(self, layers, hidden: int, n_q: int, n_kv: int, inter: int, act: str, eps: float, norm_f: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
+                 cluster: int):
+        self._keep = (layers, norm_f, cos, sin)
+        kc = layers[0]["caches"][0]
+        self.device, (self.B, _, self.T, self.D) = kc.device, kc.shape
+        rows = [[_ptr(t) for name in ("codes", "scales", "norms", "caches") for t in lay[name]] for lay in layers]
+        if any(p % 16 for r in rows for p in r[:7] + r[14:]) or any(not t.is_contiguous() for lay in layers for name in ("codes", "norms", "caches") for t in lay[name]):
+            raise ValueError("DecodeLayers needs contiguous, 16-byte aligned tensors")
+        self._dev = torch.tensor(rows, dtype=torch.long).to(self.device)
+        self.hidden, self.n_q, self.n_kv, self.inter, self.act, self.eps, self.cluster = hidden, n_q, n_kv, inter, 0 if act == "silu" else 1, eps, cluster
+
+    def run(self, h: torch.Tensor, xf: torch.Tensor, pos: torch.Tensor, pdl: bool = False):
+        """h [B, hidden]: embeddings; xf: the output of the last layer behind the final norm; pos: int64 scalar."""
+        _, norm_f, cos, sin = self._keep
+        with torch.cuda.device(self.device):
+            L.check(L.lib().wf_decode_layers_bf16(self._dev.data_ptr(), self._dev.shape[0], h.data_ptr(), norm_f.data_ptr(), xf.data_ptr(), cos.data_ptr(),
+                                                  sin.data_ptr(), pos.data_ptr(), self.B, self.hidden, self.n_q, self.n_kv, self.D, self.inter, self.T, self.act,
+                                                  self.eps, 1e-5, self.D ** -0.5, self.cluster, L.FLAG_PDL if pdl else 0, _stream()), "wf_decode_layers_bf16")
+        return xf
+
+
 def add_rmsnorm_(h: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Tensor, out: torch.Tensor, eps: float,
                  pdl: bool = False):
     """h += delta (if given), out = rmsnorm(h) * weight; bf16, contiguous [M, K].  `pdl`: chain the launch to its

@@ -309,6 +309,12 @@ int wf_bitlinear_prefill_batched(const void* x, int x_dtype, int64_t ldx, const 
                                  int32_t* acc_out, int64_t batch, int64_t M, int64_t N, int64_t K, float eps,
                                  void* workspace, size_t workspace_bytes, unsigned flags, void* stream);
 
+/* Several projections of the same quantized tokens in one call: their rows side by side in `codes` [N, K/4] (WF_LAYOUT_WF16) and
+ * `row_scale` [N], the weight scale of each row; y [M, N] (row stride ldy).  workspace as for wf_bitlinear_prefill.  The reference's
+ * fused q/k/v and MLP operators share one quantization in the same way (sgl-kernel/csrc/cpu/bitnet_fused_layer.cpp:150-375). */
+int wf_bitlinear_prefill_rows(const int8_t* x, int64_t ldx, const float* x_scale, const uint8_t* codes, const float* row_scale, void* y, int y_dtype, int64_t ldy,
+                              int64_t M, int64_t N, int64_t K, void* workspace, size_t workspace_bytes, void* stream);
+
 /* The quantization step of wf_bitlinear_prefill(_batched) on its own: per-token absmax int8 codes, scales and row sums
  * of x [M, K] (M = batch * tokens for a batched call) into `workspace` (wf_prefill_workspace_bytes(M, K) bytes), for
  * later calls with WF_FLAG_WS_READY on the same workspace.  Same arithmetic as wf_act_quant_i8 in per-token mode
@@ -350,6 +356,9 @@ int wf_rope_kv_bf16(void* q, const void* k, const void* v, const float* cos, con
  * packages/training/src/wrinklefree/models/attention.py:41-64). */
 int wf_rope_kv_prompt_bf16(void* q, const void* k, const void* v, const float* cos, const float* sin, void* kcache, void* vcache, int64_t B,
                            int64_t S, int nq, int nkv, int D, int64_t T, unsigned flags, void* stream);
+/* ... with row strides of q and of k and v (multiples of 8), for results that lie side by side */
+int wf_rope_kv_prompt_ld_bf16(void* q, int64_t ldq, const void* k, const void* v, int64_t ldkv, const float* cos, const float* sin, void* kcache, void* vcache,
+                              int64_t B, int64_t S, int nq, int nkv, int D, int64_t T, unsigned flags, void* stream);
 int wf_act_mul_bf16(const void* gate, const void* up, void* out, int64_t n, int mode, unsigned flags, void* stream);
 /*
  * The same two kernels with the per-token int8 quantization of the projection that follows fused in (the reference's
@@ -362,6 +371,9 @@ int wf_add_rmsnorm_quant_bf16(void* h, const void* delta, const void* weight, vo
                               int64_t K, float eps, float quant_eps, unsigned flags, void* stream);
 int wf_act_mul_quant_bf16(const void* gate, const void* up, void* out, int8_t* q, float* q_scale, int64_t M, int64_t I, int mode,
                           float quant_eps, unsigned flags, void* stream);
+/* ... with one row stride (a multiple of 8) of gate and up */
+int wf_act_mul_quant_ld_bf16(const void* gate, const void* up, int64_t ld, void* out, int8_t* q, float* q_scale, int64_t M, int64_t I, int mode,
+                             float quant_eps, unsigned flags, void* stream);
 
 /*
  * Decode-step attention over the bf16 KV cache (one new token per sequence, grouped-query heads): for every query head
@@ -380,6 +392,12 @@ int wf_act_mul_quant_bf16(const void* gate, const void* up, void* out, int8_t* q
 size_t wf_attn_decode_workspace_bytes(int64_t B, int nq, int nkv, int D, int T);
 int wf_attn_decode_bf16(const void* q, const void* kcache, const void* vcache, const int64_t* pos, void* out, int64_t B, int nq,
                         int nkv, int D, int T, float scale, void* workspace, size_t workspace_bytes, unsigned flags, void* stream);
+
+/* Causal attention of a prompt on the same caches (the reference model's attention over a prompt, attention.py:186-208): query (b, s) at
+ * row b * S + s of q (row stride ldq, a multiple of 8; rotated) attends to positions 0 .. s; out [B * S, nq * D].  S <= T, D = 64 or
+ * 128, tensors 16-byte aligned.  Takes WF_FLAG_PDL. */
+int wf_attn_prompt_bf16(const void* q, int64_t ldq, const void* kcache, const void* vcache, void* out, int64_t B, int64_t S, int nq, int nkv, int D,
+                        int64_t T, float scale, unsigned flags, void* stream);
 
 /*
  * All layers of a ternary decoder for one new token per sequence (bf16), in one launch: a thread-block cluster carries a sequence

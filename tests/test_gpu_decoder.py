@@ -602,3 +602,48 @@ def test_argmax_of_the_head(wf, B, V):
         out, pos = torch.full((B,), -1, dtype=torch.long, device=dev), torch.tensor(41, device=dev)
         ops.argmax_(x, out, pos)
         assert torch.equal(out, x.argmax(-1)) and int(pos) == 42, i
+
+
+@pytest.mark.parametrize("B,S,nq,nkv,D,T,wide", [(1, 1, 1, 1, 64, 1, 0), (2, 63, 9, 3, 64, 70, 0), (1, 64, 4, 1, 128, 64, 64), (3, 65, 6, 2, 64, 200, 384),
+                                                 (1, 130, 32, 8, 128, 140, 0), (2, 512, 2, 2, 64, 512, 8)])
+def test_prompt_attention_kernel(wf, B, S, nq, nkv, D, T, wide):
+    """Causal attention of a prompt over the caches against fp32 softmax attention: max|a-b| / max|b| <= 1e-2 (probabilities are rounded
+    to bf16 in front of the second product, the output is bf16); positions behind the prompt hold garbage that must not leak in;
+    query rows inside wider rows."""
+    from wrinklefree_monorepo_b200 import ops
+
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(S * 10 + D)
+    q = torch.randn(B * S, nq * D + wide, generator=g, device=dev).bfloat16()[:, :nq * D]
+    kc, vc = (torch.randn(B, nkv, T, D, generator=g, device=dev).bfloat16() for _ in range(2))
+    kc[:, :, S:] = 1e4
+    vc[:, :, S:] = float("nan")
+    out = torch.full((B * S, nq * D), 7.0, dtype=torch.bfloat16, device=dev)
+    ops.attn_prompt(q, kc, vc, out, S)
+    qf = q.float().reshape(B, S, nkv, nq // nkv, D)
+    s = torch.einsum("bshgd,bhtd->bhgst", qf, kc[:, :, :S].float()) * D ** -0.5
+    s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device=dev).triu(1), float("-inf"))
+    ref = torch.einsum("bhgst,bhtd->bshgd", torch.softmax(s, -1), vc[:, :, :S].float()).reshape(B * S, nq * D)
+    err = float((out.float() - ref).abs().max() / ref.abs().max())
+    assert err <= 1e-2, err
+
+
+@pytest.mark.parametrize("m,ns,k", [(1, (64, 64, 64), 64), (17, (100, 28, 130), 576), (64, (576, 192), 128), (65, (576, 192, 192), 576), (121, (1536, 1536), 576),
+                                    (300, (200, 7), 1536), (1000, (1024, 256, 256), 1024)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_projections_side_by_side(wf, m, ns, k, dtype):
+    """Several projections of the same tokens as one contraction with a scale per row: the bits of the separate calls."""
+    from wrinklefree_monorepo_b200 import ops
+
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(m + k)
+    packed = [wf.pack_ternary(torch.randn(n, k, generator=g, device=dev) * 0.02 * (i + 1)) for i, n in enumerate(ns)]
+    q, s = ops.act_quant_i8(torch.randn(m, k, generator=g, device=dev).bfloat16(), eps=1e-5)
+    want = torch.cat([wf.bitlinear(q, c, w, x_scale=s, out_dtype=dtype) for c, w in packed], 1)
+    codes, scales = torch.cat([c for c, _ in packed]), torch.cat([w[:1].expand(c.shape[0]) for c, w in packed])
+    out = torch.full((m, sum(ns) + 8), 7.0, dtype=dtype, device=dev)
+    ops.bitlinear_rows(q, s, codes, scales, out[:, :sum(ns)], ops.rows_workspace(m, [(sum(ns), k)], dev))
+    assert torch.equal(out[:, :sum(ns)], want) and bool((out[:, sum(ns):] == 7.0).all())
+    small = torch.empty(wf._lib.lib().wf_prefill_workspace_bytes(m, k), dtype=torch.uint8, device=dev)  # no room for expanded weights
+    assert torch.equal(ops.bitlinear_rows(q, s, codes, scales, out[:, :sum(ns)], small), want)
+    wf.device_status()

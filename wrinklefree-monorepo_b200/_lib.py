@@ -88,6 +88,10 @@ _SIGNATURES = {
     "wf_linear_bf16": (_int, [_p, _i64, _p, _i64, _p, _int, _i64, _i64, _i64, _i64, _u32, _p]),
     "wf_decode_layers_cluster": (_int, [_i64, _int, _int, _int, _int, _int, _i64]),
     "wf_decode_layers_bf16": (_int, [_p, _int, _p, _p, _p, _p, _p, _p, _i64, _int, _int, _int, _int, _int, _i64, _int, _f32, _f32, _f32, _int, _u32, _p]),
+    "wf_attn_prompt_bf16": (_int, [_p, _i64, _p, _p, _p, _i64, _i64, _int, _int, _int, _i64, _f32, _u32, _p]),
+    "wf_bitlinear_prefill_rows": (_int, [_p, _i64, _p, _p, _p, _p, _int, _i64, _i64, _i64, _i64, _p, _sz, _p]),
+    "wf_rope_kv_prompt_ld_bf16": (_int, [_p, _i64, _p, _p, _i64, _p, _p, _p, _p, _i64, _i64, _int, _int, _int, _i64, _u32, _p]),
+    "wf_act_mul_quant_ld_bf16": (_int, [_p, _p, _i64, _p, _p, _p, _i64, _i64, _int, _f32, _u32, _p]),
     "wf_argmax_bf16": (_int, [_p, _i64, _i64, _i64, _p, _p, _u32, _p]),
     "wf_ar_handle_bytes": (_int, []),
     "wf_ar_init": (_int, [_int, _int, _sz, C.POINTER(C.c_void_p), _p]),

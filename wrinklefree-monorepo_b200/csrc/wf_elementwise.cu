@@ -173,7 +173,7 @@ __global__ void rope_kv_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat1
 __global__ void __launch_bounds__(256) rope_kv_prompt_kernel(__nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v,
                                                              const float* __restrict__ cosv, const float* __restrict__ sinv,
                                                              __nv_bfloat16* __restrict__ kcache, __nv_bfloat16* __restrict__ vcache, int S, int nq, int nkv,
-                                                             int D, int T, int64_t total) {
+                                                             int D, int T, int64_t ldq, int64_t ldkv, int64_t total) {
     pdl_trigger();
     pdl_wait();
     const int half = D / 2, parts = half / 8, heads = nq + nkv;
@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(256) rope_kv_prompt_kernel(__nv_bfloat16* q, c
         const int64_t b = row / S;
         const bool is_q = head < nq;
         const int hk = head - nq;
-        const __nv_bfloat16* src = is_q ? q + (row * nq + head) * D : k + (row * nkv + hk) * D;
-        __nv_bfloat16* dst = is_q ? q + (row * nq + head) * D : kcache + ((b * nkv + hk) * T + s) * D;
+        const __nv_bfloat16* src = is_q ? q + row * ldq + head * D : k + row * ldkv + hk * D;
+        __nv_bfloat16* dst = is_q ? q + row * ldq + head * D : kcache + ((b * nkv + hk) * T + s) * D;
         const uint4 lo = ld16_chained(src + part * 8), hi = ld16_chained(src + half + part * 8);
         const uint32_t a[4] = {lo.x, lo.y, lo.z, lo.w}, c[4] = {hi.x, hi.y, hi.z, hi.w};
         const float4* cp = reinterpret_cast<const float4*>(cosv + static_cast<int64_t>(s) * half + part * 8);
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(256) rope_kv_prompt_kernel(__nv_bfloat16* q, c
         *reinterpret_cast<uint4*>(dst + part * 8) = make_uint4(o0[0], o0[1], o0[2], o0[3]);
         *reinterpret_cast<uint4*>(dst + half + part * 8) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
         if (!is_q) {
-            const __nv_bfloat16* pv = v + (row * nkv + hk) * D;
+            const __nv_bfloat16* pv = v + row * ldkv + hk * D;
             __nv_bfloat16* dv = vcache + ((b * nkv + hk) * T + s) * D;
             *reinterpret_cast<uint4*>(dv + part * 8) = ld16_chained(pv + part * 8);
             *reinterpret_cast<uint4*>(dv + half + part * 8) = ld16_chained(pv + half + part * 8);
@@ -256,7 +256,7 @@ constexpr int AMQ_THREADS = 512;
 constexpr int AMQ_CHUNKS = 4;  // rows up to 16384 elements
 __global__ void __launch_bounds__(AMQ_THREADS) act_mul_quant_kernel(const __nv_bfloat16* g, const __nv_bfloat16* u,
                                                                     __nv_bfloat16* __restrict__ out, int8_t* __restrict__ q,
-                                                                    float* __restrict__ q_scale, int I, int mode, float q_eps) {
+                                                                    float* __restrict__ q_scale, int I, int64_t ldg, int mode, float q_eps) {
     __shared__ float sh[AMQ_THREADS / 32];
     pdl_trigger();
     pdl_wait();
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(AMQ_THREADS) act_mul_quant_kernel(const __nv_b
     for (int c = 0; c < AMQ_CHUNKS; ++c) {
         const int i = tid + c * AMQ_THREADS;
         if (i < chunks) {
-            const uint4 a = ld16_chained(g + m * I + 8 * i), b = ld16_chained(u + m * I + 8 * i);
+            const uint4 a = ld16_chained(g + m * ldg + 8 * i), b = ld16_chained(u + m * ldg + 8 * i);
             const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -392,16 +392,22 @@ extern "C" int wf_add_rmsnorm_quant_bf16(void* h, const void* delta, const void*
 
 extern "C" int wf_act_mul_quant_bf16(const void* gate, const void* up, void* out, int8_t* q, float* q_scale, int64_t M, int64_t I, int mode,
                                      float quant_eps, unsigned flags, void* stream) {
+    return wf_act_mul_quant_ld_bf16(gate, up, I, out, q, q_scale, M, I, mode, quant_eps, flags, stream);
+}
+
+extern "C" int wf_act_mul_quant_ld_bf16(const void* gate, const void* up, int64_t ld, void* out, int8_t* q, float* q_scale, int64_t M, int64_t I, int mode,
+                                        float quant_eps, unsigned flags, void* stream) {
     WF_REQUIRE(gate && up && q && q_scale, "wf_act_mul_quant_bf16: null pointer");
     WF_REQUIRE(M > 0 && M < (1LL << 31) && I > 0 && I % 8 == 0 && I <= static_cast<int64_t>(AMQ_THREADS) * AMQ_CHUNKS * 8 && (mode == 0 || mode == 1),
                "wf_act_mul_quant_bf16: rows of a multiple of 8 elements, at most %d; mode 0 or 1", AMQ_THREADS * AMQ_CHUNKS * 8);
+    WF_REQUIRE(ld >= I && ld % 8 == 0, "wf_act_mul_quant_bf16: the row stride must cover the row and be a multiple of 8");
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     WF_REQUIRE(al16(gate) && al16(up) && (!out || al16(out)) && (reinterpret_cast<uintptr_t>(q) & 7) == 0,
                "wf_act_mul_quant_bf16: tensors must be 16-byte aligned (q: 8)");
     if (int rc = require_device()) return rc;
     WF_CUDA(launch(act_mul_quant_kernel, static_cast<unsigned>(M), static_cast<unsigned>(AMQ_THREADS), flags, stream,
                    static_cast<const __nv_bfloat16*>(gate), static_cast<const __nv_bfloat16*>(up), static_cast<__nv_bfloat16*>(out), q, q_scale,
-                   static_cast<int>(I), mode, quant_eps));
+                   static_cast<int>(I), ld, mode, quant_eps));
     return WF_OK;
 }
 
@@ -420,8 +426,15 @@ extern "C" int wf_rope_kv_bf16(void* q, const void* k, const void* v, const floa
 
 extern "C" int wf_rope_kv_prompt_bf16(void* q, const void* k, const void* v, const float* cos, const float* sin, void* kcache, void* vcache,
                                       int64_t B, int64_t S, int nq, int nkv, int D, int64_t T, unsigned flags, void* stream) {
+    return wf_rope_kv_prompt_ld_bf16(q, static_cast<int64_t>(nq) * D, k, v, static_cast<int64_t>(nkv) * D, cos, sin, kcache, vcache, B, S, nq, nkv, D, T, flags, stream);
+}
+
+extern "C" int wf_rope_kv_prompt_ld_bf16(void* q, int64_t ldq, const void* k, const void* v, int64_t ldkv, const float* cos, const float* sin, void* kcache,
+                                         void* vcache, int64_t B, int64_t S, int nq, int nkv, int D, int64_t T, unsigned flags, void* stream) {
     WF_REQUIRE(q && k && v && cos && sin && kcache && vcache, "wf_rope_kv_prompt_bf16: null pointer");
     WF_REQUIRE(B > 0 && S > 0 && S <= T && T < (1LL << 31) && nq > 0 && nkv > 0 && D > 0 && D % 16 == 0, "wf_rope_kv_prompt_bf16: need S <= T and a head dimension that is a multiple of 16");
+    WF_REQUIRE(ldq >= static_cast<int64_t>(nq) * D && ldkv >= static_cast<int64_t>(nkv) * D && ldq % 8 == 0 && ldkv % 8 == 0,
+               "wf_rope_kv_prompt_bf16: row strides must cover the heads and be multiples of 8");
     WF_REQUIRE(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(cos) |
                  reinterpret_cast<uintptr_t>(sin) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 15) == 0,
                "wf_rope_kv_prompt_bf16: tensors must be 16-byte aligned");
@@ -430,7 +443,7 @@ extern "C" int wf_rope_kv_prompt_bf16(void* q, const void* k, const void* v, con
     const int64_t blocks = (total + 255) / 256, most = 16 * static_cast<int64_t>(num_sms());
     WF_CUDA(launch(rope_kv_prompt_kernel, static_cast<unsigned>(blocks < most ? blocks : most), 256, flags, stream, static_cast<__nv_bfloat16*>(q),
                    static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), cos, sin, static_cast<__nv_bfloat16*>(kcache),
-                   static_cast<__nv_bfloat16*>(vcache), static_cast<int>(S), nq, nkv, D, static_cast<int>(T), total));
+                   static_cast<__nv_bfloat16*>(vcache), static_cast<int>(S), nq, nkv, D, static_cast<int>(T), ldq, ldkv, total));
     return WF_OK;
 }
 

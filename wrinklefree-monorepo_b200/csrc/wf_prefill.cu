@@ -37,6 +37,7 @@ struct PrefillParams {
     const float* x_scale;   // [M] per-token multipliers (nullable: 1)
     const int32_t* rowsum;  // [M]
     const float* w_scale;
+    const float* row_scale;  // [N] one scale per weight row (nullable; takes the place of w_scale)
     float w_scale_host;
     const void* bias;
     int bias_dtype;
@@ -457,7 +458,8 @@ __global__ void __launch_bounds__(sm_threads<NTOK>(), 1)
                 asm volatile("bar.sync 2, %0;\n" ::"n"(128 * EPI_GROUPS) : "memory");
                 cur_zb = zb;
             }
-            const float s_w = p.w_scale ? __ldg(p.w_scale + static_cast<int64_t>(z) * p.w_scale_stride) : p.w_scale_host;
+            const float s_w = p.row_scale ? (row_ok ? __ldg(p.row_scale + nrow) : 0.f)
+                                          : (p.w_scale ? __ldg(p.w_scale + static_cast<int64_t>(z) * p.w_scale_stride) : p.w_scale_host);
             const bool has_bias = p.bias != nullptr;
             const float bias = (has_bias && row_ok) ? load1_rt(p.bias, p.bias_dtype, nrow) : 0.f;
             // These warps share their schedulers with the expansion warps: the per-token work is kept to a handful of
@@ -790,7 +792,8 @@ __global__ void __launch_bounds__(SM_THREADS, 1)
                 asm volatile("bar.sync 2, 256;\n" ::: "memory");
                 cur_zb = zb;
             }
-            const float s_w = p.w_scale ? __ldg(p.w_scale + static_cast<int64_t>(z) * p.w_scale_stride) : p.w_scale_host;
+            const float s_w = p.row_scale ? (row_ok ? __ldg(p.row_scale + nrow) : 0.f)
+                                          : (p.w_scale ? __ldg(p.w_scale + static_cast<int64_t>(z) * p.w_scale_stride) : p.w_scale_host);
             const bool has_bias = p.bias != nullptr;
             const float bias = (has_bias && row_ok) ? load1_rt(p.bias, p.bias_dtype, nrow) : 0.f;
             const int64_t tok0 = static_cast<int64_t>(z) * p.M + tok_base;
@@ -881,7 +884,7 @@ extern "C" int wf_prefill_status_fetch(int* out) {
 
 int wf_quantize_expand(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, float eps, int8_t* q, float* scale, const uint8_t* codes,
                        int layout, int64_t N, int8_t* w8, void* stream);
-int wf_wide_launch(const int8_t* q, int64_t ldq, const float* x_scale, const int8_t* w8, const float* w_scale, float w_scale_host, const void* bias,
+int wf_wide_launch(const int8_t* q, int64_t ldq, const float* x_scale, const int8_t* w8, const float* w_scale, float w_scale_host, const float* row_scale, const void* bias,
                    int bias_dtype, void* y, int y_dtype, int64_t ldy, int64_t M, int64_t N, int64_t K, int bn, void* stream);
 int wf_wide_tile(int64_t M, int64_t N, int64_t K);
 
@@ -900,7 +903,7 @@ extern "C" size_t wf_prefill_workspace_bytes_for(int64_t M, int64_t N, int64_t K
 // `batch` independent problems stacked along the rows: tokens [batch*M, K], weights [batch*N, K/4],
 // outputs [batch*M, N]; problem z uses the weight scale w_scale[z * w_scale_stride].
 static int prefill_impl(const char* who, const void* x, int x_dtype, int64_t ldx, const float* x_scale, const uint8_t* codes,
-                        int layout, const float* w_scale, int64_t w_scale_stride, float w_scale_host, const void* bias,
+                        int layout, const float* w_scale, int64_t w_scale_stride, float w_scale_host, const float* row_scale, const void* bias,
                         int bias_dtype, void* y, int y_dtype, int64_t ldy, int32_t* acc_out, int64_t batch, int64_t M_one,
                         int64_t N, int64_t K, float eps, void* workspace, size_t workspace_bytes, unsigned flags, void* stream) {
     const int64_t M = batch * M_one;  // rows of the stacked activations
@@ -927,7 +930,7 @@ static int prefill_impl(const char* who, const void* x, int x_dtype, int64_t ldx
         int8_t* w8 = reinterpret_cast<int8_t*>(ws + base_bytes);
         if (int rc = wf_quantize_expand(x, x_dtype, M, K, ldx, eps, wq, wscale, codes, layout, N, w8, stream)) return rc;
         const bool given = x_dtype == WF_I8;
-        return wf_wide_launch(given ? static_cast<const int8_t*>(x) : wq, given ? ldx : K, given ? x_scale : wscale, w8, w_scale, w_scale_host, bias,
+        return wf_wide_launch(given ? static_cast<const int8_t*>(x) : wq, given ? ldx : K, given ? x_scale : wscale, w8, w_scale, w_scale_host, row_scale, bias,
                               bias_dtype, y, y_dtype, ldy, M, N, K, wide_bn, stream);
     }
 
@@ -980,7 +983,7 @@ static int prefill_impl(const char* who, const void* x, int x_dtype, int64_t ldx
         if (r != CUDA_SUCCESS) return fail(WF_E_DEVICE, "cuTensorMapEncodeTiled (packed weights) failed with %d", (int)r);
     }
     PrefillParams pp;
-    pp.x_scale = qs; pp.rowsum = wsum; pp.w_scale = w_scale; pp.w_scale_host = w_scale_host; pp.bias = bias;
+    pp.x_scale = qs; pp.rowsum = wsum; pp.w_scale = w_scale; pp.row_scale = row_scale; pp.w_scale_host = w_scale_host; pp.bias = bias;
     pp.bias_dtype = bias_dtype; pp.y = y; pp.y_dtype = y_dtype; pp.ldy = ldy; pp.acc_out = acc_out;
     pp.M = static_cast<int>(M_one); pp.N = static_cast<int>(N); pp.K = static_cast<int>(K); pp.layout = layout;
     pp.batch = static_cast<int>(batch); pp.w_scale_stride = static_cast<int>(w_scale_stride);
@@ -1040,7 +1043,7 @@ extern "C" int wf_bitlinear_prefill(const void* x, int x_dtype, int64_t ldx, con
                                     int layout, const float* w_scale, float w_scale_host, const void* bias, int bias_dtype,
                                     void* y, int y_dtype, int64_t ldy, int32_t* acc_out, int64_t M, int64_t N, int64_t K,
                                     float eps, void* workspace, size_t workspace_bytes, unsigned flags, void* stream) {
-    return prefill_impl("wf_bitlinear_prefill", x, x_dtype, ldx, x_scale, codes, layout, w_scale, 0, w_scale_host, bias,
+    return prefill_impl("wf_bitlinear_prefill", x, x_dtype, ldx, x_scale, codes, layout, w_scale, 0, w_scale_host, nullptr, bias,
                         bias_dtype, y, y_dtype, ldy, acc_out, 1, M, N, K, eps, workspace, workspace_bytes, flags, stream);
 }
 
@@ -1051,8 +1054,15 @@ extern "C" int wf_bitlinear_prefill_batched(const void* x, int x_dtype, int64_t 
     WF_REQUIRE(w_scale, "wf_bitlinear_prefill_batched: w_scale must point to the per-problem scales");
     WF_REQUIRE(x_dtype != WF_I8, "wf_bitlinear_prefill_batched: takes floating-point activations");
     return prefill_impl("wf_bitlinear_prefill_batched", x, x_dtype, ldx, nullptr, codes, layout, w_scale, w_scale_stride, 0.f,
-                        nullptr, 0, y, y_dtype, ldy, acc_out, batch, M, N, K, eps, workspace, workspace_bytes,
+                        nullptr, nullptr, 0, y, y_dtype, ldy, acc_out, batch, M, N, K, eps, workspace, workspace_bytes,
                         flags & (WF_FLAG_WS_READY | WF_FLAG_X_READY), stream);
+}
+
+extern "C" int wf_bitlinear_prefill_rows(const int8_t* x, int64_t ldx, const float* x_scale, const uint8_t* codes, const float* row_scale, void* y, int y_dtype,
+                                         int64_t ldy, int64_t M, int64_t N, int64_t K, void* workspace, size_t workspace_bytes, void* stream) {
+    WF_REQUIRE(row_scale, "wf_bitlinear_prefill_rows: row_scale must point to N scales");
+    return prefill_impl("wf_bitlinear_prefill_rows", x, WF_I8, ldx, x_scale, codes, WF_LAYOUT_WF16, nullptr, 0, 0.f, row_scale, nullptr, 0, y, y_dtype, ldy, nullptr, 1,
+                        M, N, K, 0.f, workspace, workspace_bytes, 0, stream);
 }
 
 int wf_act_quant_token_ready(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, float eps, int8_t* q, float* scale,

@@ -44,6 +44,7 @@ static_assert(WD_SMEM <= 227 * 1024, "shared memory");
 struct WideParams {
     const float* x_scale;  // [M] per-token multipliers (nullable: 1)
     const float* w_scale;
+    const float* row_scale;  // [N] one scale per weight row (nullable; takes the place of w_scale)
     float w_scale_host;
     const void* bias;
     int bias_dtype;
@@ -217,8 +218,18 @@ __global__ void __launch_bounds__(WD_THREADS, 1)
                 }
                 if (tok0 >= p.M || col0 + c >= p.N) continue;  // nothing of this box exists (uniform over the warp)
                 float o[COLS];
+                if (p.row_scale) {
 #pragma unroll
-                for (int j = 0; j < COLS; ++j) o[j] = rescale(static_cast<int>(v[j]), inv, s_w);
+                    for (int j = 0; j < COLS; j += 32) {
+                        const int n = col0 + c + j + lane;
+                        const float sc = n < p.N ? __ldg(p.row_scale + n) : 0.f;
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[j + i] = rescale(static_cast<int>(v[j + i]), inv, __shfl_sync(0xffffffffu, sc, i));
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < COLS; ++j) o[j] = rescale(static_cast<int>(v[j]), inv, s_w);
+                }
                 if (p.bias) {
 #pragma unroll
                     for (int j = 0; j < COLS; j += 32) {
@@ -337,13 +348,13 @@ int wf_wide_tile(int64_t M, int64_t N, int64_t K) {
 }
 
 // q [M, K] int8 (row stride ldq), w8 [N, K] int8 contiguous; bn from wf_wide_tile.
-int wf_wide_launch(const int8_t* q, int64_t ldq, const float* x_scale, const int8_t* w8, const float* w_scale, float w_scale_host, const void* bias,
+int wf_wide_launch(const int8_t* q, int64_t ldq, const float* x_scale, const int8_t* w8, const float* w_scale, float w_scale_host, const float* row_scale, const void* bias,
                    int bias_dtype, void* y, int y_dtype, int64_t ldy, int64_t M, int64_t N, int64_t K, int bn, void* stream) {
     EncodeTiledFn enc = pf_encode_fn();
     if (!enc) return fail(WF_E_DEVICE, "cuTensorMapEncodeTiled is not available in this driver");
     const int pairs = num_sms() / 2;
     WideParams p;
-    p.x_scale = x_scale; p.w_scale = w_scale; p.w_scale_host = w_scale_host; p.bias = bias; p.bias_dtype = bias_dtype;
+    p.x_scale = x_scale; p.w_scale = w_scale; p.row_scale = row_scale; p.w_scale_host = w_scale_host; p.bias = bias; p.bias_dtype = bias_dtype;
     p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K);
     p.bn = bn;
     p.tiles_m = static_cast<int>((M + WD_BM - 1) / WD_BM);

@@ -6,7 +6,7 @@ act(gate) * up -> down BitLinear -> residual; bf16 embedding and lm_head.  Unlik
 KV cache, launches q/k/v and gate/up as one grouped kernel each, and replays the whole decode step as a CUDA
 graph.  With `subln=True` and weights loaded under the reference's parameter names it computes the reference
 model (BitNetLlama) itself.  In the decode step the norms, RoPE + cache write, attention over the cache and the gate
-activation are kernels of this library as well; so they are in the prompt pass of a bf16 model, where only the attention is the
+activation are kernels of this library as well; so they are in the prompt pass of a bf16 model, where only the attention of long prompts is the
 framework's (an fp32 model, which the parity tests use, runs the prompt on torch operators around the projections).
 
 Tensor parallel: heads and the MLP width are split over the ranks of a process group; q/k/v/gate/up are
@@ -42,6 +42,12 @@ class DecoderConfig:
     subln: bool = False  # sub-layer norms in front of o_proj and down_proj (wrinklefree/models/attention.py:213, ffn.py:84)
     subln_eps: float = 1e-6
 
+
+# Largest B x heads x S x S x head width of a prompt whose attention runs on this library's kernel (ops.attn_prompt).  The framework's fused
+# attention is faster on the GPU beyond a few tiles, and takes 30 us more of the host: whole prompt pass in us per layer with this
+# kernel / with the framework's, 9 heads of 64: 121 tokens 115 / 147, 1024 tokens 117 / 149, 2048 tokens 146 / 150; 32 heads of 64: 512
+# tokens 118 / 150, 1024 tokens 165 / 151; 32 heads of 128: 121 tokens 127 / 149, 300 tokens 174 / 174, 512 tokens 211 / 203.
+PROMPT_KERNEL_MAX = 1 << 29
 
 SMOLLM2_135M = DecoderConfig(layers=30, hidden=576, n_q=9, n_kv=3, head_dim=64, intermediate=1536, vocab=49152, rope_theta=1e5)
 LLAMA3_8B = DecoderConfig(layers=32, hidden=4096, n_q=32, n_kv=8, head_dim=128, intermediate=14336, vocab=128256, rope_theta=5e5)
@@ -153,6 +159,12 @@ class TernaryDecoder:
             L["gate"] = (tpmod.shard_codes_rows(cg, self.i_lo, self.i_hi), sg)
             L["up"] = (tpmod.shard_codes_rows(cu, self.i_lo, self.i_hi), su)
             L["down"] = (tpmod.shard_codes_k(cd, self.i_lo, self.i_hi), sd)
+            if dtype == torch.bfloat16:  # the prompt pass runs q/k/v, and gate and up, as one contraction: their rows lie side by side
+                for fused, names in (("qkv", ("q", "k", "v")), ("gu", ("gate", "up"))):
+                    both = torch.cat([L[n][0] for n in names])
+                    L[fused + "_rows"] = (both, torch.cat([L[n][1][:1].expand(L[n][0].shape[0]) for n in names]))
+                    for n, part in zip(names, both.split([L[n][0].shape[0] for n in names])):
+                        L[n] = (part, L[n][1])
             L["n1"] = vec(pre + "input_layernorm.weight", h)
             L["n2"] = vec(pre + "post_attention_layernorm.weight", h)
             if cfg.subln:
@@ -479,35 +491,49 @@ class TernaryDecoder:
 
     def _prefill_kernels(self, ids, all_logits):
         """The prompt pass on this library's kernels (bf16): residual add + RMSNorm with the quantization that q/k/v resp. gate/up
-        share, RoPE with the cache write, gate activation with the quantization of down.  Only the attention itself is the
-        framework's.  A layer is twelve calls: 13 launches for a prompt of 40 tokens, 19 for one of 121 (a projection of more than 64
-        tokens is two launches); with torch operators around the projections, as the fp32 model runs it, 54."""
+        share, those as one contraction each, RoPE with the cache write, attention (the framework's beyond PROMPT_KERNEL_MAX), gate
+        activation with the quantization of down.  A layer is nine calls and thirteen launches; with torch operators around the
+        projections, as the fp32 model runs it, 54."""
         cfg, B, d, S = self.cfg, self.B, self.cfg.head_dim, ids.shape[1]
-        M, dev = B * S, self.dev
+        M, dev, dt = B * S, self.dev, self.dtype
+        i_loc = self.i_hi - self.i_lo
+        nqd, nkd = self.nq * d, self.nkv * d
+        own = d in (64, 128) and M * self.nq * S * d <= PROMPT_KERNEL_MAX and self.nq % self.nkv == 0
 
-        def quantized(k):
-            return torch.empty(M, k, dtype=torch.int8, device=dev), torch.empty(M, dtype=torch.float32, device=dev)
+        def empty(*shape, dtype=dt):
+            return torch.empty(*shape, dtype=dtype, device=dev)
+
+        # one set of buffers for all layers: they run one after another on this stream
+        xq, aq, s1 = empty(M, max(cfg.hidden, nqd), dtype=torch.int8), empty(M, i_loc, dtype=torch.int8), empty(M, dtype=torch.float32)
+        xq, oq = xq.view(-1)[:M * cfg.hidden].view(M, cfg.hidden), xq.view(-1)[:M * nqd].view(M, nqd)
+        qkv, gu, att, res = empty(M, nqd + 2 * nkd), empty(M, 2 * i_loc), empty(M, nqd), empty(M, cfg.hidden)
+        q, k, v = qkv.split([nqd, nkd, nkd], 1)
+        g, u = gu.split([i_loc, i_loc], 1)
+        ws = ops.rows_workspace(M, [(qkv.shape[1], cfg.hidden), (gu.shape[1], cfg.hidden)], dev)
 
         h, delta = self.embed[ids].reshape(M, cfg.hidden), None
         for L in self.layers:
-            xq, xs = ops.add_rmsnorm_quant_(h, delta, L["n1"], *quantized(cfg.hidden), cfg.eps)
-            q, k, v = (ops.bitlinear(xq, *L[n], x_scale=xs, out_dtype=self.dtype) for n in ("q", "k", "v"))
+            ops.add_rmsnorm_quant_(h, delta, L["n1"], xq, s1, cfg.eps)
+            ops.bitlinear_rows(xq, s1, *L["qkv_rows"], qkv, ws)
             ops.rope_kv_prompt_(q, k, v, self.cos, self.sin, L["kc"], L["vc"], S)
-            a = _causal_attention(q.view(B, S, self.nq, d).transpose(1, 2), L["kc"][:, :, :S], L["vc"][:, :, :S])
-            a = a.transpose(1, 2).reshape(M, self.nq * d)
-            if cfg.subln:
-                aq, as_ = ops.add_rmsnorm_quant_(a, None, L["sa"], *quantized(self.nq * d), cfg.subln_eps)
-                o = ops.bitlinear(aq, *L["o"], x_scale=as_, out_dtype=self.dtype)
+            if own:
+                a = ops.attn_prompt(q, L["kc"], L["vc"], att, S)
             else:
-                o = ops.bitlinear(a, *L["o"])
-            hq, hs = ops.add_rmsnorm_quant_(h, self._allreduce(o), L["n2"], *quantized(cfg.hidden), cfg.eps)
-            g, u = (ops.bitlinear(hq, *L[n], x_scale=hs, out_dtype=self.dtype) for n in ("gate", "up"))
+                a = _causal_attention(q.view(B, S, self.nq, d).transpose(1, 2), L["kc"][:, :, :S], L["vc"][:, :, :S])
+                a = a.transpose(1, 2).reshape(M, nqd)
             if cfg.subln:
-                act = ops.act_mul(g, u, torch.empty_like(g), cfg.act)
-                actq, acts = ops.add_rmsnorm_quant_(act, None, L["sf"], *quantized(act.shape[1]), cfg.subln_eps)
+                ops.add_rmsnorm_quant_(a, None, L["sa"], oq, s1, cfg.subln_eps)
+                o = ops.bitlinear(oq, *L["o"], x_scale=s1, out=res)
             else:
-                actq, acts = ops.act_mul_quant(g, u, *quantized(g.shape[1]), mode=cfg.act)
-            delta = self._allreduce(ops.bitlinear(actq, *L["down"], x_scale=acts, out_dtype=self.dtype))
+                o = ops.bitlinear(a, *L["o"], out=res)
+            ops.add_rmsnorm_quant_(h, self._allreduce(o), L["n2"], xq, s1, cfg.eps)
+            ops.bitlinear_rows(xq, s1, *L["gu_rows"], gu, ws)
+            if cfg.subln:
+                act = ops.act_mul(g.contiguous(), u.contiguous(), empty(M, i_loc), cfg.act)
+                ops.add_rmsnorm_quant_(act, None, L["sf"], aq, s1, cfg.subln_eps)
+            else:
+                ops.act_mul_quant(g, u, aq, s1, mode=cfg.act)
+            delta = self._allreduce(ops.bitlinear(aq, *L["down"], x_scale=s1, out=res))
         if not all_logits:
             h, delta = (t.view(B, S, cfg.hidden)[:, -1].contiguous() for t in (h, delta))
         xf = ops.add_rmsnorm_(h, delta, self.norm_f, torch.empty_like(h), cfg.eps)

@@ -461,8 +461,45 @@ def rope_kv_prompt_(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torc
     _need_cuda(q, k, v, cos, sin, kcache, vcache)
     b, nkv, t, d = kcache.shape
     with torch.cuda.device(q.device):
-        L.check(L.lib().wf_rope_kv_prompt_bf16(q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), kcache.data_ptr(), vcache.data_ptr(),
-                                               b, s, q.numel() // (b * s * d), nkv, d, t, L.FLAG_PDL if pdl else 0, _stream()), "wf_rope_kv_prompt_bf16")
+        L.check(L.lib().wf_rope_kv_prompt_ld_bf16(q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), cos.data_ptr(), sin.data_ptr(),
+                                                  kcache.data_ptr(), vcache.data_ptr(), b, s, q.numel() // (b * s * d), nkv, d, t, L.FLAG_PDL if pdl else 0,
+                                                  _stream()), "wf_rope_kv_prompt_bf16")
+
+
+def bitlinear_rows(x: torch.Tensor, x_scale: torch.Tensor, codes: torch.Tensor, row_scale: torch.Tensor, out: torch.Tensor, workspace: torch.Tensor):
+    """Several projections of the same int8 tokens [M, K] in one call: codes [N, K/4] and row_scale [N] hold their rows side by side,
+    out [M, N].  `workspace`: from `rows_workspace`, for calls of one stream."""
+    _need_cuda(x, x_scale, codes, row_scale, out)
+    m, k = x.shape
+    n = codes.shape[0]
+    if (x.dtype != torch.int8 or x.stride(1) != 1 or codes.shape[1] * 4 != k or not codes.is_contiguous() or row_scale.shape != (n,) or row_scale.dtype != torch.float32
+            or out.shape != (m, n) or out.stride(1) != 1):
+        raise ValueError("bitlinear_rows needs int8 x [M, K], contiguous codes [N, K/4], float32 row_scale [N] and out [M, N] with unit inner strides")
+    with torch.cuda.device(x.device):
+        L.check(L.lib().wf_bitlinear_prefill_rows(x.data_ptr(), x.stride(0), x_scale.data_ptr(), codes.data_ptr(), row_scale.data_ptr(), out.data_ptr(),
+                                                  _DT[out.dtype], out.stride(0), m, n, k, workspace.data_ptr(), workspace.numel(), _stream()),
+                "wf_bitlinear_prefill_rows")
+    return out
+
+
+def rows_workspace(m: int, shapes, device) -> torch.Tensor:
+    """A workspace for `bitlinear_rows` on m tokens and every (N, K) of `shapes`; on a card without room for expanded weights the
+    smaller one, with which the calls run on packed weights."""
+    try:
+        return torch.empty(max(L.lib().wf_prefill_workspace_bytes_for(m, n, k) for n, k in shapes), dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return torch.empty(max(L.lib().wf_prefill_workspace_bytes(m, k) for _, k in shapes), dtype=torch.uint8, device=device)
+
+
+def attn_prompt(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, out: torch.Tensor, s: int):
+    """Causal attention of a prompt of `s` tokens per sequence: q [B*s, nq*D] (rows may be wider apart), caches [B, nkv, T, D]
+    that hold its keys and values, out [B*s, nq*D]; bf16."""
+    _need_cuda(q, kcache, vcache, out)
+    b, nkv, t, d = kcache.shape
+    with torch.cuda.device(q.device):
+        L.check(L.lib().wf_attn_prompt_bf16(q.data_ptr(), q.stride(0), kcache.data_ptr(), vcache.data_ptr(), out.data_ptr(), b, s, out.shape[1] // d, nkv, d, t,
+                                            d ** -0.5, 0, _stream()), "wf_attn_prompt_bf16")
+    return out
 
 
 # Workspaces of attn_decode calls that bring none, by (device, stream): launches of one stream may share one, for they run one
@@ -532,7 +569,7 @@ def act_mul_quant(gate: torch.Tensor, up: torch.Tensor, q: torch.Tensor, q_scale
     _need_cuda(gate, up, q, q_scale, out)
     m, i = gate.shape
     with torch.cuda.device(gate.device):
-        L.check(L.lib().wf_act_mul_quant_bf16(gate.data_ptr(), up.data_ptr(), _ptr(out), q.data_ptr(), q_scale.data_ptr(), m, i,
+        L.check(L.lib().wf_act_mul_quant_ld_bf16(gate.data_ptr(), up.data_ptr(), gate.stride(0), _ptr(out), q.data_ptr(), q_scale.data_ptr(), m, i,
                                               0 if mode == "silu" else 1, float(quant_eps), L.FLAG_PDL if pdl else 0, _stream()),
                 "wf_act_mul_quant_bf16")
     return q, q_scale

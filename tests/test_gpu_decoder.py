@@ -647,3 +647,36 @@ def test_projections_side_by_side(wf, m, ns, k, dtype):
     small = torch.empty(wf._lib.lib().wf_prefill_workspace_bytes(m, k), dtype=torch.uint8, device=dev)  # no room for expanded weights
     assert torch.equal(ops.bitlinear_rows(q, s, codes, scales, out[:, :sum(ns)], small), want)
     wf.device_status()
+
+
+@pytest.mark.parametrize("B,S,hidden,n_q,n_kv,d,mlp,act", [(1, 1, 64, 1, 1, 64, 64, "silu"), (1, 7, 576, 9, 3, 64, 1536, "relu2"), (2, 33, 256, 4, 2, 128, 512, "silu"),
+                                                           (1, 121, 576, 9, 3, 64, 1536, "silu"), (3, 20, 2048, 16, 4, 128, 2048, "silu")])
+def test_prompt_layers_in_native_code(wf, monkeypatch, B, S, hidden, n_q, n_kv, d, mlp, act):
+    """The native loop over the layers of a prompt makes the calls of the operators one by one: same bits, on either side of the token
+    counts at which a projection changes its kernel."""
+    from wrinklefree_monorepo_b200 import ops
+    from wrinklefree_monorepo_b200.decoder import DecoderConfig, TernaryDecoder
+
+    def by_operators(layers, h, cos, sin, xbuf, aq, s1, qkv, gu, att, res, ws, b, s, nq, nkv, dim, mode, eps, *limits):
+        m, k = h.shape
+        xq, delta = xbuf[:m * k].view(m, k), None
+        for qkv_c, qkv_s, o_c, o_s, gu_c, gu_s, down_c, down_s, n1, n2, kc, vc in layers:
+            ops.add_rmsnorm_quant_(h, delta, n1, xq, s1, eps)
+            ops.bitlinear_rows(xq, s1, qkv_c, qkv_s, qkv, ws)
+            parts = qkv.split([nq * dim, nkv * dim, nkv * dim], 1)
+            ops.rope_kv_prompt_(*parts, cos, sin, kc, vc, s)
+            ops.attn_prompt(parts[0], kc, vc, att, s)
+            ops.add_rmsnorm_quant_(h, ops.bitlinear(att, o_c, o_s), n2, xq, s1, eps)
+            ops.bitlinear_rows(xq, s1, gu_c, gu_s, gu, ws)
+            ops.act_mul_quant(gu[:, :gu.shape[1] // 2], gu[:, gu.shape[1] // 2:], aq, s1, mode="silu" if mode == 0 else "relu2")
+            delta = res.copy_(ops.bitlinear(aq, down_c, down_s, x_scale=s1, out_dtype=h.dtype))
+
+    cfg = DecoderConfig(layers=2, hidden=hidden, n_q=n_q, n_kv=n_kv, head_dim=d, intermediate=mlp, vocab=300, act=act)
+    dev = torch.device("cuda", 0)
+    ids = torch.randint(0, cfg.vocab, (B, S), generator=torch.Generator().manual_seed(S)).to(dev)
+    m = TernaryDecoder(cfg, B, S + 3, dev, seed=4)
+    native = m.prefill(ids, all_logits=True), [L[c].clone() for L in m.layers for c in ("kc", "vc")]
+    monkeypatch.setattr(ops.L.host(), "prompt_layers", by_operators)
+    assert torch.equal(m.prefill(ids, all_logits=True), native[0])
+    assert all(torch.equal(a, b) for a, b in zip([L[c] for L in m.layers for c in ("kc", "vc")], native[1]))
+    wf.device_status()

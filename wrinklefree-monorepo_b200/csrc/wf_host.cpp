@@ -15,6 +15,8 @@
 #include <torch/csrc/utils/pybind.h>
 #include <torch/version.h>
 
+#include <cmath>
+
 #include "../../include/wf_b200.h"
 
 namespace {
@@ -241,7 +243,115 @@ PyObject* bitlinear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     END_HANDLE_TH_ERRORS
 }
 
+// prompt_layers(layers, h, cos, sin, xq, aq, scale, qkv, gu, att, res, ws, B, S, n_q, n_kv, D, mode, eps, decode_max_tokens,
+//               prequant_min_tokens, prequant_min_elems)
+// The layers of a decoder's prompt pass (bf16, no sub-layer norms, one GPU) on the caller's buffers; `layers`: per layer a tuple of
+// (qkv codes, qkv row scales, o codes, o scale, gate/up codes, gate/up row scales, down codes, down scale, norm 1, norm 2, keys, values).
+// The same calls as the loop in the decoder makes, thirteen launches per layer; from Python their nine wrappers took about 100 us of
+// host time per layer, which is what bounded a short prompt.  `res` holds the last layer's output of down, not yet added to h.
+PyObject* prompt_layers(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    try {
+        if (n_args != 22) raise(PyExc_TypeError, "prompt_layers takes 22 arguments");
+        struct Layer {
+            const uint8_t *qkv, *o, *gu, *down;
+            const float *qkv_s, *o_s, *gu_s, *down_s;
+            const void *n1, *n2;
+            void *kc, *vc;
+        };
+        const at::Tensor &h = tensor(a[1]), &cos = tensor(a[2]), &sin = tensor(a[3]), &xq = tensor(a[4]), &aq = tensor(a[5]), &scale = tensor(a[6]), &qkv = tensor(a[7]),
+                         &gu = tensor(a[8]), &att = tensor(a[9]), &res = tensor(a[10]), &ws = tensor(a[11]);
+        need_cuda({&h, &cos, &sin, &xq, &aq, &scale, &qkv, &gu, &att, &res, &ws});
+        const int64_t B = long_arg(a[12]), S = long_arg(a[13]);
+        const int nq = static_cast<int>(long_arg(a[14])), nkv = static_cast<int>(long_arg(a[15])), D = static_cast<int>(long_arg(a[16]));
+        const int mode = static_cast<int>(long_arg(a[17]));
+        const float eps = static_cast<float>(float_arg(a[18]));
+        const long decode_max = long_arg(a[19]), pre_tokens = long_arg(a[20]), pre_elems = long_arg(a[21]);
+        const int64_t M = h.size(0), hidden = h.size(1), qd = static_cast<int64_t>(nq) * D, kvd = static_cast<int64_t>(nkv) * D, inter = aq.size(1);
+        const auto rows_of = [&](const at::Tensor& t, int64_t width) { return t.dim() == 2 && t.size(0) == M && t.size(1) == width && t.is_contiguous(); };
+        if (h.dim() != 2 || M != B * S || xq.numel() < M * std::max(hidden, qd) || scale.numel() != M || !rows_of(aq, inter) || !rows_of(qkv, qd + 2 * kvd) ||
+            !rows_of(gu, 2 * inter) || !rows_of(att, qd) || !rows_of(res, hidden) || !h.is_contiguous())
+            raise(PyExc_ValueError, "prompt_layers: a buffer does not have its shape");
+        if (!PyList_Check(a[0])) raise(PyExc_TypeError, "prompt_layers: layers must be a list");
+        std::vector<Layer> layers(static_cast<size_t>(PyList_GET_SIZE(a[0])));
+        int64_t T = 0;
+        for (size_t i = 0; i < layers.size(); ++i) {
+            PyObject* t = PyList_GET_ITEM(a[0], static_cast<Py_ssize_t>(i));
+            if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 12) raise(PyExc_TypeError, "prompt_layers: a layer is a tuple of twelve tensors");
+            const at::Tensor* e[12];
+            for (int j = 0; j < 12; ++j) {
+                e[j] = &tensor(PyTuple_GET_ITEM(t, j));
+                if (!e[j]->is_cuda() || !e[j]->is_contiguous()) raise(PyExc_ValueError, "prompt_layers: layer tensors must be contiguous CUDA tensors");
+            }
+            T = e[10]->size(2);
+            if (e[0]->numel() * 4 != (qd + 2 * kvd) * hidden || e[1]->numel() != qd + 2 * kvd || e[2]->numel() * 4 != hidden * qd || e[4]->numel() * 4 != 2 * inter * hidden ||
+                e[5]->numel() != 2 * inter || e[6]->numel() * 4 != hidden * inter || e[8]->numel() != hidden || e[9]->numel() != hidden || e[10]->numel() != B * T * kvd ||
+                e[11]->numel() != B * T * kvd)
+                raise(PyExc_ValueError, "prompt_layers: a layer's tensor does not have its shape");
+            layers[i] = {static_cast<const uint8_t*>(e[0]->data_ptr()), static_cast<const uint8_t*>(e[2]->data_ptr()), static_cast<const uint8_t*>(e[4]->data_ptr()),
+                         static_cast<const uint8_t*>(e[6]->data_ptr()), e[1]->data_ptr<float>(), e[3]->data_ptr<float>(), e[5]->data_ptr<float>(), e[7]->data_ptr<float>(),
+                         e[8]->data_ptr(), e[9]->data_ptr(), e[10]->data_ptr(), e[11]->data_ptr()};
+        }
+        c10::cuda::CUDAGuard guard(h.device());
+        void* const stream = c10::cuda::getCurrentCUDAStream().stream();
+        int8_t* const q8 = xq.data_ptr<int8_t>();
+        int8_t* const a8 = aq.data_ptr<int8_t>();
+        float* const xs = scale.data_ptr<float>();
+        const auto bytes = h.options().dtype(at::kByte);
+        const char* what = "";
+        int rc = 0;
+        // one projection of the tokens, by the rule of bitlinear(); from bf16 (x_scale null) or int8
+        const auto project = [&](const void* x, int type, const float* x_scale, const uint8_t* codes, const float* w_scale, int64_t k) {
+            if (M > decode_max || (M >= 16 && hidden * k >= (1 << 22))) {
+                const at::Tensor own = contraction_workspace(M, hidden, k, bytes);
+                what = "wf_bitlinear_prefill";
+                return wf_bitlinear_prefill(x, type, k, x_scale, codes, WF_LAYOUT_WF16, w_scale, 0.f, nullptr, 0, res.data_ptr(), WF_BF16, hidden, nullptr, M, hidden, k, 1e-5f,
+                                            own.data_ptr(), static_cast<size_t>(own.numel()), 0, stream);
+            }
+            if (type != WF_I8 && (M >= pre_tokens || M * k >= pre_elems) && !wf_decode_fuses_quant(M, k, hidden * k, 1)) {
+                what = "wf_act_quant_i8";
+                if (const int e = wf_act_quant_i8(x, type, M, k, k, WF_ACT_PER_TOKEN, 1e-5f, q8, xs, nullptr, stream)) return e;
+                x = q8;
+                type = WF_I8;
+                x_scale = xs;
+            }
+            what = "wf_bitlinear_decode";
+            return wf_bitlinear_decode(x, type, k, x_scale, codes, WF_LAYOUT_WF16, w_scale, 0.f, nullptr, 0, res.data_ptr(), WF_BF16, hidden, nullptr, M, hidden, k, 1e-5f, 0, stream);
+        };
+        {
+            pybind11::gil_scoped_release nogil;
+            const auto step = [&](int e, const char* name) {
+                what = name;
+                return e;
+            };
+            char* const qkv_p = static_cast<char*>(qkv.data_ptr());
+            char* const gu_p = static_cast<char*>(gu.data_ptr());
+            const size_t ws_bytes = static_cast<size_t>(ws.numel());
+            bool first = true;
+            for (const Layer& L : layers) {
+                if ((rc = step(wf_add_rmsnorm_quant_bf16(h.data_ptr(), first ? nullptr : res.data_ptr(), L.n1, nullptr, q8, xs, M, hidden, eps, 1e-5f, 0, stream), "wf_add_rmsnorm_quant_bf16"))) break;
+                first = false;
+                if ((rc = step(wf_bitlinear_prefill_rows(q8, hidden, xs, L.qkv, L.qkv_s, qkv_p, WF_BF16, qd + 2 * kvd, M, qd + 2 * kvd, hidden, ws.data_ptr(), ws_bytes, stream), "wf_bitlinear_prefill_rows"))) break;
+                if ((rc = step(wf_rope_kv_prompt_ld_bf16(qkv_p, qd + 2 * kvd, qkv_p + 2 * qd, qkv_p + 2 * (qd + kvd), qd + 2 * kvd, cos.data_ptr<float>(), sin.data_ptr<float>(), L.kc, L.vc, B, S, nq,
+                                                         nkv, D, T, 0, stream), "wf_rope_kv_prompt_bf16"))) break;
+                if ((rc = step(wf_attn_prompt_bf16(qkv_p, qd + 2 * kvd, L.kc, L.vc, att.data_ptr(), B, S, nq, nkv, D, T, static_cast<float>(std::pow(static_cast<double>(D), -0.5)), 0, stream), "wf_attn_prompt_bf16"))) break;
+                if ((rc = project(att.data_ptr(), WF_BF16, nullptr, L.o, L.o_s, qd))) break;
+                if ((rc = step(wf_add_rmsnorm_quant_bf16(h.data_ptr(), res.data_ptr(), L.n2, nullptr, q8, xs, M, hidden, eps, 1e-5f, 0, stream), "wf_add_rmsnorm_quant_bf16"))) break;
+                if ((rc = step(wf_bitlinear_prefill_rows(q8, hidden, xs, L.gu, L.gu_s, gu_p, WF_BF16, 2 * inter, M, 2 * inter, hidden, ws.data_ptr(), ws_bytes, stream), "wf_bitlinear_prefill_rows"))) break;
+                if ((rc = step(wf_act_mul_quant_ld_bf16(gu_p, gu_p + 2 * inter, 2 * inter, nullptr, a8, xs, M, inter, mode, 1e-5f, 0, stream), "wf_act_mul_quant_bf16"))) break;
+                if ((rc = project(a8, WF_I8, xs, L.down, L.down_s, inter))) break;
+            }
+        }
+        check(rc, what);
+        Py_RETURN_NONE;
+    } catch (const PyFailure&) {
+        return nullptr;
+    }
+    END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"prompt_layers", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(prompt_layers)), METH_FASTCALL, nullptr},
     {"act_quant_i8", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(act_quant_i8)), METH_FASTCALL, nullptr},
     {"bitlinear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(bitlinear)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},

@@ -492,7 +492,7 @@ class TernaryDecoder:
     def _prefill_kernels(self, ids, all_logits):
         """The prompt pass on this library's kernels (bf16): residual add + RMSNorm with the quantization that q/k/v resp. gate/up
         share, those as one contraction each, RoPE with the cache write, attention (the framework's beyond PROMPT_KERNEL_MAX), gate
-        activation with the quantization of down.  A layer is nine calls and thirteen launches; with torch operators around the
+        activation with the quantization of down.  A layer is nine calls and thirteen launches, made from native code where nothing else is asked for; with torch operators around the
         projections, as the fp32 model runs it, 54."""
         cfg, B, d, S = self.cfg, self.B, self.cfg.head_dim, ids.shape[1]
         M, dev, dt = B * S, self.dev, self.dtype
@@ -504,15 +504,21 @@ class TernaryDecoder:
             return torch.empty(*shape, dtype=dtype, device=dev)
 
         # one set of buffers for all layers: they run one after another on this stream
-        xq, aq, s1 = empty(M, max(cfg.hidden, nqd), dtype=torch.int8), empty(M, i_loc, dtype=torch.int8), empty(M, dtype=torch.float32)
-        xq, oq = xq.view(-1)[:M * cfg.hidden].view(M, cfg.hidden), xq.view(-1)[:M * nqd].view(M, nqd)
+        xbuf, aq, s1 = empty(M * max(cfg.hidden, nqd), dtype=torch.int8), empty(M, i_loc, dtype=torch.int8), empty(M, dtype=torch.float32)
+        xq, oq = xbuf[:M * cfg.hidden].view(M, cfg.hidden), xbuf[:M * nqd].view(M, nqd)
         qkv, gu, att, res = empty(M, nqd + 2 * nkd), empty(M, 2 * i_loc), empty(M, nqd), empty(M, cfg.hidden)
         q, k, v = qkv.split([nqd, nkd, nkd], 1)
         g, u = gu.split([i_loc, i_loc], 1)
         ws = ops.rows_workspace(M, [(qkv.shape[1], cfg.hidden), (gu.shape[1], cfg.hidden)], dev)
 
         h, delta = self.embed[ids].reshape(M, cfg.hidden), None
-        for L in self.layers:
+        native = own and not cfg.subln and self.tp == 1 and self.layers  # the loop below, in native code
+        if native:
+            ops.L.host().prompt_layers([(*L["qkv_rows"], *L["o"], *L["gu_rows"], *L["down"], L["n1"], L["n2"], L["kc"], L["vc"]) for L in self.layers], h, self.cos, self.sin,
+                                       xbuf, aq, s1, qkv, gu, att, res, ws, B, S, self.nq, self.nkv, d, 0 if cfg.act == "silu" else 1, cfg.eps, ops.DECODE_MAX_TOKENS,
+                                       ops.PREQUANT_MIN_TOKENS, ops.PREQUANT_MIN_ELEMS)
+            delta = res
+        for L in () if native else self.layers:
             ops.add_rmsnorm_quant_(h, delta, L["n1"], xq, s1, cfg.eps)
             ops.bitlinear_rows(xq, s1, *L["qkv_rows"], qkv, ws)
             ops.rope_kv_prompt_(q, k, v, self.cos, self.sin, L["kc"], L["vc"], S)

@@ -329,16 +329,16 @@ PyObject* prompt_layers(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
             const size_t ws_bytes = static_cast<size_t>(ws.numel());
             bool first = true;
             for (const Layer& L : layers) {
-                if ((rc = step(wf_add_rmsnorm_quant_bf16(h.data_ptr(), first ? nullptr : res.data_ptr(), L.n1, nullptr, q8, xs, M, hidden, eps, 1e-5f, 0, stream), "wf_add_rmsnorm_quant_bf16"))) break;
+                if ((rc = step(wf_add_rmsnorm_quant_bf16(h.data_ptr(), first ? nullptr : res.data_ptr(), L.n1, nullptr, q8, xs, M, hidden, eps, 1e-5f, first ? 0 : WF_FLAG_PDL, stream), "wf_add_rmsnorm_quant_bf16"))) break;
                 first = false;
                 if ((rc = step(wf_bitlinear_prefill_rows(q8, hidden, xs, L.qkv, L.qkv_s, qkv_p, WF_BF16, qd + 2 * kvd, M, qd + 2 * kvd, hidden, ws.data_ptr(), ws_bytes, stream), "wf_bitlinear_prefill_rows"))) break;
                 if ((rc = step(wf_rope_kv_prompt_ld_bf16(qkv_p, qd + 2 * kvd, qkv_p + 2 * qd, qkv_p + 2 * (qd + kvd), qd + 2 * kvd, cos.data_ptr<float>(), sin.data_ptr<float>(), L.kc, L.vc, B, S, nq,
-                                                         nkv, D, T, 0, stream), "wf_rope_kv_prompt_bf16"))) break;
-                if ((rc = step(wf_attn_prompt_bf16(qkv_p, qd + 2 * kvd, L.kc, L.vc, att.data_ptr(), B, S, nq, nkv, D, T, static_cast<float>(std::pow(static_cast<double>(D), -0.5)), 0, stream), "wf_attn_prompt_bf16"))) break;
+                                                         nkv, D, T, WF_FLAG_PDL, stream), "wf_rope_kv_prompt_bf16"))) break;
+                if ((rc = step(wf_attn_prompt_bf16(qkv_p, qd + 2 * kvd, L.kc, L.vc, att.data_ptr(), B, S, nq, nkv, D, T, static_cast<float>(std::pow(static_cast<double>(D), -0.5)), WF_FLAG_PDL, stream), "wf_attn_prompt_bf16"))) break;
                 if ((rc = project(att.data_ptr(), WF_BF16, nullptr, L.o, L.o_s, qd))) break;
-                if ((rc = step(wf_add_rmsnorm_quant_bf16(h.data_ptr(), res.data_ptr(), L.n2, nullptr, q8, xs, M, hidden, eps, 1e-5f, 0, stream), "wf_add_rmsnorm_quant_bf16"))) break;
+                if ((rc = step(wf_add_rmsnorm_quant_bf16(h.data_ptr(), res.data_ptr(), L.n2, nullptr, q8, xs, M, hidden, eps, 1e-5f, WF_FLAG_PDL, stream), "wf_add_rmsnorm_quant_bf16"))) break;
                 if ((rc = step(wf_bitlinear_prefill_rows(q8, hidden, xs, L.gu, L.gu_s, gu_p, WF_BF16, 2 * inter, M, 2 * inter, hidden, ws.data_ptr(), ws_bytes, stream), "wf_bitlinear_prefill_rows"))) break;
-                if ((rc = step(wf_act_mul_quant_ld_bf16(gu_p, gu_p + 2 * inter, 2 * inter, nullptr, a8, xs, M, inter, mode, 1e-5f, 0, stream), "wf_act_mul_quant_bf16"))) break;
+                if ((rc = step(wf_act_mul_quant_ld_bf16(gu_p, gu_p + 2 * inter, 2 * inter, nullptr, a8, xs, M, inter, mode, 1e-5f, WF_FLAG_PDL, stream), "wf_act_mul_quant_bf16"))) break;
                 if ((rc = project(a8, WF_I8, xs, L.down, L.down_s, inter))) break;
             }
         }

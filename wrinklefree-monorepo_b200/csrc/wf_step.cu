@@ -9,7 +9,7 @@
 //   * what follows an exchange (residual add, norm, quantization) is repeated by every CTA on the whole row: it is short
 //     where this form pays, and cheaper than one more exchange;
 //   * packed weights, norm weights and scales do not depend on the step: one producer warp streams them with bulk copies through a
-//     ring of shared-memory stages, as far ahead as the ring reaches (two layers of width 576), so that no phase waits for them;
+//     ring of shared-memory stages, as far ahead as the ring reaches (a layer of width 576), so that no phase waits for them;
 //   * attention: a KV head's positions are split over up to cluster / n_kv CTAs (one until the context is long enough to share);
 //     eight or sixteen lanes hold a position, keys and values go from global memory to registers, and the first tile is
 //     requested before the CTA waits for q, because older positions do not depend on it.  Partial results are exchanged in fp32.

@@ -92,7 +92,8 @@ class TernaryDecoder:
         or the activation, so it pays only for short rows and few of them; measured on B200 per layer: one sequence 27.5 -> 25.1 us
         (576 wide), 45.2 -> 43.3 (2560), 58.8 -> 69.7 (4096); two 29.3 -> 26.9 (576), 47 -> 54 (2560).  By default it is on where it
         pays (`_fusing_pays`: up to 2560 wide for one sequence, up to 1024 for two, MLPs that its launches take) and no `prefetch` is
-        asked for (the fused step has none).
+        asked for (the fused step has none).  Without `fuse` and `prefetch`, small models run all layers of a step in one launch instead
+        (`resident`, see _resident_layers).
         `fuse_exchange` (tensor parallel, up to 8 sequences, bf16): the row-parallel projections push their partial outputs to every rank inside their own launch and the residual add + RMSNorm that follows sums them (default: from two
         sequences on; True / False force it)."""
         self._fuse_opt = fuse

@@ -305,7 +305,8 @@ class TernaryDecoder:
         if (self.tp > 1 or self._fuse_opt is not None or self.prefetch or self.dtype != torch.bfloat16 or cfg.subln or cfg.layers == 0
                 or cfg.n_q % cfg.n_kv):
             return None
-        cluster = ops.L.lib().wf_decode_layers_cluster(self.B, cfg.hidden, cfg.n_q, cfg.n_kv, cfg.head_dim, cfg.intermediate, self.T)
+        with torch.cuda.device(self.dev):  # what fits is a question to the device that the decoder lives on
+            cluster = ops.L.lib().wf_decode_layers_cluster(self.B, cfg.hidden, cfg.n_q, cfg.n_kv, cfg.head_dim, cfg.intermediate, self.T)
         if not cluster:
             return None
         names = ("q", "k", "v", "o", "gate", "up", "down")

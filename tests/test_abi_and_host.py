@@ -327,3 +327,51 @@ def test_flags_match_the_header_and_the_stack_rule(wf):
         uses = [wf.stack_uses_contraction(m, k) for m in range(1, 65)]
         assert uses == sorted(uses) and uses[-1] and not uses[0]  # once on the contraction, always from there on
     assert wf.stack_uses_contraction(4, 6912) and not wf.stack_uses_contraction(4, 2560) and wf.stack_uses_contraction(8, 2560)
+
+
+@pytest.fixture
+def launches(wf, monkeypatch):
+    """The calls that the operators make into the library, recorded instead of made: (name, arguments)."""
+    import contextlib
+
+    from wrinklefree_monorepo_b200 import ops
+
+    calls = []
+
+    class Recorder:
+        def __getattr__(self, name):
+            return lambda *a: calls.append((name, a)) or 0
+
+    monkeypatch.setattr(ops, "_need_cuda", lambda *ts: None)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops.L, "lib", lambda: Recorder())
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+    return calls
+
+
+def test_rope_of_a_prompt_takes_rows_only(wf, launches):
+    """The row strides that the launch gets: those of contiguous tensors of any shape and of rows inside wider ones; a tensor whose rows
+    lie otherwise is refused, where its first stride was once taken for a row's (and memory far behind the tensor read and written)."""
+    from wrinklefree_monorepo_b200 import ops
+
+    b, s, nq, nkv, d, t = 2, 5, 6, 2, 64, 9
+    cos = torch.zeros(t, d // 2)
+    cache = torch.zeros(b, nkv, t, d, dtype=torch.bfloat16)
+    z = lambda *shape: torch.zeros(*shape, dtype=torch.bfloat16)  # noqa: E731
+    q, k, v = z(b * s, (nq + 2 * nkv) * d).split([nq * d, nkv * d, nkv * d], 1)
+    call = lambda q, k, v: ops.rope_kv_prompt_(q, k, v, cos, cos, cache, cache, s)  # noqa: E731
+    good = [((z(b * s, nq * d), z(b * s, nkv * d), z(b * s, nkv * d)), nq * d, nkv * d), ((q, k, v), (nq + 2 * nkv) * d, (nq + 2 * nkv) * d),
+            ((z(b, s, nq * d), z(b, s, nkv, d), z(b, s, nkv * d)), nq * d, nkv * d), ((z(b, s, nq, d), z(b * s, nkv * d), z(b, s, nkv, d)), nq * d, nkv * d),
+            ((z(b * s * nq * d), k, v), nq * d, (nq + 2 * nkv) * d)]
+    for args, ldq, ldk in good:
+        del launches[:]
+        call(*args)
+        (name, a), = launches
+        assert name == "wf_rope_kv_prompt_ld_bf16" and a[1] == ldq and a[4] == ldk and a[9:15] == (b, s, nq, nkv, d, t), args[0].shape
+    wide = z(b, 2 * s, nq * d)[:, :s]
+    for bad in ((wide, z(b * s, nkv * d), z(b * s, nkv * d)), (q, k, v.contiguous()), (q, k.contiguous(), v), (z(b * s, nq * d), z(nkv * d, b * s).t(), z(b * s, nkv * d)),
+                (z(b * s, nq * d), z(b * s, nkv * d), z(b * s - 1, nkv * d)), (q.expand(b * s, nq * d).float(), k, v), (z(nq * d).expand(b * s, nq * d), k, v)):
+        del launches[:]
+        with pytest.raises(ValueError):
+            call(*bad)
+        assert not launches

@@ -43,6 +43,17 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
+def _row_stride(t: torch.Tensor, rows: int, width: int, name: str) -> int:
+    """Elements from one row of `width` to the next of a bf16 tensor that holds at least `rows` of them: contiguous in any shape, or
+    two-dimensional with unit inner stride."""
+    if t.dtype == torch.bfloat16:
+        if t.is_contiguous() and t.numel() >= rows * width:
+            return width
+        if t.dim() == 2 and t.shape[0] >= rows and t.shape[1] == width and t.stride(1) == 1 and t.stride(0) >= width:
+            return t.stride(0)
+    raise ValueError(f"{name} must be bf16 rows [{rows}, {width}], contiguous or two-dimensional with unit inner stride; got {t.dtype} {tuple(t.shape)} with strides {t.stride()}")
+
+
 def check_kernel_available() -> bool:
     """True when the compiled library is loadable and the current device is sm_100
     (name kept from sgl_kernel/quantization/bitnet.py:39-45)."""
@@ -457,12 +468,17 @@ def rope_kv_(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tenso
 def rope_kv_prompt_(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, kcache: torch.Tensor,
                     vcache: torch.Tensor, s: int, pdl: bool = False):
     """`rope_kv_` for a prompt of `s` tokens per sequence: q [B*s, nq*D] (rotated in place), k, v [B*s, nkv*D]; positions 0 .. s - 1
-    of the caches [B, nkv, T, D] receive the rotated keys and the values."""
+    of the caches [B, nkv, T, D] receive the rotated keys and the values.  q, k and v are contiguous, or rows of wider ones; k and v then
+    lie equally far apart."""
     _need_cuda(q, k, v, cos, sin, kcache, vcache)
     b, nkv, t, d = kcache.shape
+    nq = q.numel() // max(b * s * d, 1)
+    ldq, ldk, ldv = _row_stride(q, b * s, nq * d, "q"), _row_stride(k, b * s, nkv * d, "k"), _row_stride(v, b * s, nkv * d, "v")
+    if ldk != ldv:
+        raise ValueError(f"k and v must have the same row stride, got {ldk} and {ldv}")
     with torch.cuda.device(q.device):
-        L.check(L.lib().wf_rope_kv_prompt_ld_bf16(q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), cos.data_ptr(), sin.data_ptr(),
-                                                  kcache.data_ptr(), vcache.data_ptr(), b, s, q.numel() // (b * s * d), nkv, d, t, L.FLAG_PDL if pdl else 0,
+        L.check(L.lib().wf_rope_kv_prompt_ld_bf16(q.data_ptr(), ldq, k.data_ptr(), v.data_ptr(), ldk, cos.data_ptr(), sin.data_ptr(),
+                                                  kcache.data_ptr(), vcache.data_ptr(), b, s, nq, nkv, d, t, L.FLAG_PDL if pdl else 0,
                                                   _stream()), "wf_rope_kv_prompt_bf16")
 
 

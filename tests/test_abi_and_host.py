@@ -375,3 +375,25 @@ def test_rope_of_a_prompt_takes_rows_only(wf, launches):
         with pytest.raises(ValueError):
             call(*bad)
         assert not launches
+
+
+def test_gate_activation_takes_rows_only(wf, launches):
+    """gate and up share one row stride: contiguous ones in any shape of up, rows of wider tensors when both are; up was once read at
+    gate's stride whatever its own."""
+    from wrinklefree_monorepo_b200 import ops
+
+    m, i = 5, 64
+    z = lambda *shape: torch.zeros(*shape, dtype=torch.bfloat16)  # noqa: E731
+    g, u = z(m, 2 * i).split(i, 1)
+    q, scale = torch.zeros(m, i, dtype=torch.int8), torch.zeros(m)
+    for gate, up, ld, rows in ((z(m, i), z(m, i), i, m), (z(m, i), z(m * i), i, m), (g, u, 2 * i, m), (g[:1], u[:1], i, 1), (g[::2], u[::2], 4 * i, 3)):
+        del launches[:]
+        ops.act_mul_quant(gate, up, q, scale)
+        (name, a), = launches
+        assert name == "wf_act_mul_quant_ld_bf16" and a[2] == ld and a[6:8] == (rows, i)
+    for gate, up in ((g, u.contiguous()), (g.contiguous(), u), (z(i, m).t(), z(i, m).t()), (g, u[::2]), (z(m, i), z(m - 1, i)), (g.float(), u.float()),
+                     (z(1, i).expand(m, i), z(1, i).expand(m, i))):
+        del launches[:]
+        with pytest.raises(ValueError):
+            ops.act_mul_quant(gate, up, q, scale)
+        assert not launches

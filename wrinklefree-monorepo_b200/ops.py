@@ -581,12 +581,16 @@ def add_rmsnorm_quant_(h: torch.Tensor, delta: Optional[torch.Tensor], weight: t
 def act_mul_quant(gate: torch.Tensor, up: torch.Tensor, q: torch.Tensor, q_scale: torch.Tensor, mode: str = "silu",
                   out: Optional[torch.Tensor] = None, quant_eps: float = 1e-5, pdl: bool = False):
     """act(gate) * up per token row [M, I], quantized to int8 per token into `q` / `q_scale` (and written as bf16 into
-    `out` when given): the activation in front of down_proj with that projection's quantization."""
+    `out` when given): the activation in front of down_proj with that projection's quantization.  gate and up are contiguous, or rows
+    of wider tensors that lie equally far apart."""
     _need_cuda(gate, up, q, q_scale, out)
     m, i = gate.shape
+    ld, ld_up = _row_stride(gate, m, i, "gate"), _row_stride(up, m, i, "up")
+    if ld != ld_up:
+        raise ValueError(f"gate and up must have the same row stride, got {ld} and {ld_up}")
     with torch.cuda.device(gate.device):
-        L.check(L.lib().wf_act_mul_quant_ld_bf16(gate.data_ptr(), up.data_ptr(), gate.stride(0), _ptr(out), q.data_ptr(), q_scale.data_ptr(), m, i,
-                                              0 if mode == "silu" else 1, float(quant_eps), L.FLAG_PDL if pdl else 0, _stream()),
+        L.check(L.lib().wf_act_mul_quant_ld_bf16(gate.data_ptr(), up.data_ptr(), ld, _ptr(out), q.data_ptr(), q_scale.data_ptr(), m, i,
+                                                 0 if mode == "silu" else 1, float(quant_eps), L.FLAG_PDL if pdl else 0, _stream()),
                 "wf_act_mul_quant_bf16")
     return q, q_scale
 

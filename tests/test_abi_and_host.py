@@ -397,3 +397,20 @@ def test_gate_activation_takes_rows_only(wf, launches):
         with pytest.raises(ValueError):
             ops.act_mul_quant(gate, up, q, scale)
         assert not launches
+
+
+def test_argmax_increments_an_int64_scalar_only(wf, launches):
+    """`pos` is written as one int64: another type or length, or another device's tensor, is refused."""
+    from wrinklefree_monorepo_b200 import ops
+
+    x, out = torch.zeros(3, 8, dtype=torch.bfloat16), torch.zeros(3, dtype=torch.long)
+    for pos in (None, torch.zeros((), dtype=torch.long), torch.zeros(1, dtype=torch.long)):
+        ops.argmax_(x, out, pos)
+    assert len(launches) == 3
+    for pos in (torch.zeros((), dtype=torch.int32), torch.zeros(()), torch.zeros(0, dtype=torch.long), torch.zeros(2, dtype=torch.long),
+                torch.zeros((), dtype=torch.long, device="meta")):
+        with pytest.raises(ValueError):
+            ops.argmax_(x, out, pos)
+    with pytest.raises(ValueError):
+        ops.argmax_(x, out.to("meta"))
+    assert len(launches) == 3

@@ -410,6 +410,10 @@ def argmax_(x: torch.Tensor, out: torch.Tensor, pos: Optional[torch.Tensor] = No
     b, v = x.shape
     if x.dtype != torch.bfloat16 or out.dtype != torch.long or x.stride(1) != 1 or out.numel() != b or not out.is_contiguous():
         raise ValueError("argmax_ needs bf16 rows with unit inner stride and a contiguous int64 output of one element per row")
+    if pos is not None and (pos.dtype != torch.long or pos.numel() != 1):
+        raise ValueError("argmax_ increments an int64 scalar")
+    if any(t is not None and t.device != x.device for t in (out, pos)):
+        raise ValueError("argmax_ needs its tensors on one device")
     with torch.cuda.device(x.device):
         L.check(L.lib().wf_argmax_bf16(x.data_ptr(), x.stride(0), b, v, out.data_ptr(), _ptr(pos), L.FLAG_PDL if pdl else 0, _stream()), "wf_argmax_bf16")
     return out

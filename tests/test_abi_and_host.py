@@ -414,3 +414,19 @@ def test_argmax_increments_an_int64_scalar_only(wf, launches):
     with pytest.raises(ValueError):
         ops.argmax_(x, out.to("meta"))
     assert len(launches) == 3
+
+
+def test_projections_side_by_side_take_their_scales_and_workspace_only(wf, launches):
+    """What the launch reads by address alone: the scale of each token and row, and the workspace by its bytes."""
+    from wrinklefree_monorepo_b200 import ops
+
+    m, n, k = 3, 10, 64
+    good = dict(x=torch.zeros(m, k, dtype=torch.int8), x_scale=torch.zeros(m), codes=torch.zeros(n, k // 4, dtype=torch.uint8), row_scale=torch.zeros(n),
+                out=torch.zeros(m, n + 2)[:, :n], workspace=torch.zeros(4096, dtype=torch.uint8))
+    ops.bitlinear_rows(**good)
+    assert len(launches) == 1 and launches[0][1][8:11] == (m, n, k)
+    for name, bad in (("x_scale", torch.zeros(m - 1)), ("x_scale", torch.zeros(m).half()), ("x_scale", torch.zeros(2 * m)[::2]), ("row_scale", torch.zeros(2 * n)[::2]),
+                      ("codes", torch.zeros(n, k // 4)), ("workspace", torch.zeros(4096)), ("workspace", good["workspace"].to("meta")), ("x_scale", torch.zeros(m, device="meta"))):
+        with pytest.raises(ValueError):
+            ops.bitlinear_rows(**{**good, name: bad})
+    assert len(launches) == 1

@@ -489,9 +489,13 @@ def rope_kv_prompt_(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torc
 def bitlinear_rows(x: torch.Tensor, x_scale: torch.Tensor, codes: torch.Tensor, row_scale: torch.Tensor, out: torch.Tensor, workspace: torch.Tensor):
     """Several projections of the same int8 tokens [M, K] in one call: codes [N, K/4] and row_scale [N] hold their rows side by side,
     out [M, N].  `workspace`: from `rows_workspace`, for calls of one stream."""
-    _need_cuda(x, x_scale, codes, row_scale, out)
+    _need_cuda(x, x_scale, codes, row_scale, out, workspace)
     m, k = x.shape
     n = codes.shape[0]
+    if x_scale.dtype != torch.float32 or x_scale.numel() != m or not x_scale.is_contiguous() or not row_scale.is_contiguous() or codes.dtype != torch.uint8:
+        raise ValueError("bitlinear_rows needs contiguous float32 scales, x_scale [M] and row_scale [N], and uint8 codes")
+    if workspace.element_size() != 1 or not workspace.is_contiguous() or any(t.device != x.device for t in (x_scale, codes, row_scale, out, workspace)):
+        raise ValueError("bitlinear_rows needs a workspace of bytes, and its tensors on one device")
     if (x.dtype != torch.int8 or x.stride(1) != 1 or codes.shape[1] * 4 != k or not codes.is_contiguous() or row_scale.shape != (n,) or row_scale.dtype != torch.float32
             or out.shape != (m, n) or out.stride(1) != 1):
         raise ValueError("bitlinear_rows needs int8 x [M, K], contiguous codes [N, K/4], float32 row_scale [N] and out [M, N] with unit inner strides")

@@ -430,3 +430,24 @@ def test_projections_side_by_side_take_their_scales_and_workspace_only(wf, launc
         with pytest.raises(ValueError):
             ops.bitlinear_rows(**{**good, name: bad})
     assert len(launches) == 1
+
+
+def test_prompt_attention_takes_rows_only(wf, launches):
+    """q in rows of its own or of a wider tensor, whole caches and output: the launch writes B * s rows of out and reads as many of q."""
+    from wrinklefree_monorepo_b200 import ops
+
+    b, s, nq, nkv, d, t = 2, 5, 6, 2, 64, 9
+    z = lambda *shape: torch.zeros(*shape, dtype=torch.bfloat16)  # noqa: E731
+    good = dict(q=z(b * s, nq * d), kcache=z(b, nkv, t, d), vcache=z(b, nkv, t, d), out=z(b * s, nq * d), s=s)
+    for q, ld in ((good["q"], nq * d), (z(b * s, nq * d + 16)[:, :nq * d], nq * d + 16), (z(b, s, nq * d), nq * d)):
+        del launches[:]
+        ops.attn_prompt(**{**good, "q": q})
+        (name, a), = launches
+        assert name == "wf_attn_prompt_bf16" and a[1] == ld and a[5:11] == (b, s, nq, nkv, d, t)
+    del launches[:]
+    for name, bad in (("q", z(b, 2 * s, nq * d)[:, :s]), ("q", z(b * s - 1, nq * d)), ("q", good["q"].float()), ("out", z(b * s - 1, nq * d)), ("out", z(b * s, nq * d + 8)[:, :nq * d]),
+                      ("out", z(b * s, (nq + 1) * d)), ("out", good["out"].float()), ("kcache", z(b, nkv, 2 * t, d)[:, :, :t]), ("vcache", z(b, nkv, t - 1, d)),
+                      ("vcache", good["vcache"].to("meta"))):
+        with pytest.raises(ValueError):
+            ops.attn_prompt(**{**good, name: bad})
+    assert not launches

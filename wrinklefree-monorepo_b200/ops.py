@@ -520,8 +520,13 @@ def attn_prompt(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, out
     that hold its keys and values, out [B*s, nq*D]; bf16."""
     _need_cuda(q, kcache, vcache, out)
     b, nkv, t, d = kcache.shape
+    if any(c.dtype != torch.bfloat16 or not c.is_contiguous() for c in (kcache, vcache, out)) or vcache.shape != kcache.shape:
+        raise ValueError("attn_prompt needs contiguous bf16 caches of one shape and a contiguous bf16 output")
+    if out.dim() != 2 or out.shape[0] != b * s or out.shape[1] % (nkv * d) or any(c.device != q.device for c in (kcache, vcache, out)):
+        raise ValueError("attn_prompt needs out [B*s, nq*D] with whole groups of heads, and its tensors on one device")
+    ldq = _row_stride(q, b * s, out.shape[1], "q")
     with torch.cuda.device(q.device):
-        L.check(L.lib().wf_attn_prompt_bf16(q.data_ptr(), q.stride(0), kcache.data_ptr(), vcache.data_ptr(), out.data_ptr(), b, s, out.shape[1] // d, nkv, d, t,
+        L.check(L.lib().wf_attn_prompt_bf16(q.data_ptr(), ldq, kcache.data_ptr(), vcache.data_ptr(), out.data_ptr(), b, s, out.shape[1] // d, nkv, d, t,
                                             d ** -0.5, 0, _stream()), "wf_attn_prompt_bf16")
     return out
 

@@ -451,3 +451,36 @@ def test_prompt_attention_takes_rows_only(wf, launches):
         with pytest.raises(ValueError):
             ops.attn_prompt(**{**good, name: bad})
     assert not launches
+
+
+def test_layers_in_one_launch_take_their_shapes_only(wf, launches):
+    """The launch has nothing but addresses: what lies behind each is looked at when the descriptors are made, and at each run."""
+    from wrinklefree_monorepo_b200 import ops
+
+    B, hidden, nq, nkv, d, inter, t = 2, 128, 4, 2, 64, 192, 5
+    z = lambda *shape, dtype=torch.bfloat16: torch.zeros(*shape, dtype=dtype)  # noqa: E731
+    shapes = ((nq * d, hidden), (nkv * d, hidden), (nkv * d, hidden), (hidden, nq * d), (inter, hidden), (inter, hidden), (hidden, inter))
+
+    def layer(**other):
+        return {**dict(codes=[z(n, k // 4, dtype=torch.uint8) for n, k in shapes], scales=[torch.zeros(2) for _ in shapes], norms=[z(hidden), z(hidden)],
+                       caches=[z(B, nkv, t, d), z(B, nkv, t, d)]), **other}
+
+    def make(*layers, norm_f=z(hidden), cos=torch.zeros(t, d // 2)):
+        return ops.DecodeLayers(list(layers), hidden, nq, nkv, inter, "silu", 1e-5, norm_f, cos, torch.zeros(t, d // 2), 16)
+
+    good = make(layer(), layer())
+    h, pos = z(B, hidden), torch.zeros((), dtype=torch.long)
+    good.run(h, h, pos)
+    assert len(launches) == 1 and launches[0][1][8:15] == (B, hidden, nq, nkv, d, inter, t)
+    for bad in ((h[:1], h, pos), (h.float(), h, pos), (h, z(B, 2 * hidden)[:, :hidden], pos), (h, h, pos.int()), (h, h, torch.zeros(2, dtype=torch.long)), (h, h, pos.to("meta"))):
+        with pytest.raises(ValueError):
+            good.run(*bad)
+    assert len(launches) == 1
+    codes = layer()["codes"]
+    for bad in (dict(caches=[z(B, nkv, t + 1, d), z(B, nkv, t + 1, d)]), dict(caches=[z(B, nkv, t, d), z(B, nkv, t, d).float()]), dict(norms=[z(hidden), z(inter)]),
+                dict(codes=codes[:6] + codes[:1]), dict(codes=[c.to(torch.int16) for c in codes]), dict(scales=[torch.zeros(2, dtype=torch.float64)] * 7), dict(scales=[torch.zeros(1)] * 6)):
+        with pytest.raises(ValueError):
+            make(layer(), layer(**bad))
+    for bad in (dict(norm_f=z(inter)), dict(norm_f=torch.zeros(hidden)), dict(cos=torch.zeros(t - 1, d // 2)), dict(cos=torch.zeros(t, d // 2, dtype=torch.float64))):
+        with pytest.raises(ValueError):
+            make(layer(), **bad)

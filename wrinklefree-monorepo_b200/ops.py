@@ -431,12 +431,29 @@ class DecodeLayers:
         rows = [[_ptr(t) for name in ("codes", "scales", "norms", "caches") for t in lay[name]] for lay in layers]
         if any(p % 16 for r in rows for p in r[:7] + r[14:]) or any(not t.is_contiguous() for lay in layers for name in ("codes", "norms", "caches") for t in lay[name]):
             raise ValueError("DecodeLayers needs contiguous, 16-byte aligned tensors")
+        qd, kvd = n_q * self.D, n_kv * self.D
+        want = {"codes": [(torch.uint8, n * k // 4) for n, k in ((qd, hidden), (kvd, hidden), (kvd, hidden), (hidden, qd), (inter, hidden), (inter, hidden), (hidden, inter))],
+                "norms": [(torch.bfloat16, hidden)] * 2, "caches": [(torch.bfloat16, self.B * kvd * self.T)] * 2}
+        for lay in layers:
+            for name, kinds in want.items():
+                if [(t.dtype, t.numel()) for t in lay[name]] != kinds:
+                    raise ValueError(f"DecodeLayers: {name} must be {kinds}, got {[(t.dtype, t.numel()) for t in lay[name]]}")
+            if len(lay["scales"]) != 7 or any(t.dtype != torch.float32 or t.numel() < 1 for t in lay["scales"]) or any(t.shape != kc.shape for t in lay["caches"]):
+                raise ValueError("DecodeLayers needs seven float32 scales and caches of one shape")
+        if (any(t.device != self.device for lay in layers for name in (*want, "scales") for t in lay[name]) or any(t.device != self.device for t in self._keep[1:])
+                or norm_f.dtype != torch.bfloat16 or norm_f.numel() != hidden or not norm_f.is_contiguous()
+                or any(t.dtype != torch.float32 or t.numel() < self.T * (self.D // 2) or not t.is_contiguous() for t in (cos, sin))):
+            raise ValueError("DecodeLayers needs a bf16 norm weight, float32 rotary tables of T rows, and all tensors on one device")
         self._dev = torch.tensor(rows, dtype=torch.long).to(self.device)
         self.hidden, self.n_q, self.n_kv, self.inter, self.act, self.eps, self.cluster = hidden, n_q, n_kv, inter, 0 if act == "silu" else 1, eps, cluster
 
     def run(self, h: torch.Tensor, xf: torch.Tensor, pos: torch.Tensor, pdl: bool = False):
         """h [B, hidden]: embeddings; xf: the output of the last layer behind the final norm; pos: int64 scalar."""
         _, norm_f, cos, sin = self._keep
+        if any(t.dtype != torch.bfloat16 or t.shape != (self.B, self.hidden) or not t.is_contiguous() for t in (h, xf)):
+            raise ValueError(f"DecodeLayers needs contiguous bf16 h and xf of {(self.B, self.hidden)}")
+        if pos.dtype != torch.long or pos.numel() != 1 or any(t.device != self.device for t in (h, xf, pos)):
+            raise ValueError("DecodeLayers needs an int64 scalar as the position, and its tensors on one device")
         with torch.cuda.device(self.device):
             L.check(L.lib().wf_decode_layers_bf16(self._dev.data_ptr(), self._dev.shape[0], h.data_ptr(), norm_f.data_ptr(), xf.data_ptr(), cos.data_ptr(),
                                                   sin.data_ptr(), pos.data_ptr(), self.B, self.hidden, self.n_q, self.n_kv, self.D, self.inter, self.T, self.act,

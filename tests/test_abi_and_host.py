@@ -484,3 +484,33 @@ def test_layers_in_one_launch_take_their_shapes_only(wf, launches):
     for bad in (dict(norm_f=z(inter)), dict(norm_f=torch.zeros(hidden)), dict(cos=torch.zeros(t - 1, d // 2)), dict(cos=torch.zeros(t, d // 2, dtype=torch.float64))):
         with pytest.raises(ValueError):
             make(layer(), **bad)
+
+
+def test_native_prompt_loop_takes_its_shapes_only(wf):
+    """The loop over the layers has the types and shapes of all it is given looked at before anything else: tensors that pass it on
+    the CPU are refused for not being on the GPU, others for what they are."""
+    B, S, nq, nkv, d, inter, t = 2, 3, 4, 2, 64, 192, 5
+    hidden, qd, kvd, m = 128, nq * d, nkv * d, B * S
+    z = lambda *shape, dtype=torch.bfloat16: torch.zeros(*shape, dtype=dtype)  # noqa: E731
+    codes = lambda n, k: z(n, k // 4, dtype=torch.uint8)  # noqa: E731
+
+    def layer(**other):
+        one = dict(qkv=codes(qd + 2 * kvd, hidden), qkv_s=torch.zeros(qd + 2 * kvd), o=codes(hidden, qd), o_s=torch.zeros(2), gu=codes(2 * inter, hidden), gu_s=torch.zeros(2 * inter),
+                   down=codes(hidden, inter), down_s=torch.zeros(2), n1=z(hidden), n2=z(hidden), kc=z(B, nkv, t, d), vc=z(B, nkv, t, d))
+        return tuple({**one, **other}.values())
+
+    def call(*layers, **other):
+        a = dict(h=z(m, hidden), cos=torch.zeros(t, d // 2), sin=torch.zeros(t, d // 2), xq=z(m * qd, dtype=torch.int8), aq=z(m, inter, dtype=torch.int8), scale=torch.zeros(m),
+                 qkv=z(m, qd + 2 * kvd), gu=z(m, 2 * inter), att=z(m, qd), res=z(m, hidden), ws=z(4096, dtype=torch.uint8))
+        wf._lib.host().prompt_layers(list(layers), *{**a, **other}.values(), B, S, nq, nkv, d, 0, 1e-5, 64, 16, 4096)
+
+    with pytest.raises(RuntimeError, match="CUDA"):
+        call(layer(), layer())
+    for bad in (dict(h=torch.zeros(m, hidden)), dict(res=torch.zeros(m, hidden)), dict(qkv=z(m, qd + 2 * kvd).half()), dict(scale=torch.zeros(m).double()), dict(ws=torch.zeros(4096)),
+                dict(cos=torch.zeros(S - 1, d // 2)), dict(aq=z(m, inter, dtype=torch.uint8)), dict(att=z(m - 1, qd))):
+        with pytest.raises(ValueError):
+            call(layer(), **bad)
+    for bad in (dict(kc=z(B, nkv, t, d).float(), vc=z(B, nkv, t, d).float()), dict(kc=z(B, nkv, t - 1, d), vc=z(B, nkv, t - 1, d)), dict(n1=torch.zeros(hidden)),
+                dict(o=codes(hidden, qd).to(torch.int8)), dict(o_s=torch.zeros(0)), dict(down_s=torch.zeros(2).half()), dict(kc=z(B * nkv, t, d)), dict(gu_s=torch.zeros(2 * inter + 1))):
+        with pytest.raises(ValueError):
+            call(layer(), layer(**bad))

@@ -15,6 +15,7 @@
 #include <torch/csrc/utils/pybind.h>
 #include <torch/version.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "../../include/wf_b200.h"
@@ -261,7 +262,6 @@ PyObject* prompt_layers(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
         };
         const at::Tensor &h = tensor(a[1]), &cos = tensor(a[2]), &sin = tensor(a[3]), &xq = tensor(a[4]), &aq = tensor(a[5]), &scale = tensor(a[6]), &qkv = tensor(a[7]),
                          &gu = tensor(a[8]), &att = tensor(a[9]), &res = tensor(a[10]), &ws = tensor(a[11]);
-        need_cuda({&h, &cos, &sin, &xq, &aq, &scale, &qkv, &gu, &att, &res, &ws});
         const int64_t B = long_arg(a[12]), S = long_arg(a[13]);
         const int nq = static_cast<int>(long_arg(a[14])), nkv = static_cast<int>(long_arg(a[15])), D = static_cast<int>(long_arg(a[16]));
         const int mode = static_cast<int>(long_arg(a[17]));
@@ -272,26 +272,37 @@ PyObject* prompt_layers(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
         if (h.dim() != 2 || M != B * S || xq.numel() < M * std::max(hidden, qd) || scale.numel() != M || !rows_of(aq, inter) || !rows_of(qkv, qd + 2 * kvd) ||
             !rows_of(gu, 2 * inter) || !rows_of(att, qd) || !rows_of(res, hidden) || !h.is_contiguous())
             raise(PyExc_ValueError, "prompt_layers: a buffer does not have its shape");
+        const auto all_of = [](at::ScalarType type, std::initializer_list<const at::Tensor*> ts) {
+            return std::all_of(ts.begin(), ts.end(), [&](const at::Tensor* t) { return t->scalar_type() == type && t->is_contiguous(); });
+        };
+        if (B < 1 || S < 1 || nq < 1 || nkv < 1 || D < 2 || !all_of(at::kBFloat16, {&h, &qkv, &gu, &att, &res}) || !all_of(at::kChar, {&xq, &aq}) ||
+            !all_of(at::kFloat, {&cos, &sin, &scale}) || !all_of(at::kByte, {&ws}) || cos.numel() < S * (D / 2) || sin.numel() < S * (D / 2))
+            raise(PyExc_ValueError, "prompt_layers: a buffer does not have its type, or the rotary tables are shorter than the prompt");
         if (!PyList_Check(a[0])) raise(PyExc_TypeError, "prompt_layers: layers must be a list");
         std::vector<Layer> layers(static_cast<size_t>(PyList_GET_SIZE(a[0])));
         int64_t T = 0;
+        bool together = true;  // on one device
         for (size_t i = 0; i < layers.size(); ++i) {
             PyObject* t = PyList_GET_ITEM(a[0], static_cast<Py_ssize_t>(i));
             if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 12) raise(PyExc_TypeError, "prompt_layers: a layer is a tuple of twelve tensors");
             const at::Tensor* e[12];
-            for (int j = 0; j < 12; ++j) {
-                e[j] = &tensor(PyTuple_GET_ITEM(t, j));
-                if (!e[j]->is_cuda() || !e[j]->is_contiguous()) raise(PyExc_ValueError, "prompt_layers: layer tensors must be contiguous CUDA tensors");
-            }
+            for (int j = 0; j < 12; ++j) e[j] = &tensor(PyTuple_GET_ITEM(t, j));
+            if (!all_of(at::kByte, {e[0], e[2], e[4], e[6]}) || !all_of(at::kFloat, {e[1], e[3], e[5], e[7]}) || !all_of(at::kBFloat16, {e[8], e[9], e[10], e[11]}))
+                raise(PyExc_ValueError, "prompt_layers: a layer's tensor does not have its type, or is not contiguous");
+            if (e[10]->dim() != 4 || (i && e[10]->size(2) != T)) raise(PyExc_ValueError, "prompt_layers: caches are [B, heads, T, D] with one T for all layers");
             T = e[10]->size(2);
-            if (e[0]->numel() * 4 != (qd + 2 * kvd) * hidden || e[1]->numel() != qd + 2 * kvd || e[2]->numel() * 4 != hidden * qd || e[4]->numel() * 4 != 2 * inter * hidden ||
-                e[5]->numel() != 2 * inter || e[6]->numel() * 4 != hidden * inter || e[8]->numel() != hidden || e[9]->numel() != hidden || e[10]->numel() != B * T * kvd ||
-                e[11]->numel() != B * T * kvd)
+            if (e[0]->numel() * 4 != (qd + 2 * kvd) * hidden || e[1]->numel() != qd + 2 * kvd || e[2]->numel() * 4 != hidden * qd || e[3]->numel() < 1 ||
+                e[4]->numel() * 4 != 2 * inter * hidden || e[5]->numel() != 2 * inter || e[6]->numel() * 4 != hidden * inter || e[7]->numel() < 1 ||
+                e[8]->numel() != hidden || e[9]->numel() != hidden || e[10]->numel() != B * T * kvd || e[11]->numel() != B * T * kvd || S > T)
                 raise(PyExc_ValueError, "prompt_layers: a layer's tensor does not have its shape");
+            for (const at::Tensor* one : e) together = together && one->device() == h.device();
             layers[i] = {static_cast<const uint8_t*>(e[0]->data_ptr()), static_cast<const uint8_t*>(e[2]->data_ptr()), static_cast<const uint8_t*>(e[4]->data_ptr()),
                          static_cast<const uint8_t*>(e[6]->data_ptr()), e[1]->data_ptr<float>(), e[3]->data_ptr<float>(), e[5]->data_ptr<float>(), e[7]->data_ptr<float>(),
                          e[8]->data_ptr(), e[9]->data_ptr(), e[10]->data_ptr(), e[11]->data_ptr()};
         }
+        for (const at::Tensor* one : {&cos, &sin, &xq, &aq, &scale, &qkv, &gu, &att, &res, &ws}) together = together && one->device() == h.device();
+        need_cuda({&h});
+        if (!together) raise(PyExc_ValueError, "prompt_layers: tensors on different devices");
         c10::cuda::CUDAGuard guard(h.device());
         void* const stream = c10::cuda::getCurrentCUDAStream().stream();
         int8_t* const q8 = xq.data_ptr<int8_t>();

@@ -680,3 +680,23 @@ def test_prompt_layers_in_native_code(wf, monkeypatch, B, S, hidden, n_q, n_kv, 
     assert torch.equal(m.prefill(ids, all_logits=True), native[0])
     assert all(torch.equal(a, b) for a, b in zip([L[c] for L in m.layers for c in ("kc", "vc")], native[1]))
     wf.device_status()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_prompt_attention_behind_scores_that_overflow(wf, D):
+    """A tile of keys whose scores are all -inf in fp32 counts for nothing once a later score is finite, as in softmax; the queries that
+    see nothing else are NaN, as there.  The 1e-2 of the test above."""
+    from wrinklefree_monorepo_b200 import ops
+
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(D)
+    S = 150
+    q, kc, vc = (torch.randn(*shape, generator=g, device=dev).bfloat16() for shape in ((S, D), (1, 1, S, D), (1, 1, S, D)))
+    q[:, 0], kc[:, :, :, 0] = 1e20, 0.0
+    kc[:, :, :70, 0] = -1e30
+    out = ops.attn_prompt(q, kc, vc, torch.zeros_like(q), S)
+    s = (q.float() @ kc[0, 0].float().t() * D ** -0.5).masked_fill(torch.ones(S, S, dtype=torch.bool, device=dev).triu(1), float("-inf"))
+    ref = torch.softmax(s, -1) @ vc[0, 0].float()
+    assert bool(ref[:70].isnan().all()) and bool(ref[70:].isfinite().all())
+    assert bool(out[:70].isnan().all())
+    assert float((out[70:].float() - ref[70:]).abs().max() / ref[70:].abs().max()) <= 1e-2

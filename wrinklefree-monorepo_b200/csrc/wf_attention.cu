@@ -402,8 +402,9 @@ __global__ void __launch_bounds__(AT_THREADS) attn_prompt_kernel(const PromptPar
                     mx = fmaxf(mx, v);
                 }
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));  // finite: position 0 is open to every query
-            corr[h] = exp2f(m[h] - mx);
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float base = mx == -INFINITY ? 0.f : mx;  // every score of the row so far has overflowed to -inf: weights of zero, not inf - inf
+            corr[h] = exp2f(m[h] - base);
             m[h] = mx;
             float ps = 0.f;
 #pragma unroll
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_prompt_kernel(const PromptPar
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     float& v = sc[n][2 * h + e];
-                    v = exp2f(v - mx);
+                    v = exp2f(v - base);
                     ps += v;
                 }
             l[h] = l[h] * corr[h] + ps;  // this thread's columns; summed over the four threads of the row at the end

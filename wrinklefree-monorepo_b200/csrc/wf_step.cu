@@ -63,6 +63,15 @@ __device__ __forceinline__ uint32_t st_pack(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 __device__ __forceinline__ void st_sync() { asm volatile("bar.sync 1, 480;\n" ::: "memory"); }  // the consumer warps
+// ... and whether `v` holds for any of their threads: the same answer for all of them
+__device__ __forceinline__ bool st_sync_any(bool v) {
+    unsigned r;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, 1, 480, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(r)
+                 : "r"(static_cast<unsigned>(v))
+                 : "memory");
+    return r != 0;
+}
 __device__ __forceinline__ uint32_t st_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ uint32_t st_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ uint32_t st_map(uint32_t addr, uint32_t rank) {
@@ -92,12 +101,12 @@ __device__ __forceinline__ unsigned st_test(uint32_t bar, unsigned parity) {
                  : "memory");
     return ok;
 }
-__device__ __noinline__ void st_wait_long(uint32_t bar, unsigned parity, volatile int* poisoned) {
+__device__ __noinline__ bool st_wait_long(uint32_t bar, unsigned parity, volatile int* poisoned) {
     unsigned long long t0 = 0;
     for (unsigned it = 1;; ++it) {
-        if (st_test(bar, parity)) return;
+        if (st_test(bar, parity)) return true;
         if ((it & 1023) == 0) {
-            if (*poisoned) return;
+            if (*poisoned) return false;
             unsigned long long now;
             asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(now));
             if (t0 == 0) t0 = now;
@@ -106,10 +115,23 @@ __device__ __noinline__ void st_wait_long(uint32_t bar, unsigned parity, volatil
     }
     *poisoned = 1;
     atomicExch(&WF_STATUS_WORD, WF_E_LIMIT);
+    return false;
 }
-__device__ __forceinline__ void st_wait(uint64_t* bar, unsigned parity, volatile int* poisoned) {
+// False when the phase has not completed within the limit, or another wait of this CTA has given up meanwhile: what it stands for has not
+// arrived, and its barrier may not be armed again.  The whole warp calls it and gets one answer.
+__device__ __forceinline__ bool st_wait(uint64_t* bar, unsigned parity, volatile int* poisoned) {
     const uint32_t a = smem_u32(bar);
-    if (!st_test(a, parity)) st_wait_long(a, parity, poisoned);
+    return __all_sync(0xffffffffu, st_test(a, parity) || st_wait_long(a, parity, poisoned));
+}
+// Time for what is on its way into this CTA's shared memory to land.
+__device__ __noinline__ void st_settle() {
+    unsigned long long t0, now;
+    asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t0));
+    for (int it = 0; it < 1000; ++it) {
+        __nanosleep(2000);
+        asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(now));
+        if (now - t0 > 500000) break;
+    }
 }
 
 // Rows [r0, r0 + n) of this CTA: whole groups of four rows (8 bytes of results), shared out evenly; never empty (N >= 4 CTAs).
@@ -204,7 +226,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
     if (warp == ST_WARPS) {
         // ---- producer: norm weights and scales of a layer, then its packed rows, stage by stage, as far ahead as there is room
         int s = 0;
-        unsigned lap = 0;
+        unsigned lap = 0, norms[2] = {0, 0};  // norms: how often either layer's barrier was armed
         constexpr int NPTR = sizeof(wf_step_layer) / 8;
         static_assert(NPTR == 18, "codes, scales, norms, caches");
         const uint64_t* table = reinterpret_cast<const uint64_t*>(p.layers);
@@ -238,6 +260,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
             __syncwarp();
             if (lane == 0 && !poisoned) {
                 mbar_expect_tx(&meta_full[ms], hidden * 4);
+                if (ms) ++norms[1]; else ++norms[0];
                 bulk_copy_g2s(meta + 48, reinterpret_cast<const void*>(n1), hidden * 2, &meta_full[ms]);
                 bulk_copy_g2s(meta + 48 + hidden * 2, reinterpret_cast<const void*>(n2), hidden * 2, &meta_full[ms]);
                 // q/k/v: rows of up to three matrices side by side
@@ -273,6 +296,15 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
                 }
             }
             __syncwarp();
+        }
+        if (poisoned && lane == 0) {  // the copies in flight land before the shared memory goes away: the last one of every stage and of both layers' norms
+            volatile int drained = 0;
+            for (int i = 0; i < p.stages; ++i) {
+                const unsigned n = lap + (i < s ? 1 : 0);
+                if (n > 0) mbar_wait(&full[i], (n - 1) & 1, &drained);
+            }
+            for (int i = 0; i < 2; ++i)
+                if (norms[i] > 0) mbar_wait(&meta_full[i], (norms[i] - 1) & 1, &drained);
         }
     } else {
         // ---- consumers.  One body of code for the four projections of a layer, loops that are not unrolled: a step runs through all of
@@ -320,20 +352,25 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
             rope[i] = i < D / 2 ? __ldg(p.cosv + static_cast<int64_t>(slot) * (D / 2) + i) : __ldg(p.sinv + static_cast<int64_t>(slot) * (D / 2) + i - D / 2);
         st_sync();
 
+        // A wait that has run out ends the CTA's part: its warps agree on it at the next barrier in front of a send or a cache write and
+        // leave, so that nothing goes out that is computed from what has not arrived; the cluster's other CTAs, which wait for it, run
+        // out in turn.  A barrier whose phase has not completed is not armed again.
+        bool ok = true;
 #pragma unroll 1
         for (int l = 0; l <= p.L; ++l) {  // the turn behind the last layer: its residual add and the final norm
             const int ms = l & 1;
             const uint8_t* meta = smem + p.o_meta + ms * p.meta_bytes;
             const float* scale = reinterpret_cast<const float*>(meta);
-            if (l < p.L) st_wait(&meta_full[ms], (l >> 1) & 1, &poisoned);
+            if (l < p.L) ok &= st_wait(&meta_full[ms], (l >> 1) & 1, &poisoned);
 #pragma unroll 1
             for (int ph = 0; ph < 4; ++ph) {  // q/k/v, o, gate/up, down
                 const int K = ph == 1 ? QD : (ph == 3 ? inter : hidden);
                 // ---- what it waits for; the barrier is armed again at once for the next layer
                 if (l + ph > 0) {
                     const int b = ph == 0 ? B_DOWN : (ph == 1 ? B_ATTN : (ph == 2 ? B_O : B_ACT));
-                    st_wait(&xbar[b], (ph == 0 ? l - 1 : l) & 1, &poisoned);
-                    if (tid == 0) mbar_expect_tx(&xbar[b], ph == 1 ? bytes_attn : (ph == 3 ? inter : hidden) * 2);
+                    const bool here = st_wait(&xbar[b], (ph == 0 ? l - 1 : l) & 1, &poisoned);
+                    ok &= here;
+                    if (tid == 0 && here) mbar_expect_tx(&xbar[b], ph == 1 ? bytes_attn : (ph == 3 ? inter : hidden) * 2);
                 }
                 // ---- its input as bf16, this thread's share, and the largest magnitude
                 uint32_t mx = 0;
@@ -427,7 +464,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
                 const int ll = p.lpr_log2[ph], lpr = 1 << ll, col = lane & (lpr - 1), sub = lane >> ll, rpw = 32 >> ll;
 #pragma unroll 1
                 for (int b = 0; b < sp.count; ++b) {
-                    st_wait(&full[s], lap & 1, &poisoned);
+                    if (!st_wait(&full[s], lap & 1, &poisoned)) {
+                        ok = false;
+                        break;
+                    }
                     const uint8_t* st = ring + static_cast<size_t>(s) * p.stage_bytes;
                     const int n = min(sp.per, r.n - b * sp.per), pairs = ph == 2 ? n : (n + 1) >> 1, total = ph == 2 ? 2 * n : n;
 #pragma unroll 1
@@ -472,7 +512,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
                     if (++s == p.stages) { s = 0; ++lap; }
                 }
                 if (ph == 3 && lane == 0) mbar_arrive(&meta_empty[ms]);
-                st_sync();
+                if (st_sync_any(!ok)) goto given_up;
                 // ---- the results to every CTA, 8 bytes per store
                 {
                     uint8_t* dst = smem + (ph == 0 ? p.o_qkv : (ph == 1 ? p.o_o : (ph == 2 ? p.o_act : p.o_down))) + 2 * r.r0;
@@ -503,8 +543,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
                     }
                 };
                 if (nw > 0) load_tile(tile0);  // a warp without a tile loads nothing: its positions are not valid
-                st_wait(&xbar[B_QKV], l & 1, &poisoned);
-                if (tid == 0) mbar_expect_tx(&xbar[B_QKV], NQKV * 2);
+                const bool here = st_wait(&xbar[B_QKV], l & 1, &poisoned);
+                ok &= here;
+                if (tid == 0 && here) mbar_expect_tx(&xbar[B_QKV], NQKV * 2);
                 if (nw == 0) continue;
 #pragma unroll 1
                 for (int i = tid; i < (G + 1) * (D / 2); i += ST_CONSUMERS) {  // the last "head" is the key
@@ -520,7 +561,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
                         kn[e + D / 2] = y2;
                     }
                 }
-                st_sync();
+                if (st_sync_any(!ok)) goto given_up;
                 const __nv_bfloat16* vn = qkv_s + QD + KVD + kvh * D;
                 if (split == 0 && tid < D / 4) {  // the new position goes to the caches
                     const bool is_k = tid < D / 8;
@@ -625,10 +666,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
                 }
             }
         }
+    given_up:;
     }
-    if (poisoned) __nanosleep(500000);  // what is still on its way lands before the shared memory goes away
     __syncwarp();
     st_cluster_sync();  // no CTA leaves while another may still send to it
+    if (poisoned) st_settle();  // what was sent to a CTA that has stopped waiting for it
 }
 
 static int st_align(int v, int a) { return (v + a - 1) / a * a; }

@@ -700,3 +700,34 @@ def test_prompt_attention_behind_scores_that_overflow(wf, D):
     assert bool(ref[:70].isnan().all()) and bool(ref[70:].isfinite().all())
     assert bool(out[:70].isnan().all())
     assert float((out[70:].float() - ref[70:]).abs().max() / ref[70:].abs().max()) <= 1e-2
+
+
+def test_layer_launch_with_a_split_of_infinite_scores(wf):
+    """Two CTAs share a head's positions, and all scores of one of them are -inf: its part counts for nothing, as in the framework's
+    attention over the same cache.  The 3e-2 of the comparison with the separate launches."""
+    from wrinklefree_monorepo_b200.decoder import DecoderConfig, TernaryDecoder
+
+    cfg = DecoderConfig(layers=1, hidden=256, n_q=2, n_kv=2, head_dim=64, intermediate=512, vocab=300)
+    dev = torch.device("cuda", 0)
+    ms = [TernaryDecoder(cfg, 1, 300, dev, seed=3, fuse=fuse) for fuse in (None, False)]
+    assert ms[0].resident is not None
+    ms[1].attention = "library"
+    g = torch.Generator(device=dev).manual_seed(1)
+    caches = [torch.randn(1, 2, 300, 64, generator=g, device=dev).bfloat16() for _ in range(2)]
+    logits = []
+    ms[1].pos.fill_(270)
+    ms[1]._decode_step()
+    q = ms[1].layers[0]["qkv"][0].view(2, 64)  # rotated in place
+    for head in range(2):
+        e = int(q[head].float().abs().argmax())
+        for tile in range(1, 17, 2):  # seventeen tiles of 16 positions: the second CTA takes the odd ones
+            caches[0][0, head, tile * 16:tile * 16 + 16, e] = -torch.sign(q[head, e]) * float("inf")
+    for m in ms:
+        for c, given in zip(("kc", "vc"), caches):
+            m.layers[0][c].copy_(given)
+        m.pos.fill_(270)
+        m._decode_step()
+        logits.append(m.logits.float())
+    assert bool(logits[1].isfinite().all())
+    assert float((logits[0] - logits[1]).abs().max() / logits[1].abs().max()) <= 3e-2
+    wf.device_status()

@@ -416,6 +416,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
                         float top = ml[0];
 #pragma unroll 1
                         for (int w = 1; w < S; ++w) top = fmaxf(top, ml[2 * w]);
+                        if (top == -INFINITY) top = 0.f;  // no score above -inf: weights of zero, not inf - inf
                         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
                         float ls = 0.f;
 #pragma unroll 1
@@ -644,13 +645,14 @@ __global__ void __launch_bounds__(ST_THREADS, 1) decode_layers_kernel(const __gr
                         float top = red_ml[gg * 2];
 #pragma unroll 1
                         for (int w = 1; w < nw; ++w) top = fmaxf(top, red_ml[(w * G + gg) * 2]);
+                        const float base = top == -INFINITY ? 0.f : top;  // of a split whose scores are all -inf: it counts for nothing in the other splits' sum
                         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
                         float lsum = 0.f;
 #pragma unroll 1
                         for (int w = 0; w < nw; ++w) {
                             const float2 ml = *reinterpret_cast<const float2*>(red_ml + (w * G + gg) * 2);
                             const float4 v = *reinterpret_cast<const float4*>(red_o + (w * G + gg) * D + e);
-                            const float f = st_exp2(ml.x - top);
+                            const float f = st_exp2(ml.x - base);
                             acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
                             lsum += ml.y * f;
                         }

@@ -514,3 +514,17 @@ def test_native_prompt_loop_takes_its_shapes_only(wf):
                 dict(o=codes(hidden, qd).to(torch.int8)), dict(o_s=torch.zeros(0)), dict(down_s=torch.zeros(2).half()), dict(kc=z(B * nkv, t, d)), dict(gu_s=torch.zeros(2 * inter + 1))):
         with pytest.raises(ValueError):
             call(layer(), layer(**bad))
+
+
+def test_decode_step_with_embeddings_that_require_gradients(wf):
+    """A decoder made of a model's named_parameters holds an embedding that requires gradients; a step gathers its rows all the same."""
+    from wrinklefree_monorepo_b200.decoder import SMOLLM2_135M, TernaryDecoder
+
+    m = object.__new__(TernaryDecoder)
+    m.cfg, m.B, m.masked, m.attention = SMOLLM2_135M, 2, True, "kernel"
+    m.embed, m.tok, m.h = torch.randn(5, 8, requires_grad=True), torch.tensor([3, 1]), torch.empty(2, 8)
+    m.resident = type("Resident", (), {"run": lambda *a, **k: None})()
+    m.xf = m.head_out = m.pos = None
+    m._head, m._greedy = lambda *a, **k: None, lambda *a, **k: None
+    m._decode_step()
+    assert torch.equal(m.h, m.embed[[3, 1]]) and not m.h.requires_grad

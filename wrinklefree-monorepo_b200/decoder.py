@@ -332,7 +332,7 @@ class TernaryDecoder:
         starts while its predecessor drains (the projections stream their first weights meanwhile) and waits for it
         before it reads an activation."""
         cfg, B, d = self.cfg, self.B, self.cfg.head_dim
-        torch.ops.aten.index.Tensor_out(self.embed, [self.tok], out=self.h)  # residual stream [B, hidden]
+        torch.ops.aten.index.Tensor_out(self.embed.detach(), [self.tok], out=self.h)  # residual stream [B, hidden]
         if self.resident is not None and self.masked and self.attention == "kernel":
             self.resident.run(self.h, self.xf, self.pos, pdl=True)
             return self._greedy(self._head(self.xf, self.head_out, pdl=True), advance=True)

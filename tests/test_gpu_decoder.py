@@ -731,3 +731,21 @@ def test_layer_launch_with_a_split_of_infinite_scores(wf):
     assert bool(logits[1].isfinite().all())
     assert float((logits[0] - logits[1]).abs().max() / logits[1].abs().max()) <= 3e-2
     wf.device_status()
+
+
+@pytest.mark.parametrize("m,i", [(1, 8), (5, 192), (130, 6912)])
+@pytest.mark.parametrize("mode", ["silu", "relu2"])
+def test_gate_activation_of_rows_side_by_side(wf, m, i, mode):
+    """gate and up as the halves of one contraction's rows, the activation as bf16 beside its codes: the bits of the plain activation of
+    contiguous copies, as a prompt with sub-layer norms takes it."""
+    from wrinklefree_monorepo_b200 import ops
+
+    dev = torch.device("cuda", 0)
+    rows = torch.randn(m, 2 * i, generator=torch.Generator(device=dev).manual_seed(i), device=dev).bfloat16()
+    g, u = rows.split([i, i], 1)
+    out, q, s = torch.empty(m, i, dtype=torch.bfloat16, device=dev), torch.empty(m, i, dtype=torch.int8, device=dev), torch.empty(m, device=dev)
+    ops.act_mul_quant(g, u, q, s, mode=mode, out=out)
+    want = ops.act_mul(g.contiguous(), u.contiguous(), torch.empty_like(out), mode)
+    assert torch.equal(out, want)
+    wq, ws = ops.act_quant_i8(want, eps=1e-5)
+    assert torch.equal(q, wq) and torch.equal(s, ws.view(-1))

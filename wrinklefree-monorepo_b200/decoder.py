@@ -512,6 +512,7 @@ class TernaryDecoder:
         q, k, v = qkv.split([nqd, nkd, nkd], 1)
         g, u = gu.split([i_loc, i_loc], 1)
         ws = ops.rows_workspace(M, [(qkv.shape[1], cfg.hidden), (gu.shape[1], cfg.hidden)], dev)
+        act = empty(M, i_loc) if cfg.subln else None
 
         h, delta = self.embed[ids].reshape(M, cfg.hidden), None
         native = own and not cfg.subln and self.tp == 1 and self.layers  # the loop below, in native code
@@ -537,7 +538,7 @@ class TernaryDecoder:
             ops.add_rmsnorm_quant_(h, self._allreduce(o), L["n2"], xq, s1, cfg.eps)
             ops.bitlinear_rows(xq, s1, *L["gu_rows"], gu, ws)
             if cfg.subln:
-                act = ops.act_mul(g.contiguous(), u.contiguous(), empty(M, i_loc), cfg.act)
+                ops.act_mul_quant(g, u, aq, s1, mode=cfg.act, out=act)  # takes rows of wider tensors; the codes are those of the norm, written next
                 ops.add_rmsnorm_quant_(act, None, L["sf"], aq, s1, cfg.subln_eps)
             else:
                 ops.act_mul_quant(g, u, aq, s1, mode=cfg.act)

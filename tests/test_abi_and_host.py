@@ -528,3 +528,12 @@ def test_decode_step_with_embeddings_that_require_gradients(wf):
     m._head, m._greedy = lambda *a, **k: None, lambda *a, **k: None
     m._decode_step()
     assert torch.equal(m.h, m.embed[[3, 1]]) and not m.h.requires_grad
+
+
+def test_which_prompts_the_attention_kernel_takes(wf):
+    """Shapes that the launch refuses stay with the framework's attention: 65536 sequences of one token were sent to it."""
+    from wrinklefree_monorepo_b200 import decoder
+
+    takes = decoder._prompt_kernel_takes
+    assert takes(1, 121, 9, 3, 64) and takes(65535, 1, 1, 1, 64) and not takes(65536, 1, 1, 1, 64)
+    assert not takes(1, 8, 4, 2, 96) and not takes(1, 8, 4, 3, 64) and not takes(1, 1 << 14, 1, 1, 64)

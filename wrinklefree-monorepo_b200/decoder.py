@@ -49,6 +49,13 @@ class DecoderConfig:
 # tokens 118 / 150, 1024 tokens 165 / 151; 32 heads of 128: 121 tokens 127 / 149, 300 tokens 174 / 174, 512 tokens 211 / 203.
 PROMPT_KERNEL_MAX = 1 << 29
 
+
+def _prompt_kernel_takes(B: int, S: int, nq: int, nkv: int, d: int) -> bool:
+    """Whether a prompt's attention runs on this library's kernel: the shapes that it takes (sequences are the grid's second dimension), at
+    sizes where it is the faster one."""
+    return d in (64, 128) and nq % nkv == 0 and B < 65536 and B * nq * S * S * d <= PROMPT_KERNEL_MAX
+
+
 SMOLLM2_135M = DecoderConfig(layers=30, hidden=576, n_q=9, n_kv=3, head_dim=64, intermediate=1536, vocab=49152, rope_theta=1e5)
 LLAMA3_8B = DecoderConfig(layers=32, hidden=4096, n_q=32, n_kv=8, head_dim=128, intermediate=14336, vocab=128256, rope_theta=5e5)
 
@@ -500,7 +507,7 @@ class TernaryDecoder:
         M, dev, dt = B * S, self.dev, self.dtype
         i_loc = self.i_hi - self.i_lo
         nqd, nkd = self.nq * d, self.nkv * d
-        own = d in (64, 128) and M * self.nq * S * d <= PROMPT_KERNEL_MAX and self.nq % self.nkv == 0
+        own = _prompt_kernel_takes(B, S, self.nq, self.nkv, d)
 
         def empty(*shape, dtype=dt):
             return torch.empty(*shape, dtype=dtype, device=dev)

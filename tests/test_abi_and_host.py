@@ -523,11 +523,43 @@ def test_decode_step_with_embeddings_that_require_gradients(wf):
     m = object.__new__(TernaryDecoder)
     m.cfg, m.B, m.masked, m.attention = SMOLLM2_135M, 2, True, "kernel"
     m.embed, m.tok, m.h = torch.randn(5, 8, requires_grad=True), torch.tensor([3, 1]), torch.empty(2, 8)
-    m.resident = type("Resident", (), {"run": lambda *a, **k: None})()
-    m.xf = m.head_out = m.pos = None
+    m.resident = type("Resident", (), {"run": lambda *a, **k: None, "holds": lambda *a: True})()
+    m.xf = m.head_out = m.pos = m.layers = m.norm_f = m.cos = m.sin = None
     m._head, m._greedy = lambda *a, **k: None, lambda *a, **k: None
     m._decode_step()
     assert torch.equal(m.h, m.embed[[3, 1]]) and not m.h.requires_grad
+
+
+@pytest.mark.parametrize("name", ["norm_f", "cos", "sin", "n1", "n2", "kc", "vc", "layers", None])
+def test_decode_step_takes_tensors_put_in_place_of_others(wf, launches, monkeypatch, name):
+    """The one launch for all layers has the addresses of what the decoder was built with.  Rotary tables, a norm weight or a cache that a
+    caller has put in another's place are what the next step computes with: it takes the separate launches then."""
+    from wrinklefree_monorepo_b200 import ops
+    from wrinklefree_monorepo_b200.decoder import DecoderConfig, TernaryDecoder
+
+    B, hidden, nq, nkv, d, inter, t = 2, 128, 4, 2, 64, 192, 5
+    z = lambda *shape, dtype=torch.bfloat16: torch.zeros(*shape, dtype=dtype)  # noqa: E731
+    shapes = dict(q=(nq * d, hidden), k=(nkv * d, hidden), v=(nkv * d, hidden), o=(hidden, nq * d), gate=(inter, hidden), up=(inter, hidden), down=(hidden, inter))
+    m = object.__new__(TernaryDecoder)
+    m.cfg = DecoderConfig(layers=2, hidden=hidden, n_q=nq, n_kv=nkv, head_dim=d, intermediate=inter, vocab=7)
+    m.B, m.T, m.tp, m.prefetch, m._fuse_opt, m.dtype, m.dev = B, t, 1, False, None, torch.bfloat16, "cpu"
+    m.masked, m.attention, m.fused, m.head_out = True, "kernel", True, None
+    m.layers = [{**{n: (z(r, k // 4, dtype=torch.uint8), torch.zeros(2)) for n, (r, k) in shapes.items()}, "n1": z(hidden), "n2": z(hidden),
+                 "kc": z(B, nkv, t, d), "vc": z(B, nkv, t, d)} for _ in range(2)]
+    m.norm_f, m.cos, m.sin = z(hidden), torch.zeros(t, d // 2), torch.zeros(t, d // 2)
+    m.embed, m.tok, m.pos, m.h, m.xf = z(7, hidden), torch.zeros(B, dtype=torch.long), torch.zeros((), dtype=torch.long), z(B, hidden), z(B, hidden)
+    cluster = type("Lib", (), {"wf_decode_layers_cluster": lambda *a: 16, "__getattr__": lambda s, n: lambda *a: launches.append((n, a)) or 0})()
+    monkeypatch.setattr(ops.L, "lib", lambda: cluster)
+    m.resident = m._resident_layers()
+    m._head, m._greedy, m._decode_step_fused = lambda *a, **k: None, lambda *a, **k: None, lambda: launches.append(("separate", ()))
+    if name in ("norm_f", "cos", "sin"):
+        setattr(m, name, getattr(m, name).clone())
+    elif name == "layers":
+        m.layers = m.layers[:1]
+    elif name:
+        m.layers[1][name] = m.layers[1][name].clone()
+    m._decode_step()
+    assert [n for n, _ in launches] == ["separate" if name else "wf_decode_layers_bf16"]
 
 
 def test_which_prompts_the_attention_kernel_takes(wf):

@@ -340,7 +340,8 @@ class TernaryDecoder:
         before it reads an activation."""
         cfg, B, d = self.cfg, self.B, self.cfg.head_dim
         torch.ops.aten.index.Tensor_out(self.embed.detach(), [self.tok], out=self.h)  # residual stream [B, hidden]
-        if self.resident is not None and self.masked and self.attention == "kernel":
+        if (self.resident is not None and self.masked and self.attention == "kernel"
+                and self.resident.holds(self.layers, self.norm_f, self.cos, self.sin)):  # else the separate launches, which take what is there now
             self.resident.run(self.h, self.xf, self.pos, pdl=True)
             return self._greedy(self._head(self.xf, self.head_out, pdl=True), advance=True)
         if self.fused:

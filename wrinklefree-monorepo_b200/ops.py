@@ -447,6 +447,13 @@ class DecodeLayers:
         self._dev = torch.tensor(rows, dtype=torch.long).to(self.device)
         self.hidden, self.n_q, self.n_kv, self.inter, self.act, self.eps, self.cluster = hidden, n_q, n_kv, inter, 0 if act == "silu" else 1, eps, cluster
 
+    def holds(self, layers, norm_f: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> bool:
+        """Whether a decoder's layers, final norm and rotary tables are the tensors that this launch was made for: it has their addresses,
+        and does not follow a tensor put in the place of another."""
+        kept, *rest = self._keep
+        return (len(layers) == len(kept) and all(a is b for a, b in zip(rest, (norm_f, cos, sin)))
+                and all(L[n] is t for L, lay in zip(layers, kept) for n, t in zip(("n1", "n2", "kc", "vc"), (*lay["norms"], *lay["caches"]))))
+
     def run(self, h: torch.Tensor, xf: torch.Tensor, pos: torch.Tensor, pdl: bool = False):
         """h [B, hidden]: embeddings; xf: the output of the last layer behind the final norm; pos: int64 scalar."""
         _, norm_f, cos, sin = self._keep

@@ -47,10 +47,13 @@ def _row_stride(t: torch.Tensor, rows: int, width: int, name: str) -> int:
     """Elements from one row of `width` to the next of a bf16 tensor that holds at least `rows` of them: contiguous in any shape, or
     two-dimensional with unit inner stride."""
     if t.dtype == torch.bfloat16:
-        if t.is_contiguous() and t.numel() >= rows * width:
-            return width
-        if t.dim() == 2 and t.shape[0] >= rows and t.shape[1] == width and t.stride(1) == 1 and t.stride(0) >= width:
-            return t.stride(0)
+        if t.is_contiguous():
+            if t.numel() >= rows * width:
+                return width
+        elif t.dim() == 2:
+            (n, w), (ld, inner) = t.shape, t.stride()
+            if n >= rows and w == width and inner == 1 and ld >= width:
+                return ld
     raise ValueError(f"{name} must be bf16 rows [{rows}, {width}], contiguous or two-dimensional with unit inner stride; got {t.dtype} {tuple(t.shape)} with strides {t.stride()}")
 
 
@@ -514,18 +517,19 @@ def bitlinear_rows(x: torch.Tensor, x_scale: torch.Tensor, codes: torch.Tensor, 
     """Several projections of the same int8 tokens [M, K] in one call: codes [N, K/4] and row_scale [N] hold their rows side by side,
     out [M, N].  `workspace`: from `rows_workspace`, for calls of one stream."""
     _need_cuda(x, x_scale, codes, row_scale, out, workspace)
-    m, k = x.shape
-    n = codes.shape[0]
-    if x_scale.dtype != torch.float32 or x_scale.numel() != m or not x_scale.is_contiguous() or not row_scale.is_contiguous() or codes.dtype != torch.uint8:
+    (m, k), (ldx, inner), (n, packed), (ldy, inner_y), dev = x.shape, x.stride(), codes.shape, out.stride(), x.device
+    # one expression each: a prompt of few tokens is bound by the host, and these calls by their checks
+    if not (x_scale.dtype == torch.float32 and x_scale.numel() == m and x_scale.is_contiguous() and row_scale.is_contiguous() and codes.dtype == torch.uint8):
         raise ValueError("bitlinear_rows needs contiguous float32 scales, x_scale [M] and row_scale [N], and uint8 codes")
-    if workspace.element_size() != 1 or not workspace.is_contiguous() or any(t.device != x.device for t in (x_scale, codes, row_scale, out, workspace)):
+    if not (workspace.element_size() == 1 and workspace.is_contiguous() and x_scale.device == dev and codes.device == dev and row_scale.device == dev
+            and out.device == dev and workspace.device == dev):
         raise ValueError("bitlinear_rows needs a workspace of bytes, and its tensors on one device")
-    if (x.dtype != torch.int8 or x.stride(1) != 1 or codes.shape[1] * 4 != k or not codes.is_contiguous() or row_scale.shape != (n,) or row_scale.dtype != torch.float32
-            or out.shape != (m, n) or out.stride(1) != 1):
+    if not (x.dtype == torch.int8 and inner == 1 and packed * 4 == k and codes.is_contiguous() and row_scale.shape == (n,) and row_scale.dtype == torch.float32
+            and out.shape == (m, n) and inner_y == 1):
         raise ValueError("bitlinear_rows needs int8 x [M, K], contiguous codes [N, K/4], float32 row_scale [N] and out [M, N] with unit inner strides")
     with torch.cuda.device(x.device):
-        L.check(L.lib().wf_bitlinear_prefill_rows(x.data_ptr(), x.stride(0), x_scale.data_ptr(), codes.data_ptr(), row_scale.data_ptr(), out.data_ptr(),
-                                                  _DT[out.dtype], out.stride(0), m, n, k, workspace.data_ptr(), workspace.numel(), _stream()),
+        L.check(L.lib().wf_bitlinear_prefill_rows(x.data_ptr(), ldx, x_scale.data_ptr(), codes.data_ptr(), row_scale.data_ptr(), out.data_ptr(),
+                                                  _DT[out.dtype], ldy, m, n, k, workspace.data_ptr(), workspace.numel(), _stream()),
                 "wf_bitlinear_prefill_rows")
     return out
 

@@ -317,8 +317,8 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(const AttnPa
 // Causal attention of a prompt, queries [B, S] against the first S positions of the caches.  A CTA takes 64 queries of one head (a warp 16
 // of them, the rows of the matrix instruction) through the tiles of 64 positions up to its own; keys and values come through the
 // same swizzled tiles as above, one tile ahead.  What bounds it at the lengths it is chosen for is the chain of its few tiles; a
-// framework call in its place costs 30 us more of the host, which is what bounds a short prompt (the prompt pass of a layer of width
-// 576 at 121 tokens: 147 us with it, 115 with this kernel).  Blocks with the most tiles start first.
+// framework call in its place keeps the loop over the layers in Python, and the host is what bounds a short prompt (the prompt pass of a layer
+// of width 576 at 121 tokens: 133 us with it, 61 with this kernel).  Of one head's blocks those with the most tiles start first.
 struct PromptParams {
     const __nv_bfloat16* q;    // row b * S + s, stride ldq: [nq * D], rotated
     const __nv_bfloat16* k;    // [B, nkv, T, D]

@@ -13,8 +13,9 @@
 //   * attention: a KV head's positions are split over up to cluster / n_kv CTAs (one until the context is long enough to share);
 //     eight or sixteen lanes hold a position, keys and values go from global memory to registers, and the first tile is
 //     requested before the CTA waits for q, because older positions do not depend on it.  Partial results are exchanged in fp32.
-// Measured, us per layer (all of a step's launches) against the separate launches, context 140: width 576 (MLP 1536) 16 / 25 for one sequence
-// and 16 / 42 for seven; 960 (2560) 22 / 33 for two; 1024 (4096) 23 / 37 for four; 1536 (4096) 38 / 37 for one, 2560 (6912) 89 / 44.
+// Measured, us per layer of a captured step with a head of 512 rows, against the separate launches, context 140: width 576 (MLP 1536) 13.0 / 22.8
+// for one sequence and 13.0 / 39.2 for seven; 960 (2560) 17.3 / 29.5 for two; 1024 (4096) 19.0 / 33.2 for four.  Where it does not pay (with
+// the whole head): 1536 (4096) 38 / 37 for one, 2560 (6912) 89 / 44.
 // Clusters are independent of one another (no grid-wide wait: sequences that do not fit at once run one after another).  Every wait
 // is bounded.  Arithmetic: that of the separate kernels, step by step, except the order of fp32 sums (norm, softmax) and
 // probabilities that stay fp32.
@@ -770,8 +771,13 @@ static int st_clusters(const StepParams& p, int C) {
 using namespace wf;
 
 // Where it pays, in us per layer: 11 for the chain of a layer, 1.1 per 2^20 weights and 3.8 per 2^20 of context x query width with 16 CTAs,
-// twice that with 8 (fitted to widths of 576 to 4096 at contexts of 140 to 4000; within 4 of each up to 45).  The separate
-// launches take 30 to 35 for one or two sequences up to a width of 1024, 36 and more for others.
+// twice that with 8 (within 4 of what was measured for widths of 256 to 4096 and contexts of 140 to 10000, up to 45).  The separate launches take,
+// for one or two sequences, 21 to 32 at context 140 and 28 to 35 at the longest context that the rule takes; for three and more 33 to 44
+// and 37 to 54.  It is the slower one nowhere among the 210 shapes measured (widths of 256 to 1280, one to twelve sequences, at the end of the cache); at the line,
+// this kernel / the separate launches: width 512, context 8900, one sequence 28.8 / 29.5, two 32.2 / 32.1; 576, 7300, 29.8 / 32.0 and 29.6 /
+// 35.1; 1024, 600, one 20.7 / 29.2; four, 2300, 28.9 / 38.4; 576, 10000, seven 35.2 / 53.6.
+// T is the length of the cache: one captured step serves every position.  The kernel reads the valid positions only, so that a short context in
+// a long cache would gain more than the rule assumes, and a cache longer than it allows gets none of it.
 static bool st_pays(int64_t B, int hidden, int nq, int nkv, int D, int inter, int64_t T, int C) {
     const double mi = 1.0 / (1 << 20), weights = mi * hidden * (2.0 * nq * D + 2.0 * nkv * D + 3.0 * inter), context = mi * nq * D * static_cast<double>(T);
     return 11 + (1.1 * weights + 3.8 * context) * 16 / C <= (B <= 2 ? 30 : 36);

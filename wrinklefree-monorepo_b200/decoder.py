@@ -44,9 +44,12 @@ class DecoderConfig:
 
 
 # Largest B x heads x S x S x head width of a prompt whose attention runs on this library's kernel (ops.attn_prompt).  The framework's fused
-# attention is faster on the GPU beyond a few tiles, and takes 30 us more of the host: whole prompt pass in us per layer with this
-# kernel / with the framework's, 9 heads of 64: 121 tokens 115 / 147, 1024 tokens 117 / 149, 2048 tokens 146 / 150; 32 heads of 64: 512
-# tokens 118 / 150, 1024 tokens 165 / 151; 32 heads of 128: 121 tokens 127 / 149, 300 tokens 174 / 174, 512 tokens 211 / 203.
+# attention is faster on the GPU beyond a few tiles, and its call keeps the loop over the layers in Python.  Whole prompt pass in us per
+# layer, with this kernel and the native loop / with the framework's attention: 9 heads of 64 (width 576) 121 tokens 61 / 133, 512
+# tokens 77 / 133, 1024 97 / 133, 2048 148 / 133; 32 heads of 64 (2048) 512 tokens 124 / 151, 1024 173 / 166; 20 heads of 128 (2560) 512 tokens
+# 130 / 152, 1024 191 / 177; 32 heads of 128 (4096) 121 tokens 133 / 152, 300 tokens 169 / 173, 512 tokens 204 / 203, 1024 340 / 307.  Both are even
+# at 2 to 3 x this value for one sequence, and 16 of 121 tokens lose at 1.8 x (4096: 541 / 505): the line lies where the kernel is the faster
+# one in every shape measured.
 PROMPT_KERNEL_MAX = 1 << 29
 
 
@@ -306,8 +309,8 @@ class TernaryDecoder:
                     L["g_down"] = ops.DecodeGroup([dict(codes=L["down"][0], w_scale=L["down"][1], out=L["db"], xchg=xp, **din)])
 
     def _resident_layers(self):
-        """The launch that runs all layers of a step, or None where it does not pay or something only the separate launches have is
-        asked for."""
+        """The launch that runs all layers of a step, or None where it does not pay (a rule on the model and the length of the cache) or
+        something only the separate launches have is asked for."""
         cfg = self.cfg
         if (self.tp > 1 or self._fuse_opt is not None or self.prefetch or self.dtype != torch.bfloat16 or cfg.subln or cfg.layers == 0
                 or cfg.n_q % cfg.n_kv):
@@ -503,7 +506,11 @@ class TernaryDecoder:
         """The prompt pass on this library's kernels (bf16): residual add + RMSNorm with the quantization that q/k/v resp. gate/up
         share, those as one contraction each, RoPE with the cache write, attention (the framework's beyond PROMPT_KERNEL_MAX), gate
         activation with the quantization of down.  A layer is nine calls and thirteen launches, made from native code where nothing else is asked for; with torch operators around the
-        projections, as the fp32 model runs it, 54."""
+        projections, as the fp32 model runs it, 54.
+        q/k/v and gate/up take the contraction for every token count, where separate projections of up to 64 tokens take the kernels for few
+        tokens: one contraction in place of three or two launches is the faster form at each width.  GPU time of a captured pass per layer, with
+        separate projections (and the framework's attention) / this one, 1, 8 and 64 tokens: width 576 39 / 34, 55 / 40, 108 / 62; 2560 49 / 45, 74 / 57, 99 / 72; 4096 74 / 67, 94 / 85, 130 / 107; 8192
+        (two layers) 129 / 120, 152 / 137, 189 / 155."""
         cfg, B, d, S = self.cfg, self.B, self.cfg.head_dim, ids.shape[1]
         M, dev, dt = B * S, self.dev, self.dtype
         i_loc = self.i_hi - self.i_lo
